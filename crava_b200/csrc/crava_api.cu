@@ -993,18 +993,13 @@ crava_status fwd_xy(crava_ctx* ctx, const std::vector<const float*>& src, const 
     GridSet gs;
     gs.n = (int)std::min(g.size() - b, (size_t)kMaxGrids);
     for (int q = 0; q < gs.n; q++) { gs.p[q] = g[b + q]; gs.src[q] = src[b + q]; gs.scale[q] = sc[b + q]; }
-    if (xy_fused_supported(nxp, nyp)) {
-      ProfScope ps(ctx, KT_XY_FWD, st);
-      CUDA_TRY(launch_xy4(true, gs, nxp, nyp, nzp, px->tw, pn->tw, py->tw, st, &nl));
-    } else {
-      {
-        ProfScope ps(ctx, KT_X_R2C, st);
-        CUDA_TRY(launch_x_r2c(gs, nxp, nyp * nzp, px->lp, px->tw, pn->tw, st, &nl));
-      }
-      {
-        ProfScope ps(ctx, KT_LINE_FWD, st);
-        CUDA_TRY(launch_line_fft(gs, cnxp, nyp, (size_t)cnxp, nzp, (size_t)cnxp * nyp, py->lp, py->tw, -1.f, st, &nl));
-      }
+    {
+      ProfScope ps(ctx, KT_X_R2C, st);
+      CUDA_TRY(launch_x_r2c(gs, nxp, nyp * nzp, px->lp, px->tw, pn->tw, st, &nl));
+    }
+    {
+      ProfScope ps(ctx, KT_LINE_FWD, st);
+      CUDA_TRY(launch_line_fft(gs, cnxp, nyp, (size_t)cnxp, nzp, (size_t)cnxp * nyp, py->lp, py->tw, -1.f, st, &nl));
     }
     if (with_z) {
       ProfScope ps(ctx, KT_LINE_FWD, st);
@@ -1031,18 +1026,13 @@ crava_status inv_xy(crava_ctx* ctx, const std::vector<float*>& g, const std::vec
       ProfScope ps(ctx, KT_LINE_INV, st);
       CUDA_TRY(launch_line_fft(gs, cnxp, nzp, (size_t)cnxp * nyp, nyp, (size_t)cnxp, pz->lp, pz->tw, 1.f, st, &nl));
     }
-    if (xy_fused_supported(nxp, nyp)) {
-      ProfScope ps(ctx, KT_XY_INV, st);
-      CUDA_TRY(launch_xy4(false, gs, nxp, nyp, nzp, px->tw, pn->tw, py->tw, st, &nl));
-    } else {
-      {
-        ProfScope ps(ctx, KT_LINE_INV, st);
-        CUDA_TRY(launch_line_fft(gs, cnxp, nyp, (size_t)cnxp, nzp, (size_t)cnxp * nyp, py->lp, py->tw, 1.f, st, &nl));
-      }
-      {
-        ProfScope ps(ctx, KT_X_C2R, st);
-        CUDA_TRY(launch_x_c2r(gs, nxp, nyp * nzp, px->lp, px->tw, pn->tw, st, &nl));
-      }
+    {
+      ProfScope ps(ctx, KT_LINE_INV, st);
+      CUDA_TRY(launch_line_fft(gs, cnxp, nyp, (size_t)cnxp, nzp, (size_t)cnxp * nyp, py->lp, py->tw, 1.f, st, &nl));
+    }
+    {
+      ProfScope ps(ctx, KT_X_C2R, st);
+      CUDA_TRY(launch_x_c2r(gs, nxp, nyp * nzp, px->lp, px->tw, pn->tw, st, &nl));
     }
   }
   ctx->launches += nl;

@@ -1,5 +1,5 @@
 // Dispatch of the four-step transforms (kernels and launch templates in fft4.cuh) over the
-// size table below, and the fused xy pass (opt-in) for a few (nxp, nyp) pairs.
+// size table below.
 #include "fft4_facies.cuh"
 
 namespace crava {
@@ -173,10 +173,10 @@ cudaError_t launch_line4(const GridSet& gs, int ni, int n, size_t pstride, int n
 
 cudaError_t launch_x4(bool fwd, const GridSet& gs, int nxp, int rows, const float2* tw, const float2* twn,
                       cudaStream_t st, int* nlaunch) {
-  if (nxp & 1) return cudaErrorInvalidValue;
-  const int h = nxp / 2;
+  // the transformed length: nxp / 2 complex points, or all of an odd nxp (rows in pairs)
+  const int h = nxp % 2 == 0 ? nxp / 2 : -nxp;
   if (nlaunch) (*nlaunch)++;
-  switch (four_step_part(h)) {
+  switch (four_step_part(h < 0 ? -h : h)) {
     case 1: return four_step_x4_p1(fwd, gs, h, rows, tw, twn, st);
     case 2: return four_step_x4_p2(fwd, gs, h, rows, tw, twn, st);
     case 3: return four_step_x4_p3(fwd, gs, h, rows, tw, twn, st);
@@ -202,72 +202,6 @@ cudaError_t launch_x4_facies(const FaciesFuse& F, const FaciesCornersHost& hc, i
     case 6: return four_step_x4_facies_p6(F, C, h, rows, tw, twn, st);
     default: return cudaErrorInvalidValue;
   }
-}
-
-template <int HX1, int HX2, int NY1, int NY2>
-static cudaError_t xy4(bool fwd, const GridSet& gs, int nzp, const float2* twx, const float2* twn, const float2* twy,
-                       cudaStream_t st) {
-  constexpr int H = HX1 * HX2, NY = NY1 * NY2;
-  const int T = 256;
-  const int rpc = std::max(1, T / HX1);
-  int W = 8, lw = 3;
-  const int SK = (((W - NY2 * W) % 16) + 16) % 16;
-  const int C = std::max(1, std::min(16, tuned("xy_cluster", H, 8)));
-  const size_t work = std::max(x4_smem<HX1, HX2>(false, rpc), line4_smem<NY1, NY2>(W, SK));
-  const size_t smem = sizeof(float2) * (2 * (size_t)H + NY) + work;
-  const void* fn = fwd ? (const void*)k_xy4<HX1, HX2, NY1, NY2, true> : (const void*)k_xy4<HX1, HX2, NY1, NY2, false>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  if (C > 8 && (e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess)
-    return e;
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = C;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.blockDim = dim3(T);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cfg.gridDim = dim3(C);
-  int nclusters = 0;
-  if ((e = cudaOccupancyMaxActiveClusters(&nclusters, fn, &cfg)) != cudaSuccess) return e;
-  if (nclusters < 1) return cudaErrorInvalidConfiguration;
-  const int planes = gs.n * nzp;
-  cfg.gridDim = dim3((unsigned)(std::min(nclusters, planes) * C));
-  if (fwd) return cudaLaunchKernelEx(&cfg, k_xy4<HX1, HX2, NY1, NY2, true>, gs, nzp, rpc, W, lw, SK, twx, twn, twy);
-  return cudaLaunchKernelEx(&cfg, k_xy4<HX1, HX2, NY1, NY2, false>, gs, nzp, rpc, W, lw, SK, twx, twn, twy);
-}
-
-// (nxp, nyp) pairs with a fused xy pass
-#define CRAVA_XY_PAIRS(X)   \
-  X(64, 64, 8, 4, 8, 8)     \
-  X(540, 540, 18, 15, 27, 20) \
-  X(768, 768, 24, 16, 32, 24)
-
-// Opt-in (schedule key xy_fused, n = nxp): at 540^2 and 768^2 the two separate passes are
-// still faster, both being bound by latency rather than by HBM traffic.
-static bool xy_enabled(int nxp) { return tuned("xy_fused", nxp, 0) != 0; }
-
-bool xy_fused_supported(int nxp, int nyp) {
-  if (!xy_enabled(nxp) || !four_step_enabled(nxp)) return false;
-#define CRAVA_CASE(NX, NY, A, B, C2, D) \
-  if (nxp == NX && nyp == NY) return true;
-  CRAVA_XY_PAIRS(CRAVA_CASE)
-#undef CRAVA_CASE
-  return false;
-}
-
-cudaError_t launch_xy4(bool fwd, const GridSet& gs, int nxp, int nyp, int nzp, const float2* twx, const float2* twn,
-                       const float2* twy, cudaStream_t st, int* nlaunch) {
-  if (nlaunch) (*nlaunch)++;
-#define CRAVA_CASE(NX, NY, A, B, C2, D) \
-  if (nxp == NX && nyp == NY) return xy4<A, B, C2, D>(fwd, gs, nzp, twx, twn, twy, st);
-  CRAVA_XY_PAIRS(CRAVA_CASE)
-#undef CRAVA_CASE
-  return cudaErrorInvalidValue;
 }
 
 }  // namespace crava

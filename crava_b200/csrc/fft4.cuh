@@ -5,14 +5,13 @@
 //
 //   k_line4<N1,N2,DIR>  W columns of one strided line set: global -> pass 1 -> shared
 //                       -> pass 2 -> global
-//   k_xr2c4<N1,N2>      rows of even nxp, h = nxp/2 = N1 N2: global -> pass 1 -> shared
-//                       -> pass 2 -> shared (natural order) -> split -> global
-//   k_xc2r4<N1,N2>      global -> merge -> shared -> pass 1 -> pass 2 -> global
+//   k_xr2c4<N1,N2>      rows of even nxp, h = nxp/2 = N1 N2: global -> shared -> pass 1 -> shared
+//                       -> pass 2 and split -> shared -> global
+//   k_xc2r4<N1,N2>      global -> shared -> merge and pass 1 -> shared -> pass 2 -> shared -> global
+//   k_xr2c4o, k_xc2r4o  the same for odd nxp = N1 N2, two rows per complex line
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
-
-#include <cooperative_groups.h>
 
 #include <algorithm>
 #include <cstdlib>
@@ -167,9 +166,9 @@ __device__ __forceinline__ void xr2c4_rows(const float2* src, float2* dst, int n
   __syncthreads();
 }
 
-// nr rows of half spectra in g (pitch h + 1) to scaled real rows in place; the merge step
-// as k_x_c2r (kernels.cu).  Z: rpc * PITCH, Xs: rpc * (h + 1).  Ends with a barrier.
-// The same from rows already staged in Xs (shared), writing g; COPY: the real rows also go
+// nr rows of half spectra staged in Xs (shared, pitch h + 1) to scaled real rows in g (Xs
+// itself, or global memory; same pitch); the merge step as k_x_c2r (kernels.cu).  Z: rpc * PITCH.
+// Ends with a barrier.  COPY: the real rows also go
 // to Vc (shared, row r at r * h pairs of samples).
 template <int N1, int N2, bool COPY = false>
 __device__ __forceinline__ void xc2r4_staged(const float2* Xs, float2* g, int nr, float scale, const float2* tw,
@@ -223,26 +222,6 @@ __device__ __forceinline__ void xc2r4_staged(const float2* Xs, float2* g, int nr
   __syncthreads();
 }
 
-template <int N1, int N2>
-__device__ __forceinline__ void xc2r4_rows(float2* g, int nr, float scale, const float2* tw, const float2* twh,
-                                           float2* Z, float2* Xs) {
-  constexpr int CN = N1 * N2 + 1;
-  {
-    const uint32_t xb = smem_addr(Xs);
-    for (int e = threadIdx.x; e < nr * CN; e += blockDim.x) cp_async8(xb + 8u * (uint32_t)e, g + e);
-    cp_async_commit();
-    cp_async_wait_0();
-  }
-  __syncthreads();
-  xc2r4_staged<N1, N2>(Xs, g, nr, scale, tw, twh, Z);
-}
-
-template <int N1, int N2>
-constexpr size_t x4_smem(bool fwd, int rpc) {
-  using L = RowLayout<N1, N2>;
-  return sizeof(float2) * ((size_t)rpc * L::PITCH + (fwd ? 0 : (size_t)rpc * (L::H + 1)));
-}
-
 // L2 prefetch of the row chunk pf block indices on (x fastest): rows of (h + 1) complex values,
 // chunks of rpc rows, blockIdx.y the grid; from gs.src (FWD) or gs.p.
 template <bool FWD>
@@ -257,6 +236,59 @@ __device__ __forceinline__ void x4_prefetch(const GridSet& gs, int rows, int rpc
   for (size_t o = 0; o < n; o += 8192) l2_prefetch(s + o, 8u * min((size_t)8192, n - o), s, s + n);
 }
 
+// ------------------------------------------------------------------ staged row chunks
+//
+// A chunk of rows is one contiguous run of global memory.  It comes in by 16-byte cp.async and
+// its results, written over it in shared memory, leave by one bulk copy (cp.async.bulk, issued by
+// one thread), so the passes spend no instructions on global addresses and every global access is
+// a full line.  al16: the chunk starts on a 16-byte boundary (the grid is 16-byte aligned and the
+// chunk starts at an even row: two rows are a multiple of 16 bytes whatever nxp is); without it
+// both ways move 8-byte words.
+
+// n 8-byte words from src to dst (shared, 16-byte aligned); the caller commits and waits.
+__device__ __forceinline__ void rows_in(float2* dst, const float2* src, int n, bool al16) {
+  const uint32_t d = smem_addr(dst);
+  if (al16) {
+    const int n2 = n >> 1;
+    for (int e = threadIdx.x; e < n2; e += blockDim.x) cp_async16(d + 16u * (uint32_t)e, src + 2 * e);
+    if ((n & 1) && threadIdx.x == 0) cp_async8(d + 8u * (uint32_t)(n - 1), src + n - 1);
+  } else {
+    for (int e = threadIdx.x; e < n; e += blockDim.x) cp_async8(d + 8u * (uint32_t)e, src + e);
+  }
+  cp_async_commit();
+}
+
+// n 8-byte words from src (shared, 16-byte aligned, written by this CTA's threads, no barrier
+// since) to dst.  Returns when shared memory may be given back.
+__device__ __forceinline__ void rows_out(float2* dst, const float2* src, int n, bool al16) {
+  if (al16) {
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      const uint32_t bytes = 8u * (uint32_t)(n & ~1);
+      if (bytes)
+        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(
+                         __cvta_generic_to_global(dst)),
+                     "r"(smem_addr(src)), "r"(bytes)
+                     : "memory");
+      asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+      if (n & 1) dst[n - 1] = src[n - 1];
+      asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
+    }
+  } else {
+    __syncthreads();
+    for (int e = threadIdx.x; e < n; e += blockDim.x) dst[e] = src[e];
+  }
+}
+
+// shared layout of the row kernels: nt twiddles (rounded up to an even count, so that the rows
+// start on 16 bytes), the staged rows, the exchange buffer of the two passes
+constexpr int even_up(int n) { return (n + 1) & ~1; }
+
+// The forward rows keep their loads and stores in the passes: pass 1's loads are the first thing a
+// thread does and pass 2 stores runs of N1 points; staged both ways they measured slower (540x540x256:
+// 1.24 against 1.18 ms; staged stores alone the same), the rows' second buffer costing resident CTAs.
+//
 // stage != 0: the twiddle tables are copied into shared memory first; 0: the passes read
 // them from global memory (L1-resident: every CTA of the launch reads the same 2 h values),
 // and the CTA's first barrier and the table copy go away.
@@ -290,131 +322,148 @@ __global__ void __launch_bounds__(256) k_xr2c4(const __grid_constant__ GridSet g
 template <int N1, int N2>
 __global__ void __launch_bounds__(256) k_xc2r4(const __grid_constant__ GridSet gs, int rows, int rpc,
                                                const float2* __restrict__ twg, const float2* __restrict__ twn,
-                                               int stage, int pf) {
-  using L = RowLayout<N1, N2>;
+                                               int al16, int pf) {
   constexpr int H = N1 * N2, CN = H + 1;
-  extern __shared__ float2 sm[];
-  const float2 *tw = twg, *twh = twn;
-  float2* Z = sm;
-  const int row0 = blockIdx.x * rpc, nr = min(rpc, rows - row0);
-  float2* g = reinterpret_cast<float2*>(gs.p[blockIdx.y]) + (size_t)row0 * CN;
-  if (pf > 0) x4_prefetch<false>(gs, rows, rpc, CN, pf);
-  if (stage) {
-    float2* t1 = sm;
-    float2* t2 = t1 + H;
-    Z = t2 + H;
-    // the rows' copies go out before the tables are staged
-    float2* Xs = Z + rpc * L::PITCH;
-    const uint32_t xb = smem_addr(Xs);
-    for (int e = threadIdx.x; e < nr * CN; e += blockDim.x) cp_async8(xb + 8u * (uint32_t)e, g + e);
-    cp_async_commit();
-    for (int t = threadIdx.x; t < H; t += blockDim.x) {
-      t1[t] = twg[t];
-      t2[t] = twn[t];
-    }
-    cp_async_wait_0();
-    __syncthreads();
-    xc2r4_staged<N1, N2>(Xs, g, nr, gs.scale[blockIdx.y], t1, t2, Z);
-    return;
-  }
-  xc2r4_rows<N1, N2>(g, nr, gs.scale[blockIdx.y], tw, twh, Z, Z + rpc * L::PITCH);
-}
-
-// ------------------------------------------------------------------ persistent, pipelined
-//
-// The same row and column transforms as persistent CTAs that stage the next unit's input
-// in shared memory with cp.async while the current unit is transformed: every CTA keeps one
-// unit of loads in flight during its arithmetic.  Units are disjoint row chunks or column
-// tiles, each read and written by the one CTA that owns it, so in-place grids are safe.
-
-template <int N1, int N2, bool FWD>
-__global__ void __launch_bounds__(256) k_x4p(const __grid_constant__ GridSet gs, int rows, int rpc, int nchunk,
-                                             const float2* __restrict__ twg, const float2* __restrict__ twn) {
-  using L = RowLayout<N1, N2>;
-  constexpr int H = N1 * N2, CN = H + 1;
-  extern __shared__ float2 sm[];
+  extern __shared__ __align__(16) float2 sm[];
   float2* tw = sm;
   float2* twh = tw + H;
-  float2* const X0 = twh + H;
-  float2* const X1 = X0 + rpc * CN;
-  float2* Z = X1 + rpc * CN;
+  float2* Xs = sm + 2 * H;
+  float2* Z = Xs + even_up(rpc * CN);
+  const int row0 = blockIdx.x * rpc, nr = min(rpc, rows - row0);
+  float2* g = reinterpret_cast<float2*>(gs.p[blockIdx.y]) + (size_t)row0 * CN;
+  rows_in(Xs, g, nr * CN, al16);
+  if (pf > 0) x4_prefetch<false>(gs, rows, rpc, CN, pf);
   for (int t = threadIdx.x; t < H; t += blockDim.x) {
     tw[t] = twg[t];
     twh[t] = twn[t];
   }
-  const int units = gs.n * nchunk;
-  auto issue = [&](int u, float2* buf) {
-    const int gi = u / nchunk, c = u - gi * nchunk;
-    const int row0 = c * rpc, nr = min(rpc, rows - row0);
-    const float2* src = reinterpret_cast<const float2*>(FWD ? gs.src[gi] : gs.p[gi]) + (size_t)row0 * CN;
-    const uint32_t b = smem_addr(buf);
-    for (int e = threadIdx.x; e < nr * CN; e += blockDim.x) cp_async8(b + 8u * (uint32_t)e, src + e);
-  };
-  if ((int)blockIdx.x < units) issue(blockIdx.x, X0);
-  cp_async_commit();
-  int i = 0;
-  for (int u = blockIdx.x; u < units; u += gridDim.x, i ^= 1) {
-    if (u + (int)gridDim.x < units) issue(u + gridDim.x, i ? X0 : X1);
-    cp_async_commit();
-    cp_async_wait_1();
-    __syncthreads();
-    const int gi = u / nchunk, c = u - gi * nchunk;
-    const int row0 = c * rpc, nr = min(rpc, rows - row0);
-    float2* dst = reinterpret_cast<float2*>(gs.p[gi]) + (size_t)row0 * CN;
-    const float2* cur = i ? X1 : X0;
-    if (FWD) xr2c4_rows<N1, N2>(cur, dst, nr, gs.scale[gi], tw, twh, Z);
-    else xc2r4_staged<N1, N2>(cur, dst, nr, gs.scale[gi], tw, twh, Z);
-  }
   cp_async_wait_0();
-  (void)L::PITCH;
+  __syncthreads();
+  xc2r4_staged<N1, N2>(Xs, Xs, nr, gs.scale[blockIdx.y], tw, twh, Z);
+  rows_out(g, Xs, nr * CN, al16);
 }
 
-template <int N1, int N2, int DIR>
-__global__ void __launch_bounds__(256) k_line4p(const __grid_constant__ GridSet gs, int ni, size_t pstride, int no,
-                                                size_t ostride, int W, int lw, int nIT, int SK,
-                                                const float2* __restrict__ twg) {
-  constexpr int N = N1 * N2;
-  extern __shared__ float2 sm[];
+// ------------------------------------------------------------------ rows, odd nxp
+//
+// Odd lengths N = N1 N2 have no half-length form: two rows a, b go through one complex transform
+// of z = a + i b, so a row costs what half a complex line costs, as in the even form.
+//   forward  A[k] = (Z[k] + conj Z[N-k]) / 2,  B[k] = (Z[k] - conj Z[N-k]) / 2i;
+//            item k2 and its mirror N1 - k2 of pass 2 sit in one thread, which then holds Z[k] and
+//            Z[N-k] for all its k (as xr2c4_rows)
+//   inverse  Z[k] = A[k] + i B[k] (k <= N/2), Z[N-k] = conj A[k] + i conj B[k], formed where pass 1
+//            loads it; Im A[0] and Im B[0] have no slot in a real-output transform
+// Rows in global and staged memory have N + 1 floats; the last is written as zero.
+template <int N1, int N2>
+__global__ void __launch_bounds__(256) k_xr2c4o(const __grid_constant__ GridSet gs, int rows, int lpc,
+                                                const float2* __restrict__ twg, int al16) {
+  using L = RowLayout<N1, N2>;
+  constexpr int N = N1 * N2, CN = (N + 1) / 2, NPI = N1 / 2 + 1;
+  extern __shared__ __align__(16) float2 sm[];
   float2* tw = sm;
-  float2* const T0 = sm + N;
-  float2* const T1 = T0 + W * N;
-  float2* Y = T1 + W * N;
-  for (int t = threadIdx.x; t < N; t += blockDim.x) tw[t] = twg[t];
-  const int per_grid = nIT * no, units = gs.n * per_grid;
-  auto locate = [&](int u, int& nw) -> float2* {
-    const int gi = u / per_grid, rem = u - gi * per_grid;
-    const int o = rem / nIT, it = rem - o * nIT;
-    nw = min(W, ni - it * W);
-    return reinterpret_cast<float2*>(gs.p[gi]) + (size_t)o * ostride + (size_t)it * W;
-  };
-  auto issue = [&](int u, float2* buf) {
-    int nw;
-    const float2* g = locate(u, nw);
-    const uint32_t b = smem_addr(buf);
-    for (int e = threadIdx.x; e < N * W; e += blockDim.x) {
-      const int p = e >> lw, w = e & (W - 1);
-      const bool ok = w < nw;
-      cp_async8_zfill(b + 8u * (uint32_t)e, ok ? g + (size_t)p * pstride + w : g, ok);
-    }
-  };
-  if ((int)blockIdx.x < units) issue(blockIdx.x, T0);
-  cp_async_commit();
-  int i = 0;
-  for (int u = blockIdx.x; u < units; u += gridDim.x, i ^= 1) {
-    if (u + (int)gridDim.x < units) issue(u + gridDim.x, i ? T0 : T1);
-    cp_async_commit();
-    cp_async_wait_1();
-    __syncthreads();
-    int nw;
-    float2* g = locate(u, nw);
-    line4_tile<N1, N2, DIR>(i ? T1 : T0, (size_t)W, g, nw, pstride, W, lw, SK, tw, Y);
-  }
+  float2* Xs = sm + even_up(N);
+  float2* Z = Xs + 2 * lpc * CN;
+  const int T = blockDim.x, tid = threadIdx.x;
+  const int row0 = blockIdx.x * 2 * lpc, nr = min(2 * lpc, rows - row0), nl = (nr + 1) / 2;
+  const size_t o = (size_t)row0 * CN;
+  rows_in(Xs, reinterpret_cast<const float2*>(gs.src[blockIdx.y]) + o, nr * CN, al16);
+  for (int t = tid; t < N; t += T) tw[t] = twg[t];
   cp_async_wait_0();
+  __syncthreads();
+  const float* Xf = reinterpret_cast<const float*>(Xs);
+  for (int q = tid; q < nl * N2; q += T) {
+    const int l = q / N2, t = q - l * N2;
+    const float* a = Xf + 2 * l * (N + 1) + t;
+    const bool two = 2 * l + 1 < nr;
+    float2* z = Z + l * L::PITCH;
+    four_step_pass1<N1, N2, -1>(
+        t, tw, [&](int, int m) { return make_float2(a[m * N2], two ? a[N + 1 + m * N2] : 0.f); },
+        [&](int, int k2, float2 v) { z[L::pad(t, k2)] = v; });
+  }
+  __syncthreads();
+  const float hs = 0.5f * gs.scale[blockIdx.y];
+  for (int q = tid; q < nl * NPI; q += T) {
+    const int l = q / NPI, a = q - l * NPI;
+    const float2* z = Z + l * L::PITCH;
+    float2 va[N2], vb[N2];
+    four_step_pass2<N1, N2, -1>(a, [&](int k, int t) { return z[L::pad(t, k)]; }, va);
+    if (a != 0) four_step_pass2<N1, N2, -1>(N1 - a, [&](int k, int t) { return z[L::pad(t, k)]; }, vb);
+    float2* XA = Xs + 2 * l * CN;
+    const bool two = 2 * l + 1 < nr;
+#pragma unroll
+    for (int k1 = 0; k1 < N2; k1++) {
+      const int k = a + N1 * k1;
+      if (k == 0) {
+        XA[0] = make_float2(2.f * hs * va[0].x, 0.f);
+        if (two) XA[CN] = make_float2(2.f * hs * va[0].y, 0.f);
+        continue;
+      }
+      if (a == 0 && 2 * k > N) continue;     // item 0 mirrors itself: its upper half is done below
+      const float2 zm = a == 0 ? va[N2 - k1] : vb[N2 - 1 - k1];
+      const bool lo = 2 * k < N;
+      const int k0 = lo ? k : N - k;
+      const float2 p = lo ? va[k1] : zm, m = lo ? zm : va[k1];   // Z[k0], Z[N - k0]
+      XA[k0] = make_float2(hs * (p.x + m.x), hs * (p.y - m.y));
+      if (two) XA[CN + k0] = make_float2(hs * (p.y + m.y), hs * (m.x - p.x));
+    }
+  }
+  rows_out(reinterpret_cast<float2*>(gs.p[blockIdx.y]) + o, Xs, nr * CN, al16);
 }
 
-// Opt-in (schedule key pipe4): measured slower than the one-unit kernels for the column
-// transforms (staging a W-column tile costs more than it hides) and mixed for the rows.
-static inline bool pipe4_enabled(int n) { return tuned("pipe4", n, 0) != 0; }
+template <int N1, int N2>
+__global__ void __launch_bounds__(256) k_xc2r4o(const __grid_constant__ GridSet gs, int rows, int lpc,
+                                                const float2* __restrict__ twg, int al16) {
+  using L = RowLayout<N1, N2>;
+  constexpr int N = N1 * N2, CN = (N + 1) / 2;
+  extern __shared__ __align__(16) float2 sm[];
+  float2* tw = sm;
+  float2* Xs = sm + even_up(N);
+  float2* Z = Xs + 2 * lpc * CN;
+  const int T = blockDim.x, tid = threadIdx.x;
+  const int row0 = blockIdx.x * 2 * lpc, nr = min(2 * lpc, rows - row0), nl = (nr + 1) / 2;
+  float2* g = reinterpret_cast<float2*>(gs.p[blockIdx.y]) + (size_t)row0 * CN;
+  rows_in(Xs, g, nr * CN, al16);
+  for (int t = tid; t < N; t += T) tw[t] = twg[t];
+  cp_async_wait_0();
+  __syncthreads();
+  for (int q = tid; q < nl * N2; q += T) {
+    const int l = q / N2, t = q - l * N2;
+    const float2* XA = Xs + 2 * l * CN;
+    const bool two = 2 * l + 1 < nr;
+    float2* z = Z + l * L::PITCH;
+    four_step_pass1<N1, N2, 1>(
+        t, tw,
+        [&](int, int m) {
+          const int k = t + N2 * m;
+          const bool lo = 2 * k < N;
+          const int k0 = lo ? k : N - k;
+          float2 a = XA[k0], b = two ? XA[CN + k0] : make_float2(0.f, 0.f);
+          if (k == 0) a.y = b.y = 0.f;
+          return lo ? make_float2(a.x - b.y, a.y + b.x) : make_float2(a.x + b.y, b.x - a.y);
+        },
+        [&](int, int k2, float2 v) { z[L::pad(t, k2)] = v; });
+  }
+  __syncthreads();
+  const float scale = gs.scale[blockIdx.y];
+  float* Xf = reinterpret_cast<float*>(Xs);
+  for (int q = tid; q < nl * N1; q += T) {
+    const int l = q / N1, k2 = q - l * N1;
+    const float2* z = Z + l * L::PITCH;
+    float2 v[N2];
+    four_step_pass2<N1, N2, 1>(k2, [&](int k, int t) { return z[L::pad(t, k)]; }, v);
+    float* a = Xf + 2 * l * (N + 1);
+    const bool two = 2 * l + 1 < nr;
+#pragma unroll
+    for (int k1 = 0; k1 < N2; k1++) {
+      a[k2 + N1 * k1] = v[k1].x * scale;
+      if (two) a[N + 1 + k2 + N1 * k1] = v[k1].y * scale;
+    }
+    if (k2 == 0) {
+      a[N] = 0.f;
+      if (two) a[2 * N + 1] = 0.f;
+    }
+  }
+  rows_out(g, Xs, nr * CN, al16);
+}
 
 static inline cudaError_t resident_grid(const void* fn, int T, size_t smem, int units, int* grid) {
   int dev = 0, nsm = 0, per_sm = 0;
@@ -425,72 +474,6 @@ static inline cudaError_t resident_grid(const void* fn, int T, size_t smem, int 
   if (per_sm < 1) return cudaErrorInvalidConfiguration;
   *grid = std::max(1, std::min(units, per_sm * nsm));
   return cudaSuccess;
-}
-
-// ------------------------------------------------------------------ fused xy passes
-//
-// One z-plane of one grid at a time per cluster of C CTAs: the rows of the plane (x
-// transform, split across the cluster), a cluster barrier, then the columns (y transform,
-// split across the cluster), in place in the destination grid.  The plane (nyp half-
-// spectrum rows, 1-2.4 MB) is written by the first phase and read back by the second while
-// it sits in L2, so each grid crosses HBM once each way per xy pass.  Persistent clusters
-// walk the planes of every grid in the set.  The inverse runs the phases the other way.
-template <int HX1, int HX2, int NY1, int NY2, bool FWD>
-__global__ void __launch_bounds__(256, 2) k_xy4(const __grid_constant__ GridSet gs, int nzp, int rpc, int W, int lw,
-                                             int SK, const float2* __restrict__ twx, const float2* __restrict__ twn,
-                                             const float2* __restrict__ twy) {
-  namespace cg = cooperative_groups;
-  constexpr int H = HX1 * HX2, NY = NY1 * NY2, CN = H + 1;
-  using L = RowLayout<HX1, HX2>;
-  extern __shared__ float2 sm[];
-  float2* tx = sm;
-  float2* th = tx + H;
-  float2* ty = th + H;
-  float2* work = ty + NY;
-  for (int t = threadIdx.x; t < H; t += blockDim.x) {
-    tx[t] = twx[t];
-    th[t] = twn[t];
-  }
-  for (int t = threadIdx.x; t < NY; t += blockDim.x) ty[t] = twy[t];
-  __syncthreads();
-  cg::cluster_group cl = cg::this_cluster();
-  const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
-  const int ncl = gridDim.x / C, cid = blockIdx.x / C;
-  const int planes = gs.n * nzp;
-  const int nchunk = (NY + rpc - 1) / rpc, ntile = (CN + W - 1) / W;
-  const size_t plane = (size_t)NY * CN;
-  for (int p = cid; p < planes; p += ncl) {
-    const int gi = p / nzp, z = p - gi * nzp;
-    float2* dst = reinterpret_cast<float2*>(gs.p[gi]) + (size_t)z * plane;
-    const float scale = gs.scale[gi];
-    if (FWD) {
-      const float2* src = reinterpret_cast<const float2*>(gs.src[gi]) + (size_t)z * plane;
-      for (int c = rank; c < nchunk; c += C) {
-        const int row0 = c * rpc, nr = min(rpc, NY - row0);
-        xr2c4_rows<HX1, HX2>(src + (size_t)row0 * CN, dst + (size_t)row0 * CN, nr, scale, tx, th, work);
-      }
-      __threadfence();
-      cl.sync();
-      __threadfence();  // acquire side: no line of this plane cached before the barrier is reused
-      for (int it = rank; it < ntile; it += C) {
-        const int i0 = it * W;
-        line4_tile<NY1, NY2, -1>(dst + i0, (size_t)CN, dst + i0, min(W, CN - i0), (size_t)CN, W, lw, SK, ty, work);
-      }
-    } else {
-      for (int it = rank; it < ntile; it += C) {
-        const int i0 = it * W;
-        line4_tile<NY1, NY2, 1>(dst + i0, (size_t)CN, dst + i0, min(W, CN - i0), (size_t)CN, W, lw, SK, ty, work);
-      }
-      __threadfence();
-      cl.sync();
-      __threadfence();
-      for (int c = rank; c < nchunk; c += C) {
-        const int row0 = c * rpc, nr = min(rpc, NY - row0);
-        xc2r4_rows<HX1, HX2>(dst + (size_t)row0 * CN, nr, scale, tx, th, work, work + rpc * L::PITCH);
-      }
-    }
-    // a plane's two phases touch only that plane: the next plane needs no cluster barrier
-  }
 }
 
 // ------------------------------------------------------------------ launch templates
@@ -518,27 +501,6 @@ static cudaError_t line4(const GridSet& gs, int ni, size_t pstride, int no, size
   T = std::max(64, std::min(sign < 0.f ? 256 : 512,
                             tuned(sign < 0.f ? "line4_threads_fwd" : "line4_threads_inv", N, T) / 32 * 32));
   const int nIT = (ni + W - 1) / W;
-  if (pipe4_enabled(N)) {
-    // two staged tiles and the work tile: narrower tiles for the longest lines
-    int Wp = W;
-    while (Wp > 1 && sizeof(float2) * (2 * (size_t)Wp * N) + line4_smem<N1, N2>(Wp, SK) > 104 * 1024) Wp /= 2;
-    int lwp = 0;
-    while ((1 << lwp) < Wp) lwp++;
-    const int SKp = Wp < 16 ? (((Wp - N2 * Wp) % 16) + 16) % 16 : 0;
-    const int Tp = std::min(256, round_up32(Wp * std::max(N1, N2)));   // k_line4p is bounded at 256
-    const int nITp = (ni + Wp - 1) / Wp;
-    const size_t smem = sizeof(float2) * ((size_t)N + 2 * (size_t)Wp * N) + line4_smem<N1, N2>(Wp, SKp);
-    const void* fn = sign < 0.f ? (const void*)k_line4p<N1, N2, -1> : (const void*)k_line4p<N1, N2, 1>;
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    int grid = 0;
-    if ((e = resident_grid(fn, Tp, smem, gs.n * nITp * no, &grid)) != cudaSuccess) return e;
-    if (sign < 0.f)
-      k_line4p<N1, N2, -1><<<grid, Tp, smem, st>>>(gs, ni, pstride, no, ostride, Wp, lwp, nITp, SKp, tw);
-    else
-      k_line4p<N1, N2, 1><<<grid, Tp, smem, st>>>(gs, ni, pstride, no, ostride, Wp, lwp, nITp, SKp, tw);
-    return cudaGetLastError();
-  }
   const size_t smem = sizeof(float2) * (size_t)N + line4_smem<N1, N2>(W, SK);
   const void* fn = sign < 0.f ? (const void*)k_line4<N1, N2, -1> : (const void*)k_line4<N1, N2, 1>;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -557,51 +519,91 @@ static cudaError_t line4(const GridSet& gs, int ni, size_t pstride, int no, size
   return cudaGetLastError();
 }
 
+// Threads and lines per CTA of a row kernel whose passes have i1 and i2 items per line of c1 and
+// c2 points each.  A CTA's time is its rounds of T items, each as long as its item, plus a fixed
+// part; per line an SM spends that time over the lines it has in flight (latency), and the issue
+// slots of the T threads, idle ones of a short pass included.  (125 = 25 x 5 at 64 threads and 2
+// lines had 10 busy threads in pass 1: 250x250x200, 21 grids 1.93 ms, with this rule 0.52.)  At
+// most 36 KB of shared memory, so that six CTAs share an SM; lines a multiple of step.
+struct RowShape {
+  int T, lines;
+};
+static inline RowShape row_shape(int i1, int c1, int i2, int c2, size_t fixed, size_t per_line, int step) {
+  RowShape best{64, step};
+  double least = 1e30;
+  for (int T = 64; T <= 256; T += 32)
+    for (int n = step; n <= 64; n += step) {
+      const size_t smem = fixed + n * per_line + 1024;
+      if (n > step && smem > 37 * 1024) break;
+      const int ctas = std::min(32, std::min((int)(227 * 1024 / smem), 65536 / (96 * T)));
+      const double d = (n * i1 + T - 1) / T * (4 + c1) + (n * i2 + T - 1) / T * (4 + c2) + 12;
+      const double t = d / n * (40.0 / std::max(1, ctas) + 2.5 * T / 32);
+      if (t < least * 0.999) {
+        least = t;
+        best = {T, n};
+      }
+    }
+  return best;
+}
+
+static inline bool grids_al16(const GridSet& gs) {
+  uintptr_t a = 0;
+  for (int q = 0; q < gs.n; q++) a |= reinterpret_cast<uintptr_t>(gs.p[q]) | reinterpret_cast<uintptr_t>(gs.src[q]);
+  return a % 16 == 0;
+}
+
 template <int N1, int N2>
 static cudaError_t x4(bool fwd, const GridSet& gs, int rows, const float2* tw, const float2* twn, cudaStream_t st) {
   using L = RowLayout<N1, N2>;
-  // 128-thread blocks: more CTAs per SM and cheaper barriers than 256 (measured 15 % faster);
-  // the inverse rows up to h = 270 are faster still at 64 (3.53 vs 3.66 ms at 540x540x256)
-  const int T = std::max(64, std::min(256, tuned(fwd ? "x4_threads_fwd" : "x4_threads_inv", L::H,
-                                                   (!fwd && L::H <= 270) ? 64 : 128) / 32 * 32));
-  // rows per CTA: by default a whole number of pass-2 items per thread (N1 items per row
-  // inverse, N1 / 2 + 1 item pairs forward); the schedule entry may set up to 64
-  int rpc = std::max(1, fwd ? T / (N1 / 2 + 1) : T / N1);
-  rpc = std::max(1, std::min(64, tuned(fwd ? "x4_rpc_fwd" : "x4_rpc_inv", L::H, rpc)));
-  if (pipe4_enabled(L::H)) {
-    const int nchunk = (rows + rpc - 1) / rpc;
-    const size_t smem = sizeof(float2) * (2 * (size_t)L::H + 2 * (size_t)rpc * (L::H + 1) + (size_t)rpc * L::PITCH);
-    const void* fn = fwd ? (const void*)k_x4p<N1, N2, true> : (const void*)k_x4p<N1, N2, false>;
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    int grid = 0;
-    if ((e = resident_grid(fn, T, smem, gs.n * nchunk, &grid)) != cudaSuccess) return e;
-    if (fwd) k_x4p<N1, N2, true><<<grid, T, smem, st>>>(gs, rows, rpc, nchunk, tw, twn);
-    else k_x4p<N1, N2, false><<<grid, T, smem, st>>>(gs, rows, rpc, nchunk, tw, twn);
-    return cudaGetLastError();
-  }
-  // twiddle tables staged in shared memory (schedule key x4_stage, default 1) or read from
-  // global memory
-  const int stage = tuned(fwd ? "x4_stage_fwd" : "x4_stage_inv", L::H, 1) != 0 ? 1 : 0;
-  const size_t smem = sizeof(float2) * 2 * (size_t)L::H * stage + x4_smem<N1, N2>(fwd, rpc);
+  constexpr int H = L::H;
+  // twiddle tables staged in shared memory (schedule key x4_stage_fwd) or read from global memory
+  const int stage = !fwd || tuned("x4_stage_fwd", H, 1) != 0;
+  const size_t fixed = sizeof(float2) * 2 * (size_t)H * stage;
+  const size_t per = sizeof(float2) * (size_t)(L::PITCH + (fwd ? 0 : H + 1));
+  // the forward form, whose loads go straight into pass 1, is faster at 128 threads with one item
+  // pair each (270x270x256: 0.24 against 0.29 ms) unless that leaves half of pass 1 idle
+  // (250x250x200: 0.25 against 0.19 ms)
+  RowShape rs{128, 128 / (N1 / 2 + 1)};
+  if (!fwd || rs.lines < 1 || 2 * rs.lines * N2 < rs.T)
+    rs = row_shape(N2, N1, fwd ? N1 / 2 + 1 : N1, fwd ? 2 * N2 : N2, fixed, per, fwd ? 1 : 2);
+  const int T = std::max(64, std::min(256, tuned(fwd ? "x4_threads_fwd" : "x4_threads_inv", H, rs.T) / 32 * 32));
+  const int rpc = std::max(1, std::min(64, tuned(fwd ? "x4_rpc_fwd" : "x4_rpc_inv", H, rs.lines)));
+  const size_t smem = fixed + per * rpc + sizeof(float2);
   const void* fn = fwd ? (const void*)k_xr2c4<N1, N2> : (const void*)k_xc2r4<N1, N2>;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   dim3 grid((unsigned)((rows + rpc - 1) / rpc), gs.n);
   // L2 prefetch of the row chunk ahead of the CTAs (schedule keys x4_pf_fwd / x4_pf_inv: the
-  // distance in quarters of the resident CTAs, 0 = off; one wave, 4, measured faster for the
-  // forward rows at h = 270, slower for the inverse ones)
+  // distance in quarters of the resident CTAs, 0 = off)
   int pf = 0;
-  if (const int q = tuned(fwd ? "x4_pf_fwd" : "x4_pf_inv", L::H, fwd ? 4 : 0)) {
+  if (const int q = tuned(fwd ? "x4_pf_fwd" : "x4_pf_inv", H, fwd ? 4 : 0)) {
     int res = 0;
     if ((e = resident_grid(fn, T, smem, 1 << 30, &res)) != cudaSuccess) return e;
     pf = std::max(1, res * q / 4);
   }
+  // every chunk starts at an even row, or two rows' bytes do not matter ((h + 1) even)
+  const int al16 = grids_al16(gs) && (rpc % 2 == 0 || (H + 1) % 2 == 0);
   if (fwd) k_xr2c4<N1, N2><<<grid, T, smem, st>>>(gs, rows, rpc, tw, twn, stage, pf);
-  else k_xc2r4<N1, N2><<<grid, T, smem, st>>>(gs, rows, rpc, tw, twn, stage, pf);
+  else k_xc2r4<N1, N2><<<grid, T, smem, st>>>(gs, rows, rpc, tw, twn, al16, pf);
   return cudaGetLastError();
 }
 
-// Fused xy pass for (h, nyp) pairs; cluster size from CRAVA_XY_CLUSTER (default 8).
+// odd nxp = N1 N2: rows taken in pairs
+template <int N1, int N2>
+static cudaError_t x4_odd(bool fwd, const GridSet& gs, int rows, const float2* tw, cudaStream_t st) {
+  using L = RowLayout<N1, N2>;
+  constexpr int N = N1 * N2;
+  const size_t fixed = sizeof(float2) * even_up(N), per = sizeof(float2) * (size_t)(L::PITCH + N + 1);
+  const RowShape rs = row_shape(N2, N1, fwd ? N1 / 2 + 1 : N1, fwd ? 2 * N2 : N2, fixed, per, 1);
+  const size_t smem = fixed + per * rs.lines;
+  const void* fn = fwd ? (const void*)k_xr2c4o<N1, N2> : (const void*)k_xc2r4o<N1, N2>;
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  dim3 grid((unsigned)((rows + 2 * rs.lines - 1) / (2 * rs.lines)), gs.n);
+  const int al16 = grids_al16(gs);
+  if (fwd) k_xr2c4o<N1, N2><<<grid, rs.T, smem, st>>>(gs, rows, rs.lines, tw, al16);
+  else k_xc2r4o<N1, N2><<<grid, rs.T, smem, st>>>(gs, rows, rs.lines, tw, al16);
+  return cudaGetLastError();
+}
 
 }  // namespace crava

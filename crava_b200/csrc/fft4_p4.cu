@@ -41,10 +41,14 @@ cudaError_t four_step_line4_p4(const GridSet& gs, int ni, int n, size_t pstride,
 
 cudaError_t four_step_x4_p4(bool fwd, const GridSet& gs, int h, int rows, const float2* tw, const float2* twn,
                              cudaStream_t st) {
+  // h > 0: even rows of half length h; h < 0: odd rows of length -h
   switch (h) {
-#define CRAVA_CASE(NN, A, B) \
-  case NN:                   \
-    return x4<A, B>(fwd, gs, rows, tw, twn, st);
+#define CRAVA_CASE(NN, A, B)                                                              \
+  case NN:                                                                                \
+    return x4<A, B>(fwd, gs, rows, tw, twn, st);                                          \
+  case -NN:                                                                               \
+    if constexpr (NN % 2 == 1) return x4_odd<A, B>(fwd, gs, rows, tw, st);                \
+    else return cudaErrorInvalidValue;
     CRAVA_FOUR_STEP_PART(CRAVA_CASE)
 #undef CRAVA_CASE
     default:

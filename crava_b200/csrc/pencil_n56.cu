@@ -1,0 +1,10 @@
+// Instantiations of the pencil pass (pencil.cuh) for 5 and 6 angle stacks.
+#include "pencil.cuh"
+
+namespace crava {
+
+cudaError_t launch_pencil_n56(const ZParams& zp, int threads, cudaStream_t st) {
+  return zp.nth == 5 ? launch_pencil_m<5>(zp, threads, st) : launch_pencil_m<6>(zp, threads, st);
+}
+
+}  // namespace crava
