@@ -7,15 +7,9 @@ entries set through crava_tuning_set and times every kernel class with the libra
 CUDA-event timers (crava_ctx_set_profiling / crava_ctx_kernel_times), keeping per key the
 fastest value.  The keys swept, with their size key n:
 
-  pencil_kernel  n = nzp*16 + ntheta   1 general kernel (zpass.cu), 2 eigen form (pencil.cu)
-  pencil_w       n = nzp*16 + ntheta   eigen form: x-bins per tile (power of two)
-  pencil_sb      n = nzp*16 + ntheta   eigen form: realisations per transform batch (0: no
-                                       realisation slots, the mean stored first)
-  pencil_threads n = nzp*16 + ntheta   eigen form: threads per CTA
-  pencil_dense   n = nzp*16 + ntheta   eigen form: 1 = the 80-register instantiation
-  pencil_nb      n = nzp*16 + ntheta   eigen form: bins of one z position per thread (1 or 2)
-  zpass_w, zpass_sb, zpass_threads     general kernel: tile width, realisations per batch,
-                 n = nzp*16 + ntheta   threads per CTA
+  pencil_w       n = nzp*16 + ntheta   pencil pass: x-bins per tile (2, 4 or 8)
+  pencil_sb      n = nzp*16 + ntheta   pencil pass: realisations per transform batch (1 to 4)
+  pencil_threads n = nzp*16 + ntheta   pencil pass: threads per CTA
   line4_w_fwd, line4_w_inv   n = N     four-step column transforms: columns per tile
   line4_threads_fwd, line4_threads_inv  four-step column transforms: threads per CTA (n = N;
                                         at most 256 forward, 512 inverse)
@@ -118,47 +112,22 @@ def tune_workload(name, w, reps, entries, log):
     nxp, nyp, nzp, nth = blk.nxp, blk.nyp, blk.nzp, blk.ntheta
     pk = api.pencil_key(nzp, nth)
     log.append(f"# workload {name}: {nxp}x{nyp}x{nzp}, {nth} angles, {job.nsim} realisations")
-    # pencil pass: the eigen form's tile and threads, then the general kernel's, then the form
-    eig_best = None
-    if nzp in (128, 256, 320):
-        api.tuning_set("pencil_kernel", pk, 2)
-        sweep(ctx, job, stream, reps, "pencil_w", pk, [1, 2, 4, 8], ["zpass"], log)
-        # the realisation batch at the widest tile (without realisation slots a wider tile
-        # may fit than with them); the width is swept again below
-        w_keep = api.tuning_get("pencil_w", pk)
-        api.tuning_set("pencil_w", pk, 8)
-        sweep(ctx, job, stream, reps, "pencil_sb", pk, [0, 1, 2, 4], ["zpass"], log)
-        api.tuning_set("pencil_w", pk, w_keep)
-        eig_best = sweep(ctx, job, stream, reps, "pencil_threads", pk, [64, 128, 256, 384, 512], ["zpass"], log)
-        # the tile width again, now with the realisation batch and threads chosen
-        sweep(ctx, job, stream, reps, "pencil_w", pk, [2, 4, 8], ["zpass"], log)
-        eig_best = sweep(ctx, job, stream, reps, "pencil_threads", pk, [128, 256, 512], ["zpass"], log)
-        # one or two bins of a z position per thread in the per-bin step
-        eig_best = sweep(ctx, job, stream, reps, "pencil_nb", pk, [1, 2], ["zpass"], log)
-        # the 80-register form: two CTAs of up to 384 threads per SM
-        if nth <= 6 and nzp in (256, 320):
-            keep_w, keep_t, keep_sb = (api.tuning_get(k, pk) for k in ("pencil_w", "pencil_threads", "pencil_sb"))
-            api.tuning_set("pencil_dense", pk, 1)
-            api.tuning_set("pencil_sb", pk, 1)
-            api.tuning_set("pencil_w", pk, 4)
-            dense_best = sweep(ctx, job, stream, reps, "pencil_threads", pk, [256, 320, 384], ["zpass"], log)
-            if dense_best and dense_best[1] < eig_best[1]:
-                eig_best = dense_best
-            else:
-                api.tuning_set("pencil_dense", pk, -1)
-                for k, v in (("pencil_w", keep_w), ("pencil_threads", keep_t), ("pencil_sb", keep_sb)):
-                    api.tuning_set(k, pk, v)
-    api.tuning_set("pencil_kernel", pk, 1)
-    sweep(ctx, job, stream, reps, "zpass_w", pk, [1, 2, 4], ["zpass"], log)
-    sweep(ctx, job, stream, reps, "zpass_sb", pk, [1, 2], ["zpass"], log)
-    gen_best = sweep(ctx, job, stream, reps, "zpass_threads", pk, [256, 512], ["zpass"], log)
-    if eig_best and (not gen_best or eig_best[1] <= gen_best[1]):
-        api.tuning_set("pencil_kernel", pk, 2)
-    for key in ("pencil_kernel", "pencil_w", "pencil_sb", "pencil_threads", "pencil_dense", "pencil_nb", "zpass_w",
-                "zpass_sb", "zpass_threads"):
-        v = api.tuning_get(key, pk)
-        if v >= 0:
-            entries[(key, pk)] = v
+    # pencil pass: the realisation batch and threads of every tile width; an entry is kept only
+    # where it beats the built-in shape (pencil_shape in pencil.cu), which also weighs the lateral size
+    base = time_classes(ctx, job, stream, reps).get("zpass", 0.0)
+    best = (base, {})
+    for w in (8, 4, 2):
+        for sb in sorted({1, min(2, max(1, job.nsim)), min(4, max(1, job.nsim))}):
+            api.tuning_set("pencil_w", pk, w)
+            api.tuning_set("pencil_sb", pk, sb)
+            b = sweep(ctx, job, stream, reps, "pencil_threads", pk, [128, 192, 256, 384, 512], ["zpass"], log)
+            if b and b[1] < 0.98 * best[0]:
+                best = (b[1], {"pencil_w": w, "pencil_sb": sb, "pencil_threads": b[0]})
+    for key in ("pencil_w", "pencil_sb", "pencil_threads"):
+        api.tuning_set(key, pk, best[1].get(key, -1))
+        if best[1]:
+            entries[(key, pk)] = best[1][key]
+    log.append(f"# pencil shape {pk}: built-in {base:.3f} ms, best {best[0]:.3f} ms")
     # four-step column (y) and row (x) transforms
     for key, tkey, cls in (("line4_w_fwd", "line4_threads_fwd", ["line_fwd"]),
                            ("line4_w_inv", "line4_threads_inv", ["line_inv"])):

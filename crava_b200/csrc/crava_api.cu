@@ -53,10 +53,10 @@ bool smooth(int n) {
   return n == 1;
 }
 
-// Stage radices for a length-n transform, fewest stages first: radix 16 while four
+// Stage radices for a length-n transform, fewest stages first: radix 16 (if allowed) while four
 // factors of two remain, then 8, 4 or 2 (a lone 2 pairs with a 3 into radix 6); pairs of
 // threes become radix 9; then 3, 5, 7.
-bool make_plan(int n, LinePlan& pl, bool allow16) {
+bool make_plan(int n, LinePlan& pl, bool allow16 = false) {
   if (!smooth(n)) return false;
   pl.n = n;
   pl.nst = 0;
@@ -68,7 +68,6 @@ bool make_plan(int n, LinePlan& pl, bool allow16) {
   auto push = [&](int r) { if (pl.nst < kMaxStages) pl.radix[pl.nst++] = (int8_t)r; };
   while (allow16 && a >= 4) { push(16); a -= 4; }
   while (a >= 3) { push(8); a -= 3; }
-  if (a == 3) { push(8); a = 0; }
   if (a == 2) { push(4); a = 0; }
   if (a == 1) {
     if (b > 0 && b % 2 == 1) { push(6); b--; }
@@ -343,8 +342,8 @@ crava_status get_xplans(crava_ctx* ctx, int nxp, Plan** px, Plan** pn) {
   return get_plan(ctx, nxp, pn);
 }
 
-// Plans are cached per (length, radix-16 allowed): the pencil pass has the register room
-// for radix-16 butterflies, the row and column passes run capped at 64 registers.
+// Plans are cached per (length, radix-16 allowed): the trace transforms (thick.cu) have the
+// register room for radix-16 butterflies, the row and column passes run capped at 64 registers.
 crava_status get_plan(crava_ctx* ctx, int n, Plan** out, bool allow16) {
   std::lock_guard<std::mutex> lk(ctx->mu);
   const int key = 2 * n + (allow16 ? 1 : 0);
@@ -630,12 +629,6 @@ void build_kz_tables(const crava_job_desc& d, std::vector<float2>& kw, std::vect
   }
 }
 
-// Four-step split of a z length that the in-place pencil kernels handle (kernels.cuh
-// ZParams.zsplit): 1 16x16, 2 20x16, 3 16x8; 0 for the other lengths.
-int zsplit_of(int nzp) { return nzp == 256 ? 1 : nzp == 320 ? 2 : nzp == 128 ? 3 : 0; }
-int zsplit_n1(int zs) { return zs == 1 ? 16 : zs == 2 ? 20 : zs == 3 ? 16 : 0; }
-int zsplit_n2(int zs) { return zs == 1 ? 16 : zs == 2 ? 16 : zs == 3 ? 8 : 0; }
-
 // Eigen tables of a separable-prior job: bytes on the device (0 for other priors).
 size_t eig_table_bytes(const crava_job_desc* d) {
   if (d->prior_mode != CRAVA_PRIOR_SEPARABLE) return 0;
@@ -703,10 +696,10 @@ void sep_constants(const std::vector<double>& A, const std::vector<double>& pv, 
   }
 }
 
-// Tables of the eigen form of the separable posterior (pencil.cu), one row per z position
-// in the order the in-place four-step transform leaves the spectrum in (position
-// k1 + N2 k2 holds kz = k2 + N1 k1), float4 group g of position p at rows[4 (g nzp + p)].
-// Per inverted kz, from the float values the general kernel uses (kw, M2 = the septab
+// Tables of the eigen form of the separable posterior (pencil.cuh), one row per z position
+// in the order the in-place z transform leaves the spectrum in (position p holds kz =
+// pencil_kz(p)), float4 group g of position p at rows[4 (g nzp + p)].
+// Per inverted kz, from the float values the Cholesky form uses (kw, M2 = the septab
 // lower triangle, ed, |ct|, G0 = A P0 A^T, AP = A P0):
 //   M = |ct| (kw kw^H) o G0 + M2,  E = diag(ed),  E^-1/2 M E^-1/2 = U diag(Lam) U^H,
 //   V = U^H E^-1/2,  Q = |ct| V diag(kw) AP,  H_l = conj(Q_la) Q_lb.
@@ -720,17 +713,16 @@ bool build_eig_tables(const crava_job_desc& d, const std::vector<float2>& kw, co
                       const float (&G0)[kMaxTheta][kMaxTheta], const float (&AP)[kMaxTheta][3], double& lam_limit,
                       std::vector<float>& rows, int& n_inv_rows, std::string& why) {
   lam_limit = INFINITY;
-  const int n = d.ntheta, nzp = d.nzp, zs = zsplit_of(nzp);
-  const int N1 = zsplit_n1(zs), N2 = zsplit_n2(zs);
+  const int n = d.ntheta, nzp = d.nzp;
+  ZPlan zplan;
+  if (!pencil_plan(nzp, zplan)) { why = "z length has no plan"; return false; }
   const EigLayout L(n);
   const int G4 = L.floats / 4;
   rows.assign((size_t)L.floats * nzp, 0.f);
   n_inv_rows = 0;
   const int tri = n * (n + 1) / 2;
   for (int p = 0; p < nzp; p++) {
-    // the in-place four-step order of k_pencil at its lengths, natural kz order otherwise
-    // (k_zpass)
-    const int kz = zs ? p / N2 + N1 * (p % N2) : p;
+    const int kz = pencil_kz(zplan, p);
     if (!inv[kz]) continue;
     n_inv_rows++;
     double row[4 * 96] = {};
@@ -2452,46 +2444,11 @@ crava_status crava_job_run(crava_job* job, void* stream) {
   }
   // the fused pencil pass
   Plan* pz;
-  const int skey = d.nzp * 16 + d.ntheta;   // schedule key of the pencil pass
-  if ((s = get_plan(ctx, d.nzp, &pz, tuned("zpass_r16", d.nzp, 1) != 0))) return s;
+  if ((s = get_plan(ctx, d.nzp, &pz))) return s;
   ZParams zp;
   std::memset(&zp, 0, sizeof(zp));
   zp.nxp = d.nxp; zp.nyp = d.nyp; zp.nzp = d.nzp; zp.cnxp = job->cnxp;
   zp.nxp_even = (d.nxp % 2) == 0;
-  // pencil tile: W x-bins (power of two), GT slots per z-transform call, SB realisations
-  // per batch and T threads.  Preferred: the widest tile (longest contiguous rows, fewest
-  // tiles) with every slot of a phase in one call (GT = G), the first of the candidates
-  // that fits; 512 threads when one CTA fills the SM's shared memory, 256 when two fit.
-  // CRAVA_ZPASS_{W,T,GT,SB} override.
-  const int Gs = std::max(d.ntheta + 3, 9);
-  int W = 2, T = 256, GT = Gs, SB = 2;
-  {
-    const int cand[8][3] = {{4, Gs, 2}, {4, Gs, 1}, {2, Gs, 2}, {2, Gs, 1}, {1, Gs, 2}, {4, 3, 1}, {2, 3, 1}, {1, 3, 1}};
-    for (const auto& c : cand) {
-      if (zpass_smem_bytes(c[0], d.nzp, d.ntheta, c[1], c[2]) <= 227 * 1024) {
-        W = c[0]; GT = c[1]; SB = c[2];
-        break;
-      }
-    }
-  }
-  W = std::max(1, tuned("zpass_w", skey, W));
-  GT = std::max(3, tuned("zpass_gt", skey, GT));
-  SB = std::max(1, tuned("zpass_sb", skey, SB));
-  SB = std::min(SB, GT / 3);
-  T = zpass_smem_bytes(W, d.nzp, d.ntheta, GT, SB) > 113 * 1024 ? 512 : 256;
-  T = std::max(64, std::min(512, tuned("zpass_threads", skey, T) / 32 * 32));
-  if (zpass_smem_bytes(W, d.nzp, d.ntheta, GT, SB) > 227 * 1024)
-    return fail(CRAVA_ENOTSUP, "pencil tile does not fit in shared memory");
-  zp.GT = GT;
-  zp.SB = SB;
-  zp.W = W;
-  {
-    const bool four = tuned("zpass_four", d.nzp, 1) != 0 && GT >= Gs;
-    zp.zsplit = !four ? 0 : d.nzp == 256 ? 1 : d.nzp == 320 ? 2 : d.nzp == 128 ? 3 : 0;
-  }
-  zp.logW = 0;
-  while ((1 << zp.logW) < W) zp.logW++;
-  zp.nIT = (job->cnxp + W - 1) / W;
   zp.nth = d.ntheta;
   zp.nsim = d.nsim;
   zp.separable = grids ? 0 : 1;
@@ -2529,49 +2486,20 @@ crava_status crava_job_run(crava_job* job, void* stream) {
     for (int m = 0; m < d.ntheta; m++) zp.ecd[l][m] = 0.5 * (1.0 - d.wnc) * job->etc[l * d.ntheta + m];
     zp.edd[l] = d.wnc * job->etc[l * d.ntheta + l];
   }
-  zp.zp = pz->lp;
   zp.twz = pz->tw;
   zp.seed = d.seed;
   zp.counters = job->counters;
-  int nl = 0;
-  if (job->eig_ok && zsplit_of(d.nzp) && tuned("pencil_kernel", skey, 2) == 2) {
-    // eigen form: in-place z transforms, W x-bins per tile (schedule keys pencil_w,
-    // pencil_threads); by default two CTAs per SM where the tile's shared memory allows
-    int Wp = 1;
-    while (Wp * 2 <= std::min(16, tuned("pencil_w", skey, 4))) Wp *= 2;
-    // realisations per transform batch; 0: no realisation slots (the mean is stored first and
-    // added back to each realisation), which lets wider tiles fit
-    int SBp = tuned("pencil_sb", skey, 1);
-    if (SBp != 0) SBp = std::max(1, std::min(std::max(d.nsim, 1), SBp));
-    while (SBp > 1 && pencil_smem_bytes(Wp, d.nzp, d.ntheta, SBp) > 227 * 1024) SBp--;
-    while (Wp > 1 && pencil_smem_bytes(Wp, d.nzp, d.ntheta, SBp) > 227 * 1024) Wp /= 2;
-    if (pencil_smem_bytes(Wp, d.nzp, d.ntheta, SBp) > 227 * 1024)
-      return fail(CRAVA_ENOTSUP, "pencil tile does not fit in shared memory");
-    zp.SB = SBp;
-    zp.dense = tuned("pencil_dense", skey, 0);
-    zp.nb2 = tuned("pencil_nb", skey, 1) == 2;
+  int nl = 0, threads = 0;
+  // the eigen form of the per-bin step where its tables apply (schedule key pencil_kernel: 1 keeps
+  // the Cholesky form)
+  if (job->eig_ok && tuned("pencil_kernel", d.nzp * 16 + d.ntheta, 2) == 2) {
     zp.eig = job->eig;
     zp.n_inv_rows = job->n_inv_rows;
-    zp.zsplit = zsplit_of(d.nzp);
-    zp.W = Wp;
-    zp.logW = 0;
-    while ((1 << zp.logW) < Wp) zp.logW++;
-    zp.nIT = (job->cnxp + zp.W - 1) / zp.W;
-    const int Tp = std::max(32, std::min(512, tuned("pencil_threads", skey,
-                                                    pencil_smem_bytes(Wp, d.nzp, d.ntheta, SBp) <= 113 * 1024 ? 256
-                                                                                                         : 512) /
-                                                   32 * 32));
+  }
+  if (!pencil_shape(zp, &threads)) return fail(CRAVA_ENOTSUP, "pencil tile does not fit in shared memory");
+  {
     ProfScope ps(ctx, KT_ZPASS, st);
-    CUDA_TRY(launch_pencil(zp, Tp, st, &nl));
-  } else {
-    // the general kernel takes the eigen form of the per-bin step where its tables apply
-    // (natural kz order at the lengths without the in-place split; schedule key zpass_eig)
-    if (job->eig_ok && !zsplit_of(d.nzp) && tuned("zpass_eig", d.nzp, 1) != 0) {
-      zp.eig = job->eig;
-      zp.n_inv_rows = job->n_inv_rows;
-    }
-    ProfScope ps(ctx, KT_ZPASS, st);
-    CUDA_TRY(launch_zpass(zp, T, st, &nl));
+    CUDA_TRY(launch_pencil(zp, threads, st, &nl));
   }
   ctx->launches += nl;
   // inverse transforms (y, x) of the outputs with FFTGrid::invFFTInPlace scales
@@ -3211,8 +3139,8 @@ struct HostPlan {
   std::vector<float2> tw;
 };
 
-bool host_plan(int n, bool allow16, HostPlan& hp) {
-  if (!make_plan(n, hp.lp, allow16)) return false;
+bool host_plan(int n, HostPlan& hp) {
+  if (!make_plan(n, hp.lp)) return false;
   hp.tw.resize(n);
   for (int t = 0; t < n; t++) {
     double ang = 2.0 * M_PI * (double)t / (double)n;
@@ -3251,8 +3179,8 @@ extern "C" crava_status crava_invert_noalloc(const crava_job_desc* desc, const f
   const size_t N = (size_t)d.nxp * d.nyp * d.nzp;
   const bool even = d.nxp % 2 == 0;
   HostPlan px, pn, py, pz;
-  if (!host_plan(even ? d.nxp / 2 : d.nxp, false, px) || !host_plan(d.nxp, false, pn) ||
-      !host_plan(d.nyp, false, py) || !host_plan(d.nzp, true, pz))
+  if (!host_plan(even ? d.nxp / 2 : d.nxp, px) || !host_plan(d.nxp, pn) || !host_plan(d.nyp, py) ||
+      !host_plan(d.nzp, pz))
     return fail(CRAVA_ENOTSUP, "transform length is not 2,3,5,7-smooth");
 
   // scratch layout: data work grids, twiddle tables, per-kz tables, lateral and temporal
@@ -3336,14 +3264,6 @@ extern "C" crava_status crava_invert_noalloc(const crava_job_desc* desc, const f
   std::memset(&zp, 0, sizeof(zp));
   zp.nxp = d.nxp; zp.nyp = d.nyp; zp.nzp = d.nzp; zp.cnxp = cnxp;
   zp.nxp_even = even;
-  int W = 4, T = 256;
-  if (zpass_smem_bytes(W, d.nzp, d.ntheta) > 113 * 1024) T = 512;
-  while (W > 1 && zpass_smem_bytes(W, d.nzp, d.ntheta) > 227 * 1024) W /= 2;
-  if (zpass_smem_bytes(W, d.nzp, d.ntheta) > 227 * 1024) return fail(CRAVA_ENOTSUP, "pencil tile does not fit in shared memory");
-  zp.W = W;
-  zp.logW = 0;
-  while ((1 << zp.logW) < W) zp.logW++;
-  zp.nIT = (cnxp + W - 1) / W;
   zp.nth = d.ntheta;
   zp.nsim = d.nsim;
   zp.separable = 1;
@@ -3365,11 +3285,12 @@ extern "C" crava_status crava_invert_noalloc(const crava_job_desc* desc, const f
   zp.kz.e2 = (const float2*)(base + o_e2);
   zp.kz.inv = (const uint8_t*)(base + o_inv);
   zp.kz.ed = (const float*)(base + o_ed);
-  zp.zp = pz.lp;
   zp.twz = twz;
   zp.seed = d.seed;
   zp.counters = (unsigned long long*)(base + o_cnt);
-  CUDA_TRY(launch_zpass(zp, T, st, nullptr));
+  int threads = 0;
+  if (!pencil_shape(zp, &threads)) return fail(CRAVA_ENOTSUP, "pencil tile does not fit in shared memory");
+  CUDA_TRY(launch_pencil(zp, threads, st, nullptr));
   // inverse y, x transforms of the outputs in place
   {
     GridSet gs;
@@ -3411,8 +3332,7 @@ crava_status prewarm_plans(crava_ctx* ctx, const crava_job_desc& d) {
   crava_status s;
   if ((s = get_xplans(ctx, d.nxp, &a, &b))) return s;
   if ((s = get_plan(ctx, d.nyp, &a))) return s;
-  if ((s = get_plan(ctx, d.nzp, &a))) return s;
-  return get_plan(ctx, d.nzp, &a, tuned("zpass_r16", d.nzp, 1) != 0);
+  return get_plan(ctx, d.nzp, &a);
 }
 
 }  // namespace

@@ -5,7 +5,7 @@
 //   k_x_c2r      inverse along x: half spectrum -> real, scaled (last pass of
 //                FFTGrid::invFFTInPlace, src/fftgrid.cpp:1615-1643)
 //   k_line_fft   complex transform along a strided axis (y, or z for prior grids)
-//   (the fused pencil pass is in zpass.cu)
+//   (the fused pencil pass is in pencil.cuh)
 #include <cuda_runtime.h>
 #include <stdint.h>
 

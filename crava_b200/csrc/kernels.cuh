@@ -41,11 +41,23 @@ struct KzTables {
   const double* edd;    //   thickness); edd in double, null: the per-angle constants edd
 };
 
+// z transform plan of the pencil pass: nzp as a product of radices up to 20, stage by stage.
+struct ZPlan {
+  int n, ns;
+  int8_t radix[10];
+};
+bool pencil_plan(int n, ZPlan& z);
+// kz at position p of a line after the forward stages (in place, digits reversed)
+int pencil_kz(const ZPlan& z, int p);
+
 struct ZParams {
   int nxp, nyp, nzp, cnxp;
-  int W, logW, nIT;            // tile width in x-bins (power of two), log2 W, tiles per x-row
-  int GT, SB;                  // slots per z-transform call, realisations per batch (3 SB <= GT)
-  int zsplit;                  // four-step z transform: 0 none, 1 16x16, 2 20x16, 3 16x8
+  int W, NP, logNP, nIT;       // tile width in x-bins (power of two >= 2), pairs W / 2, tiles per x-row
+  int SB;                      // realisations per batch
+  int D, PS, swz;              // tile layout (pencil.cuh): slot of the diagonal, bytes per position,
+                               // positions swapped within fours in the per-bin steps
+  int vec;                     // 1: pairs of bins move as 16-byte words
+  ZPlan z;
   int nth, nsim;
   int separable;               // 1: prior from cxy/ct factors, 0: from spectral grids
   int base_prior;              // grids: the six prior spectra are pv x one base spectrum, only
@@ -70,19 +82,16 @@ struct ZParams {
   float G0[kMaxTheta][kMaxTheta];  // SEPARABLE: A P0 A^T
   float AP[kMaxTheta][3];          // SEPARABLE: A P0
   KzTables kz;
-  LinePlan zp;
   const float2* twz;
   uint64_t seed;
   float fp64_threshold;            // > 0: re-factorise flagged bins in FP64
   double Ad[kMaxTheta][3];         // A, ec, ed in double for that path
   double ecd[kMaxTheta][kMaxTheta];
   double edd[kMaxTheta];
-  // eigen form of the separable posterior (pencil.cu): per-position rows of the per-kz
-  // tables, float4 group g of position p at eig[g * nzp + p]; null for the general kernel
+  // eigen form of the separable posterior (pencil.cuh): per-position rows of the per-kz
+  // tables, float4 group g of position p at eig[g * nzp + p]; null: the Cholesky form
   const float4* eig;
   int n_inv_rows;                  // inverted kz (counted per tile, not per bin)
-  int dense;                       // 1: the 80-register instantiation (two CTAs per SM)
-  int nb2;                         // 1: two bins of one z position per thread in the per-bin step
   unsigned long long* counters;    // [0] inverted bins [1] chol fallbacks [2] zero sim bins
                                    // [3] bins re-factorised in FP64 [4] pencil tiles whose
                                    // input spectra are not finite
@@ -242,9 +251,10 @@ cudaError_t launch_x_c2r(const GridSet& gs, int nxp, int rows, const LinePlan& p
 //   0 <= i < ni (contiguous), 0 <= p < n (the transform axis), 0 <= o < no.
 cudaError_t launch_line_fft(const GridSet& gs, int ni, int n, size_t pstride, int no, size_t ostride,
                             const LinePlan& pl, const float2* tw, float sign, cudaStream_t st, int* nlaunch);
-cudaError_t launch_zpass(const ZParams& zp, int threads, cudaStream_t st, int* nlaunch);
-// pencil.cu: the separable-prior pencil pass in its eigen form, for the four-step z lengths
-// (zp.zsplit 1..3); zp.eig from build_eig_tables
+// pencil.cu: the pencil pass.  pencil_shape sets zp's tile (W .. swz, nIT) and the threads per CTA
+// from nzp, nth, nsim and the lateral size (schedule keys pencil_w, pencil_sb, pencil_threads, n =
+// nzp * 16 + nth); false when no tile fits in shared memory.
+bool pencil_shape(ZParams& zp, int* threads);
 cudaError_t launch_pencil(const ZParams& zp, int threads, cudaStream_t st, int* nlaunch);
 size_t pencil_smem_bytes(int W, int nzp, int nth, int SB);
 // Float layout of one position's row of the eigen tables: kw (2n floats), Lam (n), then per
@@ -262,8 +272,6 @@ struct EigLayout {
     floats = rows + n * rs;
   }
 };
-size_t zpass_smem_bytes(int W, int nzp, int nth);                  // GT = 3, SB = 1
-size_t zpass_smem_bytes(int W, int nzp, int nth, int GT, int SB);
 // facies.cu: prior[] and out[] are host arrays (copied into the launch parameters)
 cudaError_t launch_spec_mul(float2* a, const float2* b, size_t n, cudaStream_t st);
 // gridio.cu: dst[e] = src[e] with the byte order of every 4-byte word reversed (dst == src

@@ -1,14 +1,13 @@
-// The separable-prior pencil pass in its eigen form (sm_100a).
+// The pencil pass (sm_100a).
 //
-// Per (x-tile, y) pencil, like k_zpass (zpass.cu): forward z transform of the data and
-// prior-mean spectra, the per-bin posterior of AVOInversion::computePostMeanResidAndFFTCov
-// (src/avoinversion.cpp:944-1091), the realisations of AVOInversion::simulate
-// (src/avoinversion.cpp:1401-1511) and the inverse z transform of every output spectrum,
-// with the spectra kept on chip between the two transforms.
+// Per (x-tile, y) pencil: forward z transform of the data and prior-mean spectra, the per-bin
+// posterior of AVOInversion::computePostMeanResidAndFFTCov (src/avoinversion.cpp:944-1091), the
+// realisations of AVOInversion::simulate (src/avoinversion.cpp:1401-1511) and the inverse z
+// transform of every output spectrum, with the spectra kept on chip between the two transforms.
 //
-// The per-bin algebra.  With a separable prior whose temporal factor has a real spectrum
-// (a symmetric circular correlation, as SeismicParametersHolder::computeCircCorrT builds it,
-// src/seismicparametersholder.cpp:624-660), every bin of one kz has the data covariance
+// The per-bin algebra, eigen form.  With a separable prior whose temporal factor has a real
+// spectrum (a symmetric circular correlation, as SeismicParametersHolder::computeCircCorrT builds
+// it, src/seismicparametersholder.cpp:624-660), every bin of one kz has the data covariance
 //     Sd = lam M_k + E_k,   M_k = |ct_k| (kw kw^H) o G0 + M2_k,   E_k = diag(ed_k) > 0,
 // with lam = |Re corrXY-spectrum(i, j)| the only lateral variable, and K S = lam |ct_k|
 // diag(kw) A P0.  From the Hermitian eigen-decomposition E^-1/2 M_k E^-1/2 = U diag(Lam) U^H
@@ -19,473 +18,905 @@
 // which equals the reference's Sd^-1 regrouping exactly in exact arithmetic: a few small
 // matrix-vector products per bin instead of a per-bin Cholesky factorisation and solves.
 // Sd is positive definite for every lam >= 0 (Sd >= E_k), so the reference's Cholesky
-// never falls back here; the host checks that before it chooses this kernel.
+// never falls back here; the host checks that before it chooses this form.  Elsewhere the bins
+// take the Cholesky form of pencil_bin.cuh.
 //
-// The z transforms run in place: the forward four-step transform leaves kz = k2 + N1 k1 at
-// position k1 + N2 k2 (no scratch buffer), the per-bin step reads its tables in that
-// position order, and the inverse transform takes that order back to natural order.  With
-// no transform scratch the tile needs (G + 3) slots of W x nzp complex values, so two CTAs
-// share an SM at nzp = 256 with one realisation per batch.
+// Pairs.  Everything is done for two neighbouring x-bins at once (C2, fft_pair.cuh): the tile holds
+// the bins 2 q and 2 q + 1 of a line as {re, re', im, im'}, one 16-byte word, so the transforms, the
+// per-bin products and the realisations are packed FP32 instructions and their shared-memory
+// accesses 16-byte ones.  Where the z stride is an even number of bins and the grids are 16-byte
+// aligned (P.vec), the tiles of a row that starts on an odd bin begin one bin early, so that every
+// pair is one 16-byte global access; elsewhere pairs move as two 8-byte ones.
+//
+// The z transforms run in place with any split of nzp into radices up to 20: stage s of the
+// forward transform leaves the digits of kz reversed (position p holds kz = pencil_kz(p)), the
+// per-bin step reads its tables in position order, and the inverse stages take that order back to
+// natural order, the last one storing to global memory.  The stages are separate functions, one per
+// radix, so that every length shares them and the kernel is instantiated by angle count alone.
+//
+// The diagonal of S_post is real: the pair's second bin goes into the imaginary part of the first
+// one's line, which halves its share of the inverse transform (9 output spectra cost 7.5 lines) and
+// of the tile; the two are told apart after the transform by S(z) = conj S(-z).
+//
+// What bounds it: issue slots and their latency, not HBM -- see the table of figures in the launcher.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include "fft2.cuh"
-#include "fft_core.cuh"
+#include "fft_pair.cuh"
 #include "kernels.cuh"
+#include "pencil_bin.cuh"
 #include "pencil_common.cuh"
 
 namespace crava {
 
-// ------------------------------------------------------------------ in-place z transforms
+// ------------------------------------------------------------------ z transforms in place
+//
+// Line l of nl at byte base + 16 l (+ gap from line split on), its point p ps bytes further.  A
+// stage of radix R works on blocks of R sub points: v[m] at b R sub + t + sub m, t < sub.
+//   forward (DIR -1): DFT over m, times w^(t k) (w = e^{-2 pi i / (R sub)}), back to sub k
+//   inverse (DIR +1): times conj w^(t k), DFT over k, back to sub m
+// tw: the table of e^{-2 pi i t / n}, so w = tw[tws], tws = n / (R sub).  AOS: the points come as
+// {re, im, re', im'} (the way the input copies leave them).
+constexpr int even_up_z(int n) { return (n + 1) & ~1; }
 
-// Forward transform of nl lines (line l at x + l, point p at x + l + p ps) of length
-// N1 N2, natural order in, position k1 + N2 k2 <- X[k2 + N1 k1] out.
-template <int N1, int N2>
-__device__ __forceinline__ void zfwd_inplace(float2* x, int nl, int ps, const float2* tw) {
-  const int T = blockDim.x;
-  const float rl = __frcp_rn((float)nl);
-  const int mstep = N2 * ps;
-  // pass 1, item t < N2: N1-point DFT over positions t + N2 m, twiddle w^(t k2), back to
-  // positions t + N2 k2
-  for (int q = threadIdx.x; q < nl * N2; q += T) {
-    int l;
-    const int t = fdivmod(q, nl, rl, l);
-    float2* y = x + l + t * ps;
-    four_step_pass1<N1, N2, -1>(
-        t, tw, [&](int, int m) { return y[m * mstep]; }, [&](int, int k2, float2 v) { y[k2 * mstep] = v; });
-  }
-  __syncthreads();
-  // pass 2, item k2 < N1: N2-point DFT over the run t + N2 k2 (t < N2), X[k2 + N1 k1] back to
-  // position k1 + N2 k2
-  for (int q = threadIdx.x; q < nl * N1; q += T) {
-    int l;
-    const int k2 = fdivmod(q, nl, rl, l);
-    float2* y = x + l + k2 * mstep;
-    float2 v[N2];
+struct ZStage {
+  uint32_t base, tw;
+  int nl, ps, split, gap, items, sub, tws;
+};
+
+template <int R, int DIR>
+__device__ __forceinline__ void z_twiddle(C2 (&v)[R], uint32_t tw, int step) {
 #pragma unroll
-    for (int t = 0; t < N2; t++) v[t] = y[t * ps];
-    Dft<N2>::run(v, -1.f);
-#pragma unroll
-    for (int k1 = 0; k1 < N2; k1++) y[k1 * ps] = v[k1];
+  for (int k = 1; k < R; k++) {
+    const float2 w = lds2(tw + 8u * (uint32_t)(step * k));
+    v[k] = c2_mul(v[k], w.x, DIR < 0 ? w.y : -w.y);
   }
-  __syncthreads();
 }
 
-// Inverse transform (unnormalised, e^{+2 pi i}) of nl lines holding X[k2 + N1 k1] at position
-// k1 + N2 k2; natural order out:
-//   x[t + N2 m] = sum_k2 w1^(-m k2) w^(-t k2) sum_k1 w2^(-t k1) X[k2 + N1 k1].
-template <int N1, int N2>
-__device__ __forceinline__ void zinv_inplace(float2* x, int nl, int ps, const float2* tw) {
-  const int T = blockDim.x;
-  const float rl = __frcp_rn((float)nl);
-  const int mstep = N2 * ps;
-  // pass A, item k2 < N1: N2-point inverse DFT over the run k1 + N2 k2, twiddle w^(-t k2),
-  // back to positions t + N2 k2
-  for (int q = threadIdx.x; q < nl * N1; q += T) {
-    int l;
-    const int k2 = fdivmod(q, nl, rl, l);
-    float2* y = x + l + k2 * mstep;
-    float2 v[N2];
+__device__ __forceinline__ uint32_t z_line(const ZStage& a, int l) {
+  return a.base + 16u * (uint32_t)l + (l >= a.split ? (uint32_t)a.gap : 0u);
+}
+
+// one item of a stage: R points from byte ad on, st bytes apart; tstep: t tws, or 0
+template <int R, int DIR, bool AOS>
+__device__ __forceinline__ void z_load(C2 (&v)[R], uint32_t ad, uint32_t st) {
 #pragma unroll
-    for (int k1 = 0; k1 < N2; k1++) v[k1] = y[k1 * ps];
-    Dft<N2>::run(v, 1.f);
-#pragma unroll
-    for (int t = 1; t < N2; t++) {
-      float2 w = tw[t * k2];   // t k2 < N1 N2
-      v[t] = cmul(v[t], make_float2(w.x, -w.y));
+  for (int m = 0; m < R; m++) {
+    if constexpr (AOS) {
+      const float4 x = lds4(ad + m * st);
+      v[m] = {make_float2(x.x, x.z), make_float2(x.y, x.w)};
+    } else {
+      v[m] = lds_c2(ad + m * st);
     }
-#pragma unroll
-    for (int t = 0; t < N2; t++) y[t * ps] = v[t];
   }
-  __syncthreads();
-  // pass B, item t < N2: N1-point inverse DFT over positions t + N2 k2, natural order back
-  for (int q = threadIdx.x; q < nl * N2; q += T) {
-    int l;
-    const int t = fdivmod(q, nl, rl, l);
-    float2* y = x + l + t * ps;
-    float2 v[N1];
+}
+template <int R, int DIR, bool AOS, bool TW>
+__device__ __forceinline__ void z_item(uint32_t ad, uint32_t st, uint32_t tw, int tstep) {
+  C2 v[R];
+  z_load<R, DIR, AOS>(v, ad, st);
+  if (DIR > 0 && TW) z_twiddle<R, DIR>(v, tw, tstep);
+  DftP<R, DIR>::run(v);
+  if (DIR < 0 && TW) z_twiddle<R, DIR>(v, tw, tstep);
 #pragma unroll
-    for (int k2 = 0; k2 < N1; k2++) v[k2] = y[k2 * mstep];
-    Dft<N1>::run(v, 1.f);
-#pragma unroll
-    for (int m = 0; m < N1; m++) y[m * mstep] = v[m];
-  }
-  __syncthreads();
+  for (int m = 0; m < R; m++) sts_c2(ad + m * st, v[m]);
 }
 
-// The same inverse transform with its last pass writing each line's natural-order outputs
-// straight out through store(l, k, value) (line l, z index k) instead of back to x; x is
-// free for reuse after the closing barrier.
-template <int N1, int N2, class Store>
-__device__ __forceinline__ void zinv_store(float2* x, int nl, int ps, const float2* tw, Store store) {
-  const int T = blockDim.x;
-  const float rl = __frcp_rn((float)nl);
-  const int mstep = N2 * ps;
-  for (int q = threadIdx.x; q < nl * N1; q += T) {
-    int l;
-    const int k2 = fdivmod(q, nl, rl, l);
-    float2* y = x + l + k2 * mstep;
-    float2 v[N2];
-#pragma unroll
-    for (int k1 = 0; k1 < N2; k1++) v[k1] = y[k1 * ps];
-    Dft<N2>::run(v, 1.f);
-#pragma unroll
-    for (int t = 1; t < N2; t++) {
-      float2 w = tw[t * k2];
-      v[t] = cmul(v[t], make_float2(w.x, -w.y));
-    }
-#pragma unroll
-    for (int t = 0; t < N2; t++) y[t * ps] = v[t];
+template <int R, int DIR, bool AOS>
+__device__ __noinline__ void z_stage(ZStage a) {
+  const float rl = __frcp_rn((float)a.nl), rs = __frcp_rn((float)a.sub);
+  const uint32_t st = (uint32_t)(a.sub * a.ps);
+  for (int q = threadIdx.x; q < a.items; q += blockDim.x) {
+    int l, t;
+    const int j = fdivmod(q, a.nl, rl, l);
+    const int b = fdivmod(j, a.sub, rs, t);
+    const uint32_t ad = z_line(a, l) + (uint32_t)((b * R * a.sub + t) * a.ps);
+    if (a.sub > 1) z_item<R, DIR, AOS, true>(ad, st, a.tw, t * a.tws);
+    else z_item<R, DIR, AOS, false>(ad, st, a.tw, 0);
   }
-  __syncthreads();
-  for (int q = threadIdx.x; q < nl * N2; q += T) {
-    int l;
-    const int t = fdivmod(q, nl, rl, l);
-    const float2* y = x + l + t * ps;
-    float2 v[N1];
-#pragma unroll
-    for (int k2 = 0; k2 < N1; k2++) v[k2] = y[k2 * mstep];
-    Dft<N1>::run(v, 1.f);
-#pragma unroll
-    for (int m = 0; m < N1; m++) store(l, t + N2 * m, v[m]);
-  }
-  __syncthreads();
 }
 
-// ------------------------------------------------------------------ per-bin algebra
-
-// Writes one bin's results into its slots: the residual (KEEP_RESIDUAL, at global index
-// gidx), S_post's realisation factor (lib_matrCholCpx(3), simulate :1425-1443) in slots 0..5
-// with slot 0's imaginary part -1 as the mark, or S_post itself where that factorisation
-// fails, and mu_post in slots 6..8.  Returns 1 for a bin whose realisations stay zero.
-template <int NTH>
-__device__ __forceinline__ int store_bin(const ZParams& P, float2* slot, int W, const float2 (&d)[NTH],
-                                         const float2 (&mp)[3], const float2 (&sp)[6], size_t gidx) {
-  if (P.keep_resid) {
+// The last inverse stage (one block, sub = n / R): lines below split leave for global memory in
+// natural order -- line l is slot l / NP, pair l % NP, and goes to out[slot] + base + k kstride at
+// its two x-offsets, those in [wlo, nw) -- the others stay in place.
+struct ZOut {
+  uint32_t out;          // shared-memory address of the slots' grid pointers
+  size_t base, kstride;
+  int wlo, nw, logNP, vec;
+};
+// item t of line l; gs: global stride between its outputs
+template <int R, bool TW>
+__device__ __forceinline__ void z_last_item(const ZStage& a, const ZOut& o, int l, int t, uint32_t st, size_t gs) {
+  const uint32_t ad = z_line(a, l) + (uint32_t)(t * a.ps);
+  C2 v[R];
+  z_load<R, 1, false>(v, ad, st);
+  if (TW) z_twiddle<R, 1>(v, a.tw, t * a.tws);
+  DftP<R, 1>::run(v);
+  if (l >= a.split) {
 #pragma unroll
-    for (int l = 0; l < NTH; l++) P.data[l][gidx] = d[l];
+    for (int m = 0; m < R; m++) sts_c2(ad + m * st, v[m]);
+    return;
   }
-  float2 C[3][3];
-  C[0][0] = sp[0]; C[1][1] = sp[1]; C[2][2] = sp[2];
-  C[0][1] = sp[3]; C[0][2] = sp[4]; C[1][2] = sp[5];
-  C[1][0] = make_float2(sp[3].x, -sp[3].y);
-  C[2][0] = make_float2(sp[4].x, -sp[4].y);
-  C[2][1] = make_float2(sp[5].x, -sp[5].y);
-  int zero = 0;
-  if (P.nsim > 0 && chol_ref<3>(C)) {
-    slot[0] = make_float2(C[0][0].x, -1.f);
-    slot[W] = make_float2(C[1][1].x, 0.f);
-    slot[2 * W] = make_float2(C[2][2].x, 0.f);
-    slot[3 * W] = C[1][0];
-    slot[4 * W] = C[2][0];
-    slot[5 * W] = C[2][1];
+  const int w = 2 * (l & ((1 << o.logNP) - 1));
+  unsigned long long gp;
+  asm volatile("ld.shared.u64 %0, [%1];" : "=l"(gp) : "r"(o.out + 8u * (uint32_t)(l >> o.logNP)));
+  float2* g = reinterpret_cast<float2*>(gp) + o.base + (size_t)t * o.kstride + w;
+  const bool in0 = w >= o.wlo && w < o.nw, in1 = w + 1 < o.nw;
+  if (o.vec && in0 && in1) {
+#pragma unroll
+    for (int m = 0; m < R; m++, g += gs)
+      *reinterpret_cast<float4*>(g) = make_float4(v[m].r.x, v[m].i.x, v[m].r.y, v[m].i.y);
   } else {
-    if (P.nsim > 0) zero = 1;
 #pragma unroll
-    for (int q = 0; q < 6; q++) slot[q * W] = sp[q];
+    for (int m = 0; m < R; m++, g += gs) {
+      if (in0) g[0] = make_float2(v[m].r.x, v[m].i.x);
+      if (in1) g[1] = make_float2(v[m].r.y, v[m].i.y);
+    }
   }
-#pragma unroll
-  for (int a = 0; a < 3; a++) slot[(6 + a) * W] = mp[a];
-  return zero;
+}
+template <int R>
+__device__ __noinline__ void z_last(ZStage a, ZOut o) {
+  const float rl = __frcp_rn((float)a.nl);
+  const uint32_t st = (uint32_t)(a.sub * a.ps);
+  const size_t gs = (size_t)a.sub * o.kstride;
+  for (int q = threadIdx.x; q < a.items; q += blockDim.x) {
+    int l;
+    const int t = fdivmod(q, a.nl, rl, l);
+    if (a.sub > 1) z_last_item<R, true>(a, o, l, t, st, gs);
+    else z_last_item<R, false>(a, o, l, t, st, gs);
+  }
 }
 
-// S_post = L L^H of a bin whose slots 0..5 hold its realisation factor (written back there).
-// The products and sums are spelled out as explicit fused multiply-adds so that every call site
-// rounds them alike (the two realisation forms call it from different code).
-__device__ __forceinline__ void store_llh(float2* slot, int W, float2 l0, float2 l1, float2 l2, float2 l10,
-                                          float2 l20, float2 l21) {
-  slot[0] = make_float2(__fmul_rn(l0.x, l0.x), 0.f);
-  slot[W] = make_float2(__fmaf_rn(l10.x, l10.x, __fmaf_rn(l10.y, l10.y, __fmul_rn(l1.x, l1.x))), 0.f);
-  slot[2 * W] = make_float2(
-      __fmaf_rn(l20.x, l20.x,
-                __fmaf_rn(l20.y, l20.y, __fmaf_rn(l21.x, l21.x, __fmaf_rn(l21.y, l21.y, __fmul_rn(l2.x, l2.x))))),
-      0.f);
-  slot[3 * W] = make_float2(__fmul_rn(l0.x, l10.x), -__fmul_rn(l0.x, l10.y));
-  slot[4 * W] = make_float2(__fmul_rn(l0.x, l20.x), -__fmul_rn(l0.x, l20.y));
-  slot[5 * W] = make_float2(__fmaf_rn(l10.x, l20.x, __fmaf_rn(l10.y, l20.y, __fmul_rn(l1.x, l21.x))),
-                            __fmaf_rn(l10.y, l20.x, __fmaf_rn(-l10.x, l20.y, -__fmul_rn(l1.x, l21.y))));
+#define CRAVA_Z_RADICES(X) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(12) X(14) X(15) X(16) X(18) X(20)
+
+template <int DIR, bool AOS>
+__device__ __forceinline__ void z_stage_any(int R, const ZStage& a) {
+  switch (R) {
+#define CRAVA_CASE(RR) \
+  case RR: z_stage<RR, DIR, AOS>(a); break;
+    CRAVA_Z_RADICES(CRAVA_CASE)
+#undef CRAVA_CASE
+  }
+}
+__device__ __forceinline__ void z_last_any(int R, const ZStage& a, const ZOut& o) {
+  switch (R) {
+#define CRAVA_CASE(RR) \
+  case RR: z_last<RR>(a, o); break;
+    CRAVA_Z_RADICES(CRAVA_CASE)
+#undef CRAVA_CASE
+  }
+}
+
+// All stages; the caller synchronises before, every stage ends with a barrier.  R0 = 0: any plan, one
+// call per stage; R0 x R1: that split inlined, its strides constants (256 points, 5 angles, 4
+// realisations: about 300 of 2570 instructions a bin are the calls' own).
+static __device__ __noinline__ void z_forward_any(const ZPlan& z, ZStage a) {
+  int len = z.n;
+  for (int s = 0; s < z.ns; s++) {
+    const int R = z.radix[s];
+    a.sub = len / R;
+    a.tws = z.n / len;
+    a.items = a.nl * (z.n / R);
+    if (s == 0) z_stage_any<-1, true>(R, a);
+    else z_stage_any<-1, false>(R, a);
+    len = a.sub;
+    __syncthreads();
+  }
+}
+// the last stage stores the lines below split through o
+static __device__ __noinline__ void z_inverse_any(const ZPlan& z, ZStage a, const ZOut& o) {
+  int len = 1;
+  for (int s = z.ns - 1; s >= 0; s--) {
+    const int R = z.radix[s];
+    a.sub = len;
+    len *= R;
+    a.tws = z.n / len;
+    a.items = a.nl * (z.n / R);
+    if (s > 0) z_stage_any<1, false>(R, a);
+    else z_last_any(R, a, o);
+    __syncthreads();
+  }
+}
+template <int R0, int R1>
+__device__ __forceinline__ void z_forward(const ZPlan& z, ZStage a) {
+  if constexpr (R0 == 0) {
+    z_forward_any(z, a);
+  } else {
+    const float rl = __frcp_rn((float)a.nl);
+    const int ps = a.ps;
+#pragma unroll 1
+    for (int q = threadIdx.x; q < a.nl * R1; q += blockDim.x) {
+      int l;
+      const int t = fdivmod(q, a.nl, rl, l);
+      z_item<R0, -1, true, true>(z_line(a, l) + (uint32_t)(t * ps), (uint32_t)(R1 * ps), a.tw, t);
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int q = threadIdx.x; q < a.nl * R0; q += blockDim.x) {
+      int l;
+      const int b = fdivmod(q, a.nl, rl, l);
+      z_item<R1, -1, false, false>(z_line(a, l) + (uint32_t)(b * R1 * ps), (uint32_t)ps, a.tw, 0);
+    }
+    __syncthreads();
+  }
+}
+template <int R0, int R1>
+__device__ __forceinline__ void z_inverse(const ZPlan& z, ZStage a, const ZOut& o) {
+  if constexpr (R0 == 0) {
+    z_inverse_any(z, a, o);
+  } else {
+    const float rl = __frcp_rn((float)a.nl);
+    const int ps = a.ps;
+    a.tws = 1;
+#pragma unroll 1
+    for (int q = threadIdx.x; q < a.nl * R0; q += blockDim.x) {
+      int l;
+      const int b = fdivmod(q, a.nl, rl, l);
+      z_item<R1, 1, false, false>(z_line(a, l) + (uint32_t)(b * R1 * ps), (uint32_t)ps, a.tw, 0);
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int q = threadIdx.x; q < a.nl * R1; q += blockDim.x) {
+      int l;
+      const int t = fdivmod(q, a.nl, rl, l);
+      z_last_item<R0, true>(a, o, l, t, (uint32_t)(R1 * ps), (size_t)R1 * o.kstride);
+    }
+    __syncthreads();
+  }
+}
+
+// kz at position p after the forward stages
+__device__ __forceinline__ int pencil_kz_dev(const ZPlan& z, int p) {
+  int kz = 0, mul = 1, len = z.n;
+  for (int s = 0; s < z.ns; s++) {
+    len /= z.radix[s];
+    const int d = p / len;
+    p -= d * len;
+    kz += mul * d;
+    mul *= z.radix[s];
+  }
+  return kz;
+}
+
+// ------------------------------------------------------------------ per-bin algebra, eigen form
+
+constexpr int pad4(int x) { return (x + 3) / 4 * 4; }
+
+// Section of N floats (N % 4 == 0) of the row of position p: group g at e[g * stride].
+template <int N>
+__device__ __forceinline__ void ldrow(float (&out)[N], const float4* __restrict__ e, int stride) {
+#pragma unroll
+  for (int g = 0; g < N / 4; g++) {
+    const float4 v = __ldg(e + g * stride);
+    out[4 * g] = v.x;
+    out[4 * g + 1] = v.y;
+    out[4 * g + 2] = v.z;
+    out[4 * g + 3] = v.w;
+  }
+}
+
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// A pair of bins between the posterior and the realisations: mu_post, and S_post as its real
+// diagonal 00 11 22 and its entries 01 02 12.
+struct PairPost {
+  C2 mu[3];
+  float2 sd[3];
+  C2 so[3];
+};
+
+// am = A_l mu
+__device__ __forceinline__ C2 a_mu(const ZParams& P, int l, const C2 (&m)[3]) {
+  return c2_fma(P.A[l][2], m[2], c2_fma(P.A[l][1], m[1], c2_scale(m[0], P.A[l][0])));
+}
+// x - kw y
+__device__ __forceinline__ C2 c2_submul(C2 x, float kr, float ki, C2 y) {
+  return {f2_fma(f2_dup(ki), y.i, f2_fma(f2_dup(-kr), y.r, x.r)),
+          f2_fma(f2_dup(-ki), y.r, f2_fma(f2_dup(-kr), y.i, x.i))};
+}
+
+// mu_post and S_post of the two bins of one z position from that position's row e (float4 groups
+// at stride nzp, laid out as EigLayout: the angles' rows are streamed one at a time), and with
+// RES the residuals in d.
+template <int NTH>
+__device__ __forceinline__ void pair_posterior_eig(const ZParams& P, const float4* __restrict__ e, float2 lam,
+                                                   float2 rho, const C2 (&mu)[3], C2 (&d)[NTH], PairPost& o) {
+  constexpr int VP = pad4(2 * NTH), OKW = 0, OL = VP, OR = OL + pad4(NTH), RS = VP + 16;
+  const int st = P.nzp;
+  float Lm[pad4(NTH)];
+  ldrow(Lm, e + (OL / 4) * st, st);
+  {
+    float kw[VP];
+    ldrow(kw, e + (OKW / 4) * st, st);
+    // d <- y = d - K mu, K = diag(kw) A
+#pragma unroll
+    for (int l = 0; l < NTH; l++) d[l] = c2_submul(d[l], kw[2 * l], kw[2 * l + 1], a_mu(P, l, mu));
+  }
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    o.mu[a] = mu[a];
+    o.sd[a] = f2_mul(rho, f2_dup(P.pv[a]));
+    o.so[a] = {f2_mul(rho, f2_dup(P.pv[3 + a])), make_float2(0.f, 0.f)};
+  }
+#pragma unroll
+  for (int l = 0; l < NTH; l++) {
+    // r_l = (V y)_l, s_l = r_l lam / (lam Lam_l + 1), w_l = lam^2 / (lam Lam_l + 1)
+    float V[VP];
+    ldrow(V, e + ((OR + l * RS) / 4) * st, st);
+    float QH[16];
+    ldrow(QH, e + ((OR + l * RS + VP) / 4) * st, st);
+    const float* h = QH + 6;
+    C2 r = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+    for (int m = 0; m < NTH; m++) {
+      const float vr = V[2 * m], vi = V[2 * m + 1];
+      r = {f2_fma(f2_dup(-vi), d[m].i, f2_fma(f2_dup(vr), d[m].r, r.r)),
+           f2_fma(f2_dup(vi), d[m].r, f2_fma(f2_dup(vr), d[m].i, r.i))};
+    }
+    const float2 den = f2_fma(lam, f2_dup(Lm[l]), make_float2(1.f, 1.f));
+    // 1 / den (den >= 1): the hardware reciprocal and one Newton step
+    const float2 x0 = make_float2(rcp_approx(den.x), rcp_approx(den.y));
+    const float2 x1 = f2_fma(x0, f2_fma(f2_neg(den), x0, make_float2(1.f, 1.f)), x0);
+    const float2 f = f2_mul(lam, x1);
+    const C2 sl = {f2_mul(r.r, f), f2_mul(r.i, f)};
+    const float2 nw = f2_neg(f2_mul(lam, f));
+    // mu_post += conj(Q_l.) s_l;  S_post -= w_l H_l, H_l = (|Q_l0|^2, |Q_l1|^2, |Q_l2|^2,
+    // conj(Q_l0) Q_l1, conj(Q_l0) Q_l2, conj(Q_l1) Q_l2)
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      const float qr = QH[2 * a], qi = QH[2 * a + 1];
+      o.mu[a] = {f2_fma(f2_dup(qi), sl.i, f2_fma(f2_dup(qr), sl.r, o.mu[a].r)),
+                 f2_fma(f2_dup(-qi), sl.r, f2_fma(f2_dup(qr), sl.i, o.mu[a].i))};
+      o.sd[a] = f2_fma(nw, f2_dup(h[a]), o.sd[a]);
+      o.so[a] = {f2_fma(nw, f2_dup(h[3 + 2 * a]), o.so[a].r), f2_fma(nw, f2_dup(h[4 + 2 * a]), o.so[a].i)};
+    }
+  }
+  // residual d - K mu_post = y - K (mu_post - mu) (the data spectrum itself where the row is zero:
+  // kz not inverted)
+  if (P.keep_resid) {
+    float kw[VP];
+    ldrow(kw, e + (OKW / 4) * st, st);
+    C2 dm[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) dm[a] = c2_sub(o.mu[a], mu[a]);
+#pragma unroll
+    for (int l = 0; l < NTH; l++) d[l] = c2_submul(d[l], kw[2 * l], kw[2 * l + 1], a_mu(P, l, dm));
+  }
+}
+
+// lib_matrCholCpx(3) of both bins' S_post (simulate :1425-1443): chol_ref (pencil_common.cuh) on
+// pairs.  L: sd holds the diagonal, so L10, L20, L21.  Returns bit u for a bin without a factor,
+// whose entries stay S_post.
+__device__ __forceinline__ int pair_factor(PairPost& o) {
+  const float2 s11 = o.sd[1], s22 = o.sd[2], f = o.sd[0];
+  const float2 i0 = make_float2(rsqrtf(f.x), rsqrtf(f.y));
+  const float2 tol = f2_mul(f, f2_dup(1e-20f));
+  const C2 l10 = {f2_mul(o.so[0].r, i0), f2_mul(f2_neg(o.so[0].i), i0)};
+  const C2 l20 = {f2_mul(o.so[1].r, i0), f2_mul(f2_neg(o.so[1].i), i0)};
+  const float2 r1 = f2_sub(s11, f2_fma(l10.i, l10.i, f2_mul(l10.r, l10.r)));
+  const float2 i1 = make_float2(rsqrtf(r1.x), rsqrtf(r1.y));
+  // a21 - L20 conj(L10), a21 = conj(S12)
+  const float2 tr = f2_sub(o.so[2].r, f2_fma(l20.i, l10.i, f2_mul(l20.r, l10.r)));
+  const float2 ti = f2_sub(f2_neg(o.so[2].i), f2_sub(f2_mul(l20.i, l10.r), f2_mul(l20.r, l10.i)));
+  const C2 l21 = {f2_mul(tr, i1), f2_mul(ti, i1)};
+  const float2 r2 = f2_sub(f2_sub(s22, f2_fma(l20.i, l20.i, f2_mul(l20.r, l20.r))),
+                           f2_fma(l21.i, l21.i, f2_mul(l21.r, l21.r)));
+  const float2 i2 = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+  const bool ok0 = f.x > 0.f && s11.x > tol.x && r1.x > tol.x && s22.x > tol.x && r2.x > tol.x;
+  const bool ok1 = f.y > 0.f && s11.y > tol.y && r1.y > tol.y && s22.y > tol.y && r2.y > tol.y;
+  const float2 d[3] = {f2_mul(f, i0), f2_mul(r1, i1), f2_mul(r2, i2)};
+  const C2 lo[3] = {l10, l20, l21};
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    if (ok0) {
+      o.sd[a].x = d[a].x;
+      o.so[a].r.x = lo[a].r.x;
+      o.so[a].i.x = lo[a].i.x;
+    }
+    if (ok1) {
+      o.sd[a].y = d[a].y;
+      o.so[a].r.y = lo[a].r.y;
+      o.so[a].i.y = lo[a].i.y;
+    }
+  }
+  return (ok0 ? 0 : 1) | (ok1 ? 0 : 2);
+}
+
+// S_post = L L^H of the bins that have a factor (mask as pair_factor returned it).
+__device__ __forceinline__ void pair_llh(float2 (&sd)[3], C2 (&so)[3], int fail) {
+  const float2 l0 = sd[0], l1 = sd[1], l2 = sd[2];
+  const C2 l10 = so[0], l20 = so[1], l21 = so[2];
+  const float2 d[3] = {f2_mul(l0, l0), f2_fma(l10.r, l10.r, f2_fma(l10.i, l10.i, f2_mul(l1, l1))),
+                       f2_fma(l20.r, l20.r,
+                              f2_fma(l20.i, l20.i, f2_fma(l21.r, l21.r, f2_fma(l21.i, l21.i, f2_mul(l2, l2)))))};
+  const C2 s[3] = {{f2_mul(l0, l10.r), f2_neg(f2_mul(l0, l10.i))},
+                   {f2_mul(l0, l20.r), f2_neg(f2_mul(l0, l20.i))},
+                   {f2_fma(l10.r, l20.r, f2_fma(l10.i, l20.i, f2_mul(l1, l21.r))),
+                    f2_sub(f2_mul(l10.i, l20.r), f2_fma(l10.r, l20.i, f2_mul(l1, l21.i)))}};
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    if (!(fail & 1)) {
+      sd[a].x = d[a].x;
+      so[a].r.x = s[a].r.x;
+      so[a].i.x = s[a].i.x;
+    }
+    if (!(fail & 2)) {
+      sd[a].y = d[a].y;
+      so[a].r.y = s[a].r.y;
+      so[a].i.y = s[a].i.y;
+    }
+  }
 }
 
 // ------------------------------------------------------------------ the kernel
+//
+// Shared memory: tw [nzp] (float2), the grid pointers of one batch of output lines (12), perm
+// [nzp] (uint16: kz of a position), then the tile, PS bytes per position.  With NP = W / 2 pairs:
+//   slot s, pair q         16-byte word s NP + q
+//   inputs                 data 0 .. nth-1, mean nth .. nth+2
+//   after the per-bin step SB realisations' spectra 0 .. 3 SB - 1, mu_post 3 SB .. 3 SB + 2,
+//                          S_post 01 02 12 (or L10 L20 L21) 3 SB + 3 .. 3 SB + 5
+//   diagonal of S_post (L) words D NP + q: {00, 11} of the pair's first bin, then of its second;
+//                          words D NP + NP + q / 2: 22 of the first bin at float q % 2, of the second
+//                          at 2 + q % 2
+// (D >= nth + 3 keeps the diagonal, which the threads of two pairs write, clear of the inputs; x-bins
+// 2 m and 2 m + 1 share a complex line whatever W is, so W does not change the results).
+enum PencilMode { kEig = 0, kChol = 1, kCholFp64 = 2 };
 
-// Shared-memory layout of one tile (W consecutive x-bins at one y, all NZ = N1 N2 positions):
-//   tw  [NZ]             z twiddles e^{-2 pi i t / NZ}
-//   R   [NZ][G][W]       G = max(nth + 3, 9) slots per bin: data 0..nth-1, mean nth..nth+2;
-//                        after the per-bin step S_post (or its realisation factor) 0..5 and
-//                        mu_post 6..8
-//   S3  [NZ][3 SB][W]    the output spectra of SB realisations, transformed together
-// Element (slot g, position p, x-offset w) of R is R[(p G + g) W + w].
-// DENSE: bounded for two 384-thread CTAs per SM (at most 80 registers), the other form for
-// one CTA of up to 512 threads (up to 128 registers).
-template <int NTH, int N1, int N2, bool DENSE>
-__global__ void __launch_bounds__(DENSE ? 384 : 512, DENSE ? 2 : 1) k_pencil(const __grid_constant__ ZParams P) {
-  extern __shared__ float2 sm[];
-  constexpr int NZ = N1 * N2;
-  constexpr int G = NTH + 3 > 9 ? NTH + 3 : 9;
+__device__ __forceinline__ void sts1(uint32_t a, float v) {
+  asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+__device__ __forceinline__ float lds1(uint32_t a) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void diag_put(uint32_t pos, const ZParams& P, int q, const float2 (&d)[3]) {
+  const uint32_t w = pos + 16u * (uint32_t)(P.D * P.NP);
+  sts4(w + 16u * (uint32_t)q, make_float4(d[0].x, d[1].x, d[0].y, d[1].y));
+  const uint32_t x = w + 16u * (uint32_t)(P.NP + (q >> 1)) + 4u * (uint32_t)(q & 1);
+  sts1(x, d[2].x);
+  sts1(x + 8u, d[2].y);
+  if (P.NP == 1) {   // no second pair in the word: its line is zero
+    sts1(x + 4u, 0.f);
+    sts1(x + 12u, 0.f);
+  }
+}
+__device__ __forceinline__ void diag_get(uint32_t pos, const ZParams& P, int q, float2 (&d)[3]) {
+  const uint32_t w = pos + 16u * (uint32_t)(P.D * P.NP);
+  const float4 a = lds4(w + 16u * (uint32_t)q);
+  const uint32_t x = w + 16u * (uint32_t)(P.NP + (q >> 1)) + 4u * (uint32_t)(q & 1);
+  d[0] = make_float2(a.x, a.z);
+  d[1] = make_float2(a.y, a.w);
+  d[2] = make_float2(lds1(x), lds1(x + 8u));
+}
+
+template <int NTH, int MODE, int R0, int R1>
+__global__ void __launch_bounds__(512, 1) k_pencil(const __grid_constant__ ZParams P) {
+  extern __shared__ __align__(16) unsigned char smb[];
+  __shared__ unsigned long long cnt[4];
   constexpr int GIN = NTH + 3;
-  const int W = P.W, lw = P.logW, SB = P.SB;
-  const int TS = W * NZ;
-  float2* tw = sm;
-  float2* R = tw + NZ;
-  float2* S3 = R + G * TS;
-  __shared__ unsigned long long cnt[2];
+  const int NZ = P.nzp, NP = P.NP, lnp = P.logNP, W = 2 * NP, SB = P.SB, PS = P.PS;
   const int T = blockDim.x, tid = threadIdx.x;
-  const int it = blockIdx.x % P.nIT;
-  const int j = blockIdx.x / P.nIT;
-  const int i0 = it * W;
-  const int nw = min(W, P.cnxp - i0);
+  const uint32_t s_tw = smem_addr(smb), s_out = s_tw + 8u * (uint32_t)even_up_z(NZ), s_perm = s_out + 96u;
+  const uint32_t tile = s_perm + 2u * (uint32_t)((NZ + 7) & ~7);
+  const uint16_t* perm = reinterpret_cast<const uint16_t*>(smb + (s_perm - s_tw));
+  unsigned long long* outp = reinterpret_cast<unsigned long long*>(smb + (s_out - s_tw));
+  const int it = blockIdx.x % P.nIT, j = blockIdx.x / P.nIT;
+  // x-offsets w in [wlo, nw) of the tile are bins i0 + w of the grid
+  const int i0 = it * W - (P.vec ? (j * P.cnxp) & 1 : 0), wlo = i0 < 0 ? 1 : 0, nw = min(W, P.cnxp - i0);
+  if (nw <= 0) return;   // a row without the early bin may need one tile less
   const size_t kstride = (size_t)P.nyp * P.cnxp;
   const size_t base = (size_t)j * P.cnxp + i0;
 
-  if (tid < 2) cnt[tid] = 0;
-  for (int t = tid; t < NZ; t += T) tw[t] = P.twz[t];
-  // ---- inputs: slot g <- data[g] (g < NTH) or mean[g - NTH], natural kz order; x-bins
-  //      beyond the grid are zero-filled
-  {
-    const uint32_t rb = smem_addr(R);
-    for (int e = tid; e < TS; e += T) {
-      const int w = e & (W - 1), k = e >> lw;
-      const bool ok = w < nw;
-      const size_t go = base + (ok ? (size_t)k * kstride + w : 0);
-      const uint32_t sa = rb + 8u * (uint32_t)(k * G * W + w);
+  // ---- inputs, natural kz order; x-bins beyond the grid are zero-filled
+  for (int e = tid; e < NZ << lnp; e += T) {
+    const int q = e & (NP - 1), w = 2 * q, k = e >> lnp;
+    const bool in0 = w >= wlo && w < nw, in1 = w + 1 < nw;
+    const size_t go = base + (size_t)k * kstride + w;
+    const uint32_t sa = tile + (uint32_t)(k * PS) + 16u * (uint32_t)q;
+    if (P.vec && in0 && in1) {
 #pragma unroll
       for (int g = 0; g < GIN; g++)
-        cp_async8_zfill(sa + 8u * (uint32_t)(g * W), (g < NTH ? P.data[g] : P.mean[g - NTH]) + go, ok);
+        cp_async16(sa + 16u * (uint32_t)(g << lnp), (g < NTH ? P.data[g] : P.mean[g - NTH]) + go);
+    } else {
+#pragma unroll
+      for (int g = 0; g < GIN; g++) {
+        const float2* src = g < NTH ? P.data[g] : P.mean[g - NTH];
+        const uint32_t d = sa + 16u * (uint32_t)(g << lnp);
+        cp_async8_zfill(d, src + (in0 ? go : 0), in0);
+        cp_async8_zfill(d + 8u, src + (in1 ? go + 1 : 0), in1);
+      }
     }
-    cp_async_commit();
-    cp_async_wait_0();
   }
+  cp_async_commit();
+  if (tid < 4) cnt[tid] = 0;
+  for (int t = tid; t < NZ; t += T) {
+    sts2(s_tw + 8u * (uint32_t)t, __ldg(P.twz + t));
+    const_cast<uint16_t*>(perm)[t] = (uint16_t)pencil_kz_dev(P.z, t);
+  }
+  cp_async_wait_0();
   __syncthreads();
-  zfwd_inplace<N1, N2>(R, GIN * W, G * W, tw);
+  ZStage zs;
+  zs.base = tile;
+  zs.tw = s_tw;
+  zs.ps = PS;
+  zs.nl = GIN << lnp;
+  zs.split = zs.nl;
+  zs.gap = 0;
+  z_forward<R0, R1>(P.z, zs);
   // a NaN or Inf in any input grid reaches every bin through the transforms
   if (tid == 0 && P.counters) {
     float s = 0.f;
 #pragma unroll
-    for (int g = 0; g < GIN; g++) s += fabsf(R[g * W].x) + fabsf(R[g * W].y);
+    for (int g = 0; g < GIN; g++) {
+      const float4 v = lds4(tile + 16u * (uint32_t)(g << lnp));
+      s += wlo ? fabsf(v.y) + fabsf(v.w) : fabsf(v.x) + fabsf(v.z);
+    }
     if (!isfinite(s)) atomicAdd(P.counters + 4, 1ull);
   }
 
-  // ---- per-bin posterior; bin at position p holds kz = p / N2 + N1 (p % N2).  A thread takes
-  //      NB bins of one position (x-offsets w, w + W/NB, ...), so each table row it loads
-  //      serves all of them
-  unsigned long long n_zero_bins = 0;
-  const int NB = (W >= 2 && P.nb2) ? 2 : 1;
-  const int WB = W / NB, lwb = NB == 2 ? lw - 1 : lw;
-  for (int b = tid; b < TS / NB; b += T) {
-    const int p = b >> lwb, w0 = b & (WB - 1);
-    const int kz = p / N2 + N1 * (p % N2);
-    const float ctk = __ldg(P.ct + kz).x;
-    if (NB == 2) {
-      float lam[2], rho[2];
-      float2 mu[2][3], d[2][NTH], mp[2][3], sp[2][6];
+  // ---- per-bin posterior.  The positions of neighbouring threads are p and p ^ 3 swapped within
+  //      fours where that puts their words on different banks (P.swz)
+  const int items = NZ << lnp;
+  const uint32_t s_post = 16u * (uint32_t)((3 * SB) << lnp);   // byte offset of mu_post in a position
+  unsigned long long n_zero_bins = 0, n_inv = 0, n_fail = 0, n_fp64 = 0;
+  unsigned int failed = 0;                                    // two bits per item of this thread
+  auto pos_of = [&](int b) {
+    const int p = b >> lnp;
+    return P.swz ? (p & ~3) | ((p & 1) << 1) | ((p >> 1) & 1) : p;
+  };
+  {
+    int n = 0;
+#pragma unroll 1
+    for (int b = tid; b < items; b += T, n++) {
+      const int q = b & (NP - 1), p = pos_of(b), kz = perm[p];
+      const uint32_t pos = tile + (uint32_t)(p * PS), sl = pos + 16u * (uint32_t)q;
+      const bool in0 = 2 * q >= wlo && 2 * q < nw, in1 = 2 * q + 1 < nw;
+      const size_t gidx = base + (size_t)kz * kstride + 2 * q;
+      C2 mu[3], d[NTH];
 #pragma unroll
-      for (int u = 0; u < 2; u++) {
-        const int w = w0 + u * WB;
-        const bool ok = w < nw;
-        const float2 cx = ok ? __ldg(P.cxy + (size_t)j * P.cnxp + i0 + w) : make_float2(0.f, 0.f);
-        lam[u] = fabsf(cx.x);
-        rho[u] = fabsf(cx.x * ctk);
-        const float2* slot = R + p * G * W + w;
+      for (int l = 0; l < NTH; l++) d[l] = lds_c2(sl + 16u * (uint32_t)(l << lnp));
 #pragma unroll
-        for (int a = 0; a < 3; a++) mu[u][a] = slot[(NTH + a) * W];
+      for (int a = 0; a < 3; a++) mu[a] = lds_c2(sl + 16u * (uint32_t)((NTH + a) << lnp));
+      PairPost o;
+      if constexpr (MODE == kEig) {
+        float2 lam, rho;
+        {
+          const float ctk = __ldg(P.ct + kz).x;
+          const float2* cx = P.cxy + base + 2 * q;
+          const float c0 = in0 ? __ldg(cx).x : 0.f, c1 = in1 ? __ldg(cx + 1).x : 0.f;
+          lam = make_float2(fabsf(c0), fabsf(c1));
+          rho = make_float2(fabsf(c0 * ctk), fabsf(c1 * ctk));
+        }
+        pair_posterior_eig<NTH>(P, P.eig + p, lam, rho, mu, d, o);
+      } else {
+        const bool inv = P.kz.inv[kz] != 0;
 #pragma unroll
-        for (int l = 0; l < NTH; l++) d[u][l] = slot[l * W];
+        for (int u = 0; u < 2; u++) {
+          float S[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, lam = 0.f, rho = 0.f;
+          const bool in = u ? in1 : in0;
+          if (in) {
+            if (P.separable) {
+              const float2 cx = __ldg(P.cxy + base + 2 * q + u), c_t = __ldg(P.ct + kz);
+              rho = fabsf(cx.x * c_t.x - cx.y * c_t.y);
+#pragma unroll
+              for (int c = 0; c < 6; c++) S[c] = P.pv[c] * rho;
+              lam = fabsf(cx.x);
+            } else {
+              // getNextParameterCovariance: |Re/pv| pv (no division when pv == 0); a base prior's
+              // pairs share |Re/pv| of the one spectrum transformed (pv[0] != 0)
+              const size_t gi = gidx + u;
+              if (P.base_prior) {
+                const float r0 = fabsf(P.cov[0][gi].x / P.pv[0]);
+#pragma unroll
+                for (int c = 0; c < 6; c++) S[c] = r0 * P.pv[c];
+              } else {
+#pragma unroll
+                for (int c = 0; c < 6; c++) {
+                  float re = P.cov[c][gi].x;
+                  const float pv = P.pv[c];
+                  if (pv != 0.f) re = re / pv;
+                  S[c] = fabsf(re) * pv;
+                }
+              }
+              lam = fabsf(P.errspec[gi].x);
+            }
+          }
+          float2 m1[3], d1[NTH];
+#pragma unroll
+          for (int a = 0; a < 3; a++) m1[a] = u ? make_float2(mu[a].r.y, mu[a].i.y) : make_float2(mu[a].r.x, mu[a].i.x);
+#pragma unroll
+          for (int l = 0; l < NTH; l++) d1[l] = u ? make_float2(d[l].r.y, d[l].i.y) : make_float2(d[l].r.x, d[l].i.x);
+          BinOut bo;
+          bool ok = false;
+          if (inv && in) {
+            n_inv++;
+            ok = P.septab ? bin_posterior<NTH, true>(P, kz, S, lam, rho, m1, d1, bo)
+                          : bin_posterior<NTH, false>(P, kz, S, lam, rho, m1, d1, bo);
+            if constexpr (MODE == kCholFp64) {
+              if (ok) {
+                float ratio = 1.f;
+#pragma unroll
+                for (int a = 0; a < 3; a++)
+                  if (S[a] > 0.f) ratio = fminf(ratio, bo.sp[a].x / S[a]);
+                if (bo.cond > P.fp64_threshold || ratio * P.fp64_threshold < 1.f) {
+                  float2 d64[NTH];
+#pragma unroll
+                  for (int l = 0; l < NTH; l++)
+                    d64[l] = u ? make_float2(d[l].r.y, d[l].i.y) : make_float2(d[l].r.x, d[l].i.x);
+                  if (bin_posterior_fp64<NTH>(P, kz, S, lam, m1, d64, bo)) {
+                    n_fp64++;
+#pragma unroll
+                    for (int l = 0; l < NTH; l++) d1[l] = d64[l];
+                  }
+                }
+              }
+            }
+            if (!ok) n_fail++;
+          }
+          if (!ok) {
+#pragma unroll
+            for (int a = 0; a < 3; a++) bo.mu[a] = m1[a];
+#pragma unroll
+            for (int c = 0; c < 6; c++) bo.sp[c] = make_float2(S[c], 0.f);
+          }
+#pragma unroll
+          for (int a = 0; a < 3; a++) {
+            if (u == 0) {
+              o.mu[a].r.x = bo.mu[a].x;
+              o.mu[a].i.x = bo.mu[a].y;
+              o.sd[a].x = bo.sp[a].x;
+              o.so[a].r.x = bo.sp[3 + a].x;
+              o.so[a].i.x = bo.sp[3 + a].y;
+            } else {
+              o.mu[a].r.y = bo.mu[a].x;
+              o.mu[a].i.y = bo.mu[a].y;
+              o.sd[a].y = bo.sp[a].x;
+              o.so[a].r.y = bo.sp[3 + a].x;
+              o.so[a].i.y = bo.sp[3 + a].y;
+            }
+          }
+          if (P.keep_resid && in) {
+#pragma unroll
+            for (int l = 0; l < NTH; l++) P.data[l][gidx + u] = d1[l];
+          }
+        }
       }
-      bin_posterior_eig<NTH, 2>(P, P.eig + p, lam, rho, mu, d, mp, sp);
+      if constexpr (MODE == kEig) {
+        if (P.keep_resid) {
 #pragma unroll
-      for (int u = 0; u < 2; u++) {
-        const int w = w0 + u * WB;
-        if (w < nw) n_zero_bins += store_bin<NTH>(P, R + p * G * W + w, W, d[u], mp[u], sp[u],
-                                                  base + (size_t)kz * kstride + w);
+          for (int l = 0; l < NTH; l++) {
+            if (in0) P.data[l][gidx] = make_float2(d[l].r.x, d[l].i.x);
+            if (in1) P.data[l][gidx + 1] = make_float2(d[l].r.y, d[l].i.y);
+          }
+        }
       }
-    } else {
-      const int w = w0;
-      if (w >= nw) continue;
-      const float2 cx = __ldg(P.cxy + (size_t)j * P.cnxp + i0 + w);
-      float lam[1] = {fabsf(cx.x)}, rho[1] = {fabsf(cx.x * ctk)};
-      float2 mu[1][3], d[1][NTH], mp[1][3], sp[1][6];
-      const float2* slot = R + p * G * W + w;
+      // S_post is factored once for all realisations; the covariance output is rebuilt as L L^H
+      if (P.nsim > 0) {
+        const int fail = pair_factor(o);
+        failed |= (unsigned int)fail << (2 * n);
+        if ((fail & 1) && in0) n_zero_bins++;
+        if ((fail & 2) && in1) n_zero_bins++;
+      }
+      const uint32_t so = sl + s_post;
 #pragma unroll
-      for (int a = 0; a < 3; a++) mu[0][a] = slot[(NTH + a) * W];
-#pragma unroll
-      for (int l = 0; l < NTH; l++) d[0][l] = slot[l * W];
-      bin_posterior_eig<NTH, 1>(P, P.eig + p, lam, rho, mu, d, mp, sp);
-      n_zero_bins += store_bin<NTH>(P, R + p * G * W + w, W, d[0], mp[0], sp[0], base + (size_t)kz * kstride + w);
+      for (int a = 0; a < 3; a++) {
+        sts_c2(so + 16u * (uint32_t)(a << lnp), o.mu[a]);
+        sts_c2(so + 16u * (uint32_t)((3 + a) << lnp), o.so[a]);
+      }
+      diag_put(pos, P, q, o.sd);
     }
   }
+  ZOut zo;
+  zo.out = s_out;
+  zo.base = base;
+  zo.kstride = kstride;
+  zo.wlo = wlo;
+  zo.nw = nw;
+  zo.logNP = lnp;
+  zo.vec = P.vec;
   __syncthreads();
 
-  // ---- SB = 0: no realisation slots.  The posterior mean (slots 6..8) is transformed and
-  //      stored first; each realisation's L z then goes through those slots and the stored mean
-  //      is added in the last pass (IFFT(mu + L z) = IFFT(mu) + IFFT(L z)); the covariance last.
-  //      The tile needs G slots instead of G + 3, so wider tiles fit at the longer z lengths.
-  if (SB == 0) {
-    zinv_store<N1, N2>(R + 6 * W, 3 * W, G * W, tw, [&](int l, int k, float2 v) {
-      const int w = l & (W - 1);
-      if (w < nw) P.mean[l >> lw][base + (size_t)k * kstride + w] = v;
-    });
+  // ---- realisations, the mean added in the spectral domain; SB share one transform
 #pragma unroll 1
-    for (int s = 0; s < P.nsim; s++) {
-      for (int b = tid; b < TS; b += T) {
-        const int p = b >> lw, w = b & (W - 1);
-        const float2* slot = R + p * G * W + w;
-        float2* o3 = R + (p * G + 6) * W + w;
-        float2 sd[3] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-        const float2 l0 = slot[0];
-        if (w < nw && l0.y == -1.f) {
-          const int kz = p / N2 + N1 * (p % N2);
-          float2 z[3];
-          if (P.host_noise) {
-            const size_t gidx = base + (size_t)kz * kstride + w;
-#pragma unroll
-            for (int c = 0; c < 3; c++) z[c] = P.noise[3 * s + c][gidx];
-          } else {
-            device_noise3(P.seed, s, i0 + w, j, kz, P.nyp, NZ, P.cnxp, P.nxp_even, z);
-          }
-          const float2 l1 = slot[W], l2 = slot[2 * W], l10 = slot[3 * W], l20 = slot[4 * W], l21 = slot[5 * W];
-          sd[0] = make_float2(l0.x * z[0].x, l0.x * z[0].y);
-          sd[1] = cadd(cmul(l10, z[0]), make_float2(l1.x * z[1].x, l1.x * z[1].y));
-          sd[2] = cadd(cadd(cmul(l20, z[0]), cmul(l21, z[1])), make_float2(l2.x * z[2].x, l2.x * z[2].y));
-          // the last realisation leaves S_post in slots 0..5 for the covariance output
-          if (s == P.nsim - 1) store_llh(R + p * G * W + w, W, l0, l1, l2, l10, l20, l21);
-        }
-        o3[0] = sd[0];
-        o3[W] = sd[1];
-        o3[2 * W] = sd[2];
-      }
-      __syncthreads();
-      // the mean this CTA stored above (visible after the barriers), read at L2
-      zinv_store<N1, N2>(R + 6 * W, 3 * W, G * W, tw, [&](int l, int k, float2 v) {
-        const int w = l & (W - 1);
-        if (w < nw) {
-          const size_t idx = base + (size_t)k * kstride + w;
-          P.sim[3 * s + (l >> lw)][idx] = cadd(__ldcg(P.mean[l >> lw] + idx), v);
-        }
-      });
-    }
-  }
-  // ---- realisations (src/avoinversion.cpp:1401-1511), the mean added in the spectral
-  //      domain; SB realisations per batch share one transform call
-#pragma unroll 1
-  for (int s0 = 0; SB > 0 && s0 < P.nsim; s0 += SB) {
+  for (int s0 = 0; s0 < P.nsim; s0 += SB) {
     const int nb = min(SB, P.nsim - s0);
-    const int SG = 3 * SB;   // slot stride of S3
-    for (int b = tid; b < TS; b += T) {
-      const int p = b >> lw, w = b & (W - 1);
-      float2* o3 = S3 + p * SG * W + w;
-      if (w >= nw) {
-        for (int q = 0; q < 3 * nb; q++) o3[q * W] = make_float2(0.f, 0.f);
-        continue;
-      }
-      const int kz = p / N2 + N1 * (p % N2);
-      const int i = i0 + w;
-      const float2* slot = R + p * G * W + w;
-      const float2 l0 = slot[0];
-      const float2 m0 = slot[6 * W], m1 = slot[7 * W], m2 = slot[8 * W];
-      const bool fac = l0.y == -1.f;
-      float2 l1 = make_float2(0.f, 0.f), l2 = l1, l10 = l1, l20 = l1, l21 = l1;
-      if (fac) {
-        l1 = slot[W]; l2 = slot[2 * W]; l10 = slot[3 * W]; l20 = slot[4 * W]; l21 = slot[5 * W];
+    const bool last = s0 + nb == P.nsim;
+    if (tid < 3 * nb) outp[tid] = (unsigned long long)(uintptr_t)P.sim[3 * s0 + tid];
+    int n = 0;
+#pragma unroll 1
+    for (int b = tid; b < items; b += T, n++) {
+      const int q = b & (NP - 1), p = pos_of(b), kz = perm[p];
+      const uint32_t pos = tile + (uint32_t)(p * PS), sl = pos + 16u * (uint32_t)q, so = sl + s_post;
+      const int fail = (failed >> (2 * n)) & 3;
+      float2 ld[3];
+      diag_get(pos, P, q, ld);
+      C2 lo[3], mu[3];
+#pragma unroll
+      for (int a = 0; a < 3; a++) {
+        mu[a] = lds_c2(so + 16u * (uint32_t)(a << lnp));
+        lo[a] = lds_c2(so + 16u * (uint32_t)((3 + a) << lnp));
       }
 #pragma unroll 1
       for (int sb = 0; sb < nb; sb++) {
-        const int s = s0 + sb;
-        float2 sd[3] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-        if (fac) {
-          float2 z[3];
-          if (P.host_noise) {
-            const size_t gidx = base + (size_t)kz * kstride + w;
+        C2 z[3];
+        if (P.host_noise) {
+          float2 za[3], zb[3];
+          {
+            const size_t gidx = base + (size_t)kz * kstride + 2 * q;
+            const bool in0 = 2 * q >= wlo && 2 * q < nw, in1 = 2 * q + 1 < nw;
 #pragma unroll
-            for (int c = 0; c < 3; c++) z[c] = P.noise[3 * s + c][gidx];
-          } else {
-            device_noise3(P.seed, s, i, j, kz, P.nyp, NZ, P.cnxp, P.nxp_even, z);
+            for (int c = 0; c < 3; c++) {
+              za[c] = in0 ? P.noise[3 * (s0 + sb) + c][gidx] : make_float2(0.f, 0.f);
+              zb[c] = in1 ? P.noise[3 * (s0 + sb) + c][gidx + 1] : make_float2(0.f, 0.f);
+            }
           }
-          sd[0] = make_float2(l0.x * z[0].x, l0.x * z[0].y);
-          sd[1] = cadd(cmul(l10, z[0]), make_float2(l1.x * z[1].x, l1.x * z[1].y));
-          sd[2] = cadd(cadd(cmul(l20, z[0]), cmul(l21, z[1])), make_float2(l2.x * z[2].x, l2.x * z[2].y));
+#pragma unroll
+          for (int c = 0; c < 3; c++) z[c] = {make_float2(za[c].x, zb[c].x), make_float2(za[c].y, zb[c].y)};
+        } else {
+          pair_noise(P, s0 + sb, i0 + 2 * q, j, kz, z);
         }
-        o3[(3 * sb) * W] = cadd(m0, sd[0]);
-        o3[(3 * sb + 1) * W] = cadd(m1, sd[1]);
-        o3[(3 * sb + 2) * W] = cadd(m2, sd[2]);
+        // L z: rows (l0), (L10, l1), (L20, L21, l2)
+        C2 x[3];
+#pragma unroll
+        for (int a = 0; a < 3; a++) x[a] = {f2_mul(ld[a], z[a].r), f2_mul(ld[a], z[a].i)};
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+          const int r = a == 0 ? 1 : 2, c = a == 2 ? 1 : 0;
+          x[r] = {f2_sub(f2_fma(lo[a].r, z[c].r, x[r].r), f2_mul(lo[a].i, z[c].i)),
+                  f2_fma(lo[a].r, z[c].i, f2_fma(lo[a].i, z[c].r, x[r].i))};
+        }
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+          if (fail & 1) x[a].r.x = x[a].i.x = 0.f;
+          if (fail & 2) x[a].r.y = x[a].i.y = 0.f;
+          sts_c2(sl + 16u * (uint32_t)((3 * sb + a) << lnp), c2_add(mu[a], x[a]));
+        }
       }
-      // the last batch leaves S_post in slots 0..5 for the covariance output
-      if (fac && s0 + nb == P.nsim) store_llh(R + p * G * W + w, W, l0, l1, l2, l10, l20, l21);
+      if (last) {
+        pair_llh(ld, lo, fail);
+#pragma unroll
+        for (int a = 0; a < 3; a++) sts_c2(so + 16u * (uint32_t)((3 + a) << lnp), lo[a]);
+        diag_put(pos, P, q, ld);
+      }
     }
     __syncthreads();
-    // inverse z transform, the last pass storing the realisations' spectra (line l: grid
-    // 3 s0 + l / W, x-offset l % W)
-    zinv_store<N1, N2>(S3, 3 * nb * W, SG * W, tw, [&](int l, int k, float2 v) {
-      const int w = l & (W - 1);
-      if (w < nw) P.sim[3 * s0 + (l >> lw)][base + (size_t)k * kstride + w] = v;
-    });
+    zs.nl = zs.split = (3 * nb) << lnp;
+    z_inverse<R0, R1>(P.z, zs, zo);
   }
-  // (S_post = L L^H is back in slots 0..5: the last realisation wrote it)
-  // ---- inverse z transform of posterior covariance (slots 0..5, unless it stays spectral)
-  //      and mean (6..8); spectral covariance slots stay in position order
-  if (!P.cov_spectral) {
-    // slots 0..5 to cov[0..5], 6..8 to mean[0..2] (already stored when SB = 0), stored by the
-    // last pass
-    zinv_store<N1, N2>(R, (SB == 0 ? 6 : 9) * W, G * W, tw, [&](int l, int k, float2 v) {
-      const int g = l >> lw, w = l & (W - 1);
-      if (w < nw) (g < 6 ? P.cov[g] : P.mean[g - 6])[base + (size_t)k * kstride + w] = v;
-    });
+
+  // ---- inverse z transform of the posterior mean and covariance (unless it stays spectral)
+  zs.base = tile + s_post;
+  if (P.cov_spectral) {
+    if (tid < 3) outp[tid] = (unsigned long long)(uintptr_t)P.mean[tid];
+    for (int b = tid; b < items; b += T) {
+      const int q = b & (NP - 1), p = b >> lnp;
+      const uint32_t pos = tile + (uint32_t)(p * PS), so = pos + 16u * (uint32_t)q + s_post;
+      const bool in0 = 2 * q >= wlo && 2 * q < nw, in1 = 2 * q + 1 < nw;
+      const size_t gidx = base + (size_t)perm[p] * kstride + 2 * q;
+      float2 sd[3];
+      diag_get(pos, P, q, sd);
+#pragma unroll
+      for (int a = 0; a < 3; a++) {
+        const C2 s = lds_c2(so + 16u * (uint32_t)((3 + a) << lnp));
+        if (in0) {
+          P.cov[a][gidx] = make_float2(sd[a].x, 0.f);
+          P.cov[3 + a][gidx] = make_float2(s.r.x, s.i.x);
+        }
+        if (in1) {
+          P.cov[a][gidx + 1] = make_float2(sd[a].y, 0.f);
+          P.cov[3 + a][gidx + 1] = make_float2(s.r.y, s.i.y);
+        }
+      }
+    }
+    zs.nl = zs.split = 3 << lnp;
+    __syncthreads();
+    z_inverse<R0, R1>(P.z, zs, zo);
   } else {
-    // spectral covariance: slots 0..5 stay in position order, stored at their kz (the mean,
-    // slots 6..8, is already stored when SB = 0)
-    if (SB > 0) zinv_inplace<N1, N2>(R + 6 * W, 3 * W, G * W, tw);
-    for (int e = tid; e < TS; e += T) {
-      const int w = e & (W - 1), k = e >> lw;
-      if (w >= nw) continue;
-      const size_t go = base + (size_t)k * kstride + w;
-      const int so = k * G * W + w;
-      const int kz = k / N2 + N1 * (k % N2);
+    if (tid < 6) outp[tid] = (unsigned long long)(uintptr_t)(tid < 3 ? P.mean[tid] : P.cov[tid]);
+    const int ndl = NP + ((NP + 1) >> 1);               // words of the diagonal
+    zs.split = 6 << lnp;
+    zs.nl = zs.split + ndl;
+    zs.gap = 16 * ((P.D - 3 * SB - 6) << lnp);
+    __syncthreads();
+    z_inverse<R0, R1>(P.z, zs, zo);
+    // the diagonal's lines x = S_A + i S_B (S real spectra): S_A(z) = (x(z) + conj x(-z)) / 2,
+    // S_B(z) = (x(z) - conj x(-z)) / 2i
+    const int half = NZ / 2 + 1;
+    const float rd = __frcp_rn((float)ndl);
+    for (int e = tid; e < ndl * half; e += T) {
+      int l;
+      const int z = fdivmod(e, ndl, rd, l), zm = z == 0 ? 0 : NZ - z;
+      const uint32_t wd = tile + 16u * (uint32_t)((P.D << lnp) + l);
+      const float4 x = lds4(wd + (uint32_t)(z * PS)), y = lds4(wd + (uint32_t)(zm * PS));
 #pragma unroll
-      for (int g = 0; g < 6; g++) P.cov[g][base + (size_t)kz * kstride + w] = R[so + g * W];
-      if (SB > 0) {
-#pragma unroll
-        for (int a = 0; a < 3; a++) P.mean[a][go] = R[so + (6 + a) * W];
+      for (int h = 0; h < 2; h++) {
+        // complex line h of the word: entry 00 (h = 0) or 11 of pair l, or 22 of pair 2 (l - NP) + h
+        const int c = l < NP ? h : 2, q = l < NP ? l : 2 * (l - NP) + h, w = 2 * q;
+        if (q >= NP) continue;
+        const float xr = h ? x.y : x.x, xi = h ? x.w : x.z, yr = h ? y.y : y.x, yi = h ? y.w : y.z;
+        const float2 A = make_float2(0.5f * (xr + yr), 0.5f * (xi - yi));
+        const float2 B = make_float2(0.5f * (xi + yi), 0.5f * (yr - xr));
+        const bool in0 = w >= wlo && w < nw, in1 = w + 1 < nw;
+        float2* g = P.cov[c] + base + w;
+        float2 *gz = g + (size_t)z * kstride, *gm = g + (size_t)zm * kstride;
+        if (P.vec && in0 && in1) {
+          *reinterpret_cast<float4*>(gz) = make_float4(A.x, A.y, B.x, B.y);
+          if (zm != z) *reinterpret_cast<float4*>(gm) = make_float4(A.x, -A.y, B.x, -B.y);
+        } else {
+          if (in0) {
+            gz[0] = A;
+            if (zm != z) gm[0] = make_float2(A.x, -A.y);
+          }
+          if (in1) {
+            gz[1] = B;
+            if (zm != z) gm[1] = make_float2(B.x, -B.y);
+          }
+        }
       }
     }
   }
 
-  // counters: inverted bins per tile column from the host's count of inverted kz
+  // counters
   unsigned long long n_zero = n_zero_bins * (unsigned long long)P.nsim;
-  for (int off = 16; off > 0; off >>= 1) n_zero += __shfl_down_sync(0xffffffffu, n_zero, off);
-  if ((tid & 31) == 0 && n_zero) atomicAdd(&cnt[0], n_zero);
+  for (int off = 16; off > 0; off >>= 1) {
+    n_zero += __shfl_down_sync(0xffffffffu, n_zero, off);
+    if (MODE != kEig) {
+      n_inv += __shfl_down_sync(0xffffffffu, n_inv, off);
+      n_fail += __shfl_down_sync(0xffffffffu, n_fail, off);
+      n_fp64 += __shfl_down_sync(0xffffffffu, n_fp64, off);
+    }
+  }
+  if ((tid & 31) == 0) {
+    if (n_zero) atomicAdd(&cnt[2], n_zero);
+    if (MODE != kEig) {
+      atomicAdd(&cnt[0], n_inv);
+      atomicAdd(&cnt[1], n_fail);
+      atomicAdd(&cnt[3], n_fp64);
+    }
+  }
   __syncthreads();
   if (tid == 0 && P.counters) {
-    atomicAdd(P.counters + 0, (unsigned long long)P.n_inv_rows * (unsigned long long)nw);
-    if (cnt[0]) atomicAdd(P.counters + 2, cnt[0]);
+    // eigen form: inverted bins per tile column from the host's count of inverted kz
+    atomicAdd(P.counters + 0, MODE == kEig ? (unsigned long long)P.n_inv_rows * (unsigned long long)(nw - wlo) : cnt[0]);
+    if (cnt[1]) atomicAdd(P.counters + 1, cnt[1]);
+    if (cnt[2]) atomicAdd(P.counters + 2, cnt[2]);
+    if (cnt[3]) atomicAdd(P.counters + 3, cnt[3]);
   }
 }
 
 // ------------------------------------------------------------------ launch templates
 
-template <int NTH, int N1, int N2, bool DENSE>
-inline cudaError_t launch_pencil_d(const ZParams& zp, int threads, cudaStream_t st) {
+template <int NTH, int MODE, int R0, int R1>
+inline cudaError_t launch_pencil_t(const ZParams& zp, int threads, cudaStream_t st) {
   const size_t smem = pencil_smem_bytes(zp.W, zp.nzp, zp.nth, zp.SB);
-  auto fn = k_pencil<NTH, N1, N2, DENSE>;
+  auto fn = k_pencil<NTH, MODE, R0, R1>;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   fn<<<dim3((unsigned)(zp.nIT * zp.nyp)), threads, smem, st>>>(zp);
   return cudaGetLastError();
 }
-
-// The dense form is instantiated for up to 6 angle stacks and 256 / 320 points (the
-// production and precision-study lengths).
-template <int NTH, int N1, int N2>
-inline cudaError_t launch_pencil_t(const ZParams& zp, int threads, cudaStream_t st) {
-  if constexpr (NTH <= 6 && N2 == 16) {
-    if (zp.dense && threads <= 384) return launch_pencil_d<NTH, N1, N2, true>(zp, threads, st);
-  }
-  return launch_pencil_d<NTH, N1, N2, false>(zp, threads, st);
+template <int NTH>
+inline cudaError_t launch_pencil_m(const ZParams& zp, int threads, cudaStream_t st) {
+  if (zp.fp64_threshold > 0.f) return launch_pencil_t<NTH, kCholFp64, 0, 0>(zp, threads, st);
+  if (!zp.eig) return launch_pencil_t<NTH, kChol, 0, 0>(zp, threads, st);
+  // the z lengths of the benchmark blocks inline their split (pencil_plan gives the same)
+  if (zp.nzp == 256) return launch_pencil_t<NTH, kEig, 16, 16>(zp, threads, st);
+  if (zp.nzp == 320) return launch_pencil_t<NTH, kEig, 20, 16>(zp, threads, st);
+  if (zp.nzp == 128) return launch_pencil_t<NTH, kEig, 16, 8>(zp, threads, st);
+  return launch_pencil_t<NTH, kEig, 0, 0>(zp, threads, st);
 }
 
-
-// launchers of one z split each (pencil_s1.cu 16x16, pencil_s2.cu 20x16, pencil_s3.cu 16x8)
-cudaError_t launch_pencil_split1(const ZParams& zp, int threads, cudaStream_t st);
-cudaError_t launch_pencil_split2(const ZParams& zp, int threads, cudaStream_t st);
-cudaError_t launch_pencil_split3(const ZParams& zp, int threads, cudaStream_t st);
+// launchers by angle count (pencil_n12.cu, pencil_n34.cu, pencil_n56.cu, pencil_n78.cu): one
+// translation unit per pair so that they compile side by side
+cudaError_t launch_pencil_n12(const ZParams& zp, int threads, cudaStream_t st);
+cudaError_t launch_pencil_n34(const ZParams& zp, int threads, cudaStream_t st);
+cudaError_t launch_pencil_n56(const ZParams& zp, int threads, cudaStream_t st);
+cudaError_t launch_pencil_n78(const ZParams& zp, int threads, cudaStream_t st);
 
 }  // namespace crava
