@@ -207,6 +207,11 @@ struct crava_ctx {
   int fail_allocs = 0;   // crava_ctx_fail_next_allocs: job allocations still to fail
   double kt_ms[KT_COUNT] = {};
   long long kt_n[KT_COUNT] = {};
+  // stream-ordered scratch of the facies, local-noise and prior calls: a memory pool of the context's own that keeps up to
+  // kScratchKeep between calls (the default pool gives its memory back at every synchronisation,
+  // and mapping it again took up to milliseconds); destroyed with the context, emptied when a job
+  // finds no memory
+  cudaMemPool_t scratch = nullptr;
   std::mutex stage_mu;         // device staging grid of the host-grid transforms
   float* stage = nullptr;
   size_t stage_bytes = 0;
@@ -224,6 +229,26 @@ struct crava_ctx {
 };
 
 namespace {
+constexpr uint64_t kScratchKeep = 256ull << 20;
+
+cudaError_t scratch_alloc(crava_ctx* ctx, void** p, size_t bytes, cudaStream_t st) {
+  {
+    std::lock_guard<std::mutex> lk(ctx->mu);
+    if (!ctx->scratch) {
+      cudaMemPoolProps pr = {};
+      pr.allocType = cudaMemAllocationTypePinned;
+      pr.location.type = cudaMemLocationTypeDevice;
+      pr.location.id = ctx->device;
+      cudaError_t e = cudaMemPoolCreate(&ctx->scratch, &pr);
+      if (e != cudaSuccess) return e;
+      uint64_t keep = kScratchKeep;
+      e = cudaMemPoolSetAttribute(ctx->scratch, cudaMemPoolAttrReleaseThreshold, &keep);
+      if (e != cudaSuccess) return e;
+    }
+  }
+  return cudaMallocFromPoolAsync(p, bytes, ctx->scratch, st);
+}
+
 void cache_evict_locked(crava_ctx* ctx, size_t want, cudaStream_t st);
 
 // Brackets one launch with events on its stream when profiling is on.
@@ -1745,6 +1770,7 @@ crava_status crava_ctx_destroy(crava_ctx* ctx) {
   cudaDeviceSynchronize();
   for (auto& kv : ctx->plans) cudaFree(kv.second.tw);
   if (ctx->stage) cudaFree(ctx->stage);
+  if (ctx->scratch) cudaMemPoolDestroy(ctx->scratch);
   for (auto& kv : ctx->cache) {
     if (kv.second->ready) cudaEventDestroy(kv.second->ready);
     cudaFree(kv.second->mem);
@@ -2143,8 +2169,15 @@ crava_status job_create_impl(crava_ctx* ctx, const crava_job_desc* desc, cudaStr
       injected = true;
     }
   }
-  cudaError_t e = injected ? cudaErrorMemoryAllocation
-                           : async ? cudaMallocAsync((void**)&j->pool, need, st) : cudaMalloc(&j->pool, need);
+  auto pool_alloc = [&] {
+    return async ? cudaMallocAsync((void**)&j->pool, need, st) : cudaMalloc(&j->pool, need);
+  };
+  cudaError_t e = injected ? cudaErrorMemoryAllocation : pool_alloc();
+  if (e != cudaSuccess && !injected && ctx->scratch) {   // the kept scratch gives way to a job
+    cudaGetLastError();
+    cudaMemPoolTrimTo(ctx->scratch, 0);
+    e = pool_alloc();
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     j->pool = nullptr;
@@ -2673,7 +2706,7 @@ crava_status crava_job_local_noise(crava_job* job, const float* scales, void* st
   }
   for (int q = 0; q < 3 * d.nsim; q++) P.sim[q] = job->sim[q];
   float* dscale = nullptr;
-  CUDA_TRY(cudaMallocAsync((void**)&dscale, sizeof(float) * (n + 18) * nxy, st));
+  CUDA_TRY(scratch_alloc(job->ctx, (void**)&dscale, sizeof(float) * (n + 18) * nxy, st));
   P.scale = dscale;
   P.maps = dscale + n * nxy;
   cudaError_t e = cudaMemcpyAsync(dscale, scales, sizeof(float) * n * nxy, cudaMemcpyHostToDevice, st);
@@ -2734,7 +2767,7 @@ static crava_status fill_prior_impl(crava_job* job, const float* act_host, float
   if (act_host) {
     for (size_t q = 0; q < 6 * (size_t)d.nzp; q++)
       if (!std::isfinite(act_host[q])) return fail(CRAVA_ENUMERIC, "non-finite auto-covariance");
-    CUDA_TRY(cudaMallocAsync((void**)&dact, sizeof(float) * 6 * d.nzp, st));
+    CUDA_TRY(scratch_alloc(job->ctx, (void**)&dact, sizeof(float) * 6 * d.nzp, st));
     CUDA_TRY(cudaMemcpyAsync(dact, act_host, sizeof(float) * 6 * d.nzp, cudaMemcpyHostToDevice, st));
     P.act = dact;
   }
@@ -3803,34 +3836,12 @@ crava_status crava_facies_smooth(crava_ctx* ctx, const crava_facies_desc* fd, co
   const int rna = 2 * (na / 2 + 1);
   const size_t gsize = (size_t)rna * nb * nr;
   // Gaussian smoother with cyclic bin offsets, exp in float, normalised to unit sum
-  // (src/faciesprob.cpp:447-496)
-  std::vector<float> sm((size_t)na * nb * nr);
-  float sum = 0.0f;
-  const double dv0 = fd->dv[0], dv1 = fd->dv[1], dv2 = fd->dv[2];
-  const double* S = sigma_inv;
-  for (int l = 0; l < nr; l++) {
-    int ll = l <= nr / 2 ? l : l - nr;
-    for (int k = 0; k < nb; k++) {
-      int kk = k <= nb / 2 ? k : k - nb;
-      for (int j = 0; j < na; j++) {
-        int jj = j <= na / 2 ? j : j - na;
-        float factor = static_cast<float>(jj * dv0 * jj * dv0 * S[0] + kk * dv1 * kk * dv1 * S[4] +
-                                          ll * dv2 * ll * dv2 * S[8] + 2 * jj * dv0 * kk * dv1 * S[3] +
-                                          2 * jj * dv0 * ll * dv2 * S[6] + 2 * kk * dv1 * ll * dv2 * S[7]);
-        float v = std::exp(-0.5f * factor);
-        sm[j + (size_t)k * na + (size_t)l * na * nb] = v;
-        sum += v;
-      }
-    }
-  }
-  std::vector<float> g(gsize, 0.f);
-  for (int l = 0; l < nr; l++)
-    for (int k = 0; k < nb; k++)
-      for (int j = 0; j < na; j++) g[j + (size_t)rna * (k + (size_t)nb * l)] = sm[j + (size_t)k * na + (size_t)l * na * nb] / sum;
+  // (src/faciesprob.cpp:447-496); its sum in the last word
   float* d_sm = nullptr;
-  CUDA_TRY(cudaMalloc(&d_sm, sizeof(float) * gsize));
+  CUDA_TRY(scratch_alloc(ctx, (void**)&d_sm, sizeof(float) * (align256(gsize) + 1), st));
   crava_status s = CRAVA_OK;
-  cudaError_t e = cudaMemcpyAsync(d_sm, g.data(), sizeof(float) * gsize, cudaMemcpyHostToDevice, st);
+  int nl = 0;
+  cudaError_t e = launch_facies_smoother(d_sm, d_sm + align256(gsize), na, nb, nr, fd->dv, sigma_inv, st, &nl);
   // PARAMETER-scaled transforms: smoothed = IFFT(FFT(h)/sqrt(N) * FFT(s)/sqrt(N))/sqrt(N) * sqrt(N)
   const size_t N = (size_t)na * nb * nr;
   const float fs = fwd_scale(N);
@@ -3846,7 +3857,7 @@ crava_status crava_facies_smooth(crava_ctx* ctx, const crava_facies_desc* fd, co
     sc.push_back(fs);
   }
   if (e == cudaSuccess) s = fwd_xy(ctx, src, gr, sc, na, nb, nr, true, st);
-  else s = cuda_fail(e, "cudaMemcpyAsync");
+  else s = cuda_fail(e, "launch_facies_smoother");
   const size_t nbins = (size_t)(na / 2 + 1) * nb * nr;
   for (int f = 0; f < fd->nfacies && !s; f++) {
     e = launch_spec_mul((float2*)(d_hist + gsize * f), (const float2*)d_sm, nbins, st);
@@ -3858,8 +3869,9 @@ crava_status crava_facies_smooth(crava_ctx* ctx, const crava_facies_desc* fd, co
     std::vector<float> osc(out.size(), is);
     s = inv_xy(ctx, out, osc, na, nb, nr, true, st);
   }
+  ctx->launches += nl;
+  cudaFreeAsync(d_sm, st);
   cudaStreamSynchronize(st);
-  cudaFree(d_sm);
   return s;
 }
 
@@ -3931,7 +3943,7 @@ crava_status crava_facies_prob_local_noise(crava_ctx* ctx, const crava_facies_de
   cudaStream_t st = (cudaStream_t)stream;
   float* dt = nullptr;
   if (nang > 0) {
-    CUDA_TRY(cudaMallocAsync((void**)&dt, sizeof(float) * t.size(), st));
+    CUDA_TRY(scratch_alloc(ctx, (void**)&dt, sizeof(float) * t.size(), st));
     CUDA_TRY(cudaMemcpyAsync(dt, t.data(), sizeof(float) * t.size(), cudaMemcpyHostToDevice, st));
   }
   hc.t = dt;
@@ -3939,10 +3951,11 @@ crava_status crava_facies_prob_local_noise(crava_ctx* ctx, const crava_facies_de
   size_t pbytes = 0;
   for (int c = 0; c < nc; c++) pbytes += align256(facies_packed_bytes(hc.box[c], fd->nfacies));
   char* pk = nullptr;
-  CUDA_TRY(cudaMallocAsync((void**)&pk, pbytes, st));
-  for (int c = 0, off = 0; c < nc; c++) {
+  CUDA_TRY(scratch_alloc(ctx, (void**)&pk, pbytes, st));
+  size_t off = 0;
+  for (int c = 0; c < nc; c++) {
     hc.packed[c] = (float4*)(pk + off);
-    off += (int)align256(facies_packed_bytes(hc.box[c], fd->nfacies));
+    off += align256(facies_packed_bytes(hc.box[c], fd->nfacies));
   }
   // undefSum = p_undefined / (bins of the first density volume), as the reference
   const float undef_sum = fd->p_undefined / (float)(fd->nbins[0] * fd->nbins[1] * fd->nbins[2]);

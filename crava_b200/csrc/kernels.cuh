@@ -273,6 +273,8 @@ struct EigLayout {
   }
 };
 // facies.cu: prior[] and out[] are host arrays (copied into the launch parameters)
+cudaError_t launch_facies_smoother(float* g, float* sum, int na, int nb, int nr, const double* dv, const double* S,
+                                   cudaStream_t st, int* nlaunch);
 cudaError_t launch_spec_mul(float2* a, const float2* b, size_t n, cudaStream_t st);
 // gridio.cu: dst[e] = src[e] with the byte order of every 4-byte word reversed (dst == src
 // allowed)
