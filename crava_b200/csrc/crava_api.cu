@@ -654,6 +654,12 @@ void build_kz_tables(const crava_job_desc& d, std::vector<float2>& kw, std::vect
   }
 }
 
+// Jobs whose pencil pass is the scalar one (zpass.cuh): residual spectra kept, at the z lengths where
+// pencil.cuh's transform has another order of roundings.
+bool pencil_scalar(const crava_job_desc* d) {
+  return (d->flags & CRAVA_FLAG_KEEP_RESIDUAL) && d->nzp != 128 && d->nzp != 256 && d->nzp != 320;
+}
+
 // Eigen tables of a separable-prior job: bytes on the device (0 for other priors).
 size_t eig_table_bytes(const crava_job_desc* d) {
   if (d->prior_mode != CRAVA_PRIOR_SEPARABLE) return 0;
@@ -723,7 +729,7 @@ void sep_constants(const std::vector<double>& A, const std::vector<double>& pv, 
 
 // Tables of the eigen form of the separable posterior (pencil.cuh), one row per z position
 // in the order the in-place z transform leaves the spectrum in (position p holds kz =
-// pencil_kz(p)), float4 group g of position p at rows[4 (g nzp + p)].
+// pencil_kz(p); natural order for the jobs of zpass.cuh), float4 group g of position p at rows[4 (g nzp + p)].
 // Per inverted kz, from the float values the Cholesky form uses (kw, M2 = the septab
 // lower triangle, ed, |ct|, G0 = A P0 A^T, AP = A P0):
 //   M = |ct| (kw kw^H) o G0 + M2,  E = diag(ed),  E^-1/2 M E^-1/2 = U diag(Lam) U^H,
@@ -741,13 +747,14 @@ bool build_eig_tables(const crava_job_desc& d, const std::vector<float2>& kw, co
   const int n = d.ntheta, nzp = d.nzp;
   ZPlan zplan;
   if (!pencil_plan(nzp, zplan)) { why = "z length has no plan"; return false; }
+  const bool scalar_z = pencil_scalar(&d);
   const EigLayout L(n);
   const int G4 = L.floats / 4;
   rows.assign((size_t)L.floats * nzp, 0.f);
   n_inv_rows = 0;
   const int tri = n * (n + 1) / 2;
   for (int p = 0; p < nzp; p++) {
-    const int kz = pencil_kz(zplan, p);
+    const int kz = scalar_z ? p : pencil_kz(zplan, p);
     if (!inv[kz]) continue;
     n_inv_rows++;
     double row[4 * 96] = {};
@@ -999,7 +1006,8 @@ float inv_scale(size_t N, bool cov) {
 // 3D transforms of a list of grids (x, y[, z]) -- the FFTGrid::fftInPlace work split over
 // batched launches.
 crava_status fwd_xy(crava_ctx* ctx, const std::vector<const float*>& src, const std::vector<float*>& g,
-                    const std::vector<float>& sc, int nxp, int nyp, int nzp, bool with_z, cudaStream_t st) {
+                    const std::vector<float>& sc, int nxp, int nyp, int nzp, bool with_z, cudaStream_t st,
+                    bool plain = false) {
   if (g.empty()) return CRAVA_OK;
   Plan *px, *pn, *py, *pz;
   crava_status s;
@@ -1008,6 +1016,7 @@ crava_status fwd_xy(crava_ctx* ctx, const std::vector<const float*>& src, const 
   int nl = 0;
   for (size_t b = 0; b < g.size(); b += kMaxGrids) {
     GridSet gs;
+    gs.plain = plain;
     gs.n = (int)std::min(g.size() - b, (size_t)kMaxGrids);
     for (int q = 0; q < gs.n; q++) { gs.p[q] = g[b + q]; gs.src[q] = src[b + q]; gs.scale[q] = sc[b + q]; }
     {
@@ -1976,6 +1985,7 @@ crava_status lat_set_build(crava_ctx* ctx, const crava_job_desc& d, const std::v
   if ((ps = get_xplans(ctx, d.nxp, &px, &pn)) || (ps = get_plan(ctx, d.nyp, &py))) return ps;
   GridSet gs;
   gs.n = 1;
+  gs.plain = (d.flags & CRAVA_FLAG_KEEP_RESIDUAL) != 0;   // zpass.cuh
   gs.p[0] = l.grid;
   gs.src[0] = l.grid;
   gs.scale[0] = 1.0f;
@@ -1995,9 +2005,10 @@ void key_put(std::string& k, const T* p, size_t n) {
 }
 std::string kz_key(const crava_job_desc& d) {
   std::string k = "K";
-  const int iv[6] = {d.nz, d.nzp, d.ntheta, d.prior_mode, d.flags & CRAVA_FLAG_NONCONST_THICK,
-                     d.fp64_threshold > 0.f ? 1 : 0};
-  key_put(k, iv, 6);
+  // (pencil_scalar: the eigen tables' order)
+  const int iv[7] = {d.nz, d.nzp, d.ntheta, d.prior_mode, d.flags & CRAVA_FLAG_NONCONST_THICK,
+                     d.fp64_threshold > 0.f ? 1 : 0, pencil_scalar(&d) ? 1 : 0};
+  key_put(k, iv, 7);
   const double dv[2] = {d.lz, d.min_rel_thick};
   key_put(k, dv, 2);
   const float fv[3] = {d.low_cut, d.high_cut, d.wnc};
@@ -2012,8 +2023,8 @@ std::string kz_key(const crava_job_desc& d) {
 }
 std::string lat_key(const crava_job_desc& d) {
   std::string k = "L";
-  const int iv[2] = {d.nxp, d.nyp};
-  key_put(k, iv, 2);
+  const int iv[3] = {d.nxp, d.nyp, (d.flags & CRAVA_FLAG_KEEP_RESIDUAL) ? 1 : 0};
+  key_put(k, iv, 3);
   key_put(k, d.corr_xy, (size_t)d.nxp * d.nyp);
   return k;
 }
@@ -2460,7 +2471,8 @@ crava_status crava_job_run(crava_job* job, void* stream) {
     std::vector<float> sc;
     for (int l = 0; l < d.ntheta; l++) { src.push_back(job->in_data[l]); g.push_back(job->data[l]); sc.push_back(fs); }
     for (int a = 0; a < 3; a++) { src.push_back(job->in_mean[a]); g.push_back(job->mean[a]); sc.push_back(fs); }
-    if ((s = fwd_xy(ctx, src, g, sc, d.nxp, d.nyp, d.nzp, false, st))) return s;
+    // residual spectra keep the scalar transforms' roundings (zpass.cuh)
+    if ((s = fwd_xy(ctx, src, g, sc, d.nxp, d.nyp, d.nzp, false, st, (d.flags & CRAVA_FLAG_KEEP_RESIDUAL) != 0))) return s;
   }
   if (grids) {
     std::vector<const float*> src;
@@ -2477,7 +2489,8 @@ crava_status crava_job_run(crava_job* job, void* stream) {
   }
   // the fused pencil pass
   Plan* pz;
-  if ((s = get_plan(ctx, d.nzp, &pz))) return s;
+  const bool scalar_z = pencil_scalar(&d);
+  if ((s = get_plan(ctx, d.nzp, &pz, scalar_z))) return s;
   ZParams zp;
   std::memset(&zp, 0, sizeof(zp));
   zp.nxp = d.nxp; zp.nyp = d.nyp; zp.nzp = d.nzp; zp.cnxp = job->cnxp;
@@ -2529,10 +2542,12 @@ crava_status crava_job_run(crava_job* job, void* stream) {
     zp.eig = job->eig;
     zp.n_inv_rows = job->n_inv_rows;
   }
-  if (!pencil_shape(zp, &threads)) return fail(CRAVA_ENOTSUP, "pencil tile does not fit in shared memory");
+  if (scalar_z ? !zpass_shape(zp, &threads) : !pencil_shape(zp, &threads))
+    return fail(CRAVA_ENOTSUP, "pencil tile does not fit in shared memory");
+  zp.zp = pz->lp;
   {
     ProfScope ps(ctx, KT_ZPASS, st);
-    CUDA_TRY(launch_pencil(zp, threads, st, &nl));
+    CUDA_TRY(scalar_z ? launch_zpass(zp, threads, st, &nl) : launch_pencil(zp, threads, st, &nl));
   }
   ctx->launches += nl;
   // inverse transforms (y, x) of the outputs with FFTGrid::invFFTInPlace scales
@@ -3365,7 +3380,8 @@ crava_status prewarm_plans(crava_ctx* ctx, const crava_job_desc& d) {
   crava_status s;
   if ((s = get_xplans(ctx, d.nxp, &a, &b))) return s;
   if ((s = get_plan(ctx, d.nyp, &a))) return s;
-  return get_plan(ctx, d.nzp, &a);
+  if ((s = get_plan(ctx, d.nzp, &a))) return s;
+  return get_plan(ctx, d.nzp, &a, pencil_scalar(&d));
 }
 
 }  // namespace

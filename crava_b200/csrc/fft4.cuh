@@ -3,8 +3,8 @@
 // same transforms as k_x_r2c / k_x_c2r / k_line_fft (kernels.cu), with each line done in
 // two register-codelet passes (fft2.cuh) instead of one shared-memory stage per radix.
 //
-//   k_line4<N1,N2,DIR>  W columns of one strided line set: global -> pass 1 -> shared
-//                       -> pass 2 -> global
+//   k_line4<N,DIR>      W columns of one strided line set, in pairs: global -> first stage -> shared (->
+//                       middle stage) -> last stage -> global; k_line4s<N1,N2,DIR> the same one by one
 //   k_xr2c4<N1,N2>      rows of even nxp, h = nxp/2 = N1 N2: global -> shared -> pass 1 -> shared
 //                       -> pass 2 and split -> shared -> global
 //   k_xc2r4<N1,N2>      global -> shared -> merge and pass 1 -> shared -> pass 2 -> shared -> global
@@ -16,12 +16,132 @@
 #include <algorithm>
 #include <cstdlib>
 
-#include "fft2.cuh"
+#include "fft_pair.cuh"
 #include "kernels.cuh"
 
 namespace crava {
 
+// shared layout of the kernels: n twiddles (rounded up to an even count, so that what follows starts on
+// 16 bytes), the tile or the staged rows, the exchange buffer of the scalar row passes
+constexpr int even_up(int n) { return (n + 1) & ~1; }
+
 // ------------------------------------------------------------------ strided lines
+//
+// W columns (NP = W / 2 pairs of columns q, q + NP, C2 of fft_pair.cuh) of n = R0 R1 R2 points in two
+// (R2 = 1) or three stages: the first reads global memory and leaves its results in the tile, the last
+// stores to global memory in natural order.  With N1 = R1 R2 the decimation-in-frequency stages
+// are
+//   stage 0, item t < N1         x[t + N1 m] -> DFT_R0 -> w^(t k0)          at k0 N1 + t
+//   stage 1, item (k0, t < R2)   at k0 N1 + t + R2 m -> DFT_R1 -> w^(R0 t k1)  at k0 N1 + k1 R2 + t
+//   last stage, item b           at b R + m -> DFT_R -> X[rev(b) + (n / R) k]
+// rev(b) = k0 + R0 k1 for b = k0 R1 + k1.  Radices of 16 at most keep a pair's data in 64 registers.
+//
+// Tile word (position p, pair q) at 16 (p NP + q) bytes: 8 pairs, a whole 128-byte line of banks.
+struct ColSplit {
+  int r0, r1, r2;
+};
+constexpr ColSplit col_split(int n) {
+  for (int a = 2; a <= 16; a++)
+    if (n % a == 0 && n / a <= a) return {a, n / a, 1};          // smallest larger factor
+  for (int top = 2; top <= 32; top++)
+    for (int a = top; a >= 2; a--) {
+      if (n % a) continue;
+      for (int b = a; b >= 2; b--)
+        if ((n / a) % b == 0 && n / a / b <= b) return {a, b, n / a / b};
+    }
+  return {0, 0, 0};
+}
+
+template <int R, int DIR>
+__device__ __forceinline__ void col_twiddle(C2 (&v)[R], const float2* tw, int step) {
+#pragma unroll
+  for (int k = 1; k < R; k++) {
+    const float2 w = tw[step * k];
+    v[k] = c2_mul(v[k], w.x, DIR < 0 ? w.y : -w.y);
+  }
+}
+
+template <int N, int DIR>
+__global__ void __launch_bounds__(256, col_split(N).r0 <= 10 ? 4 : col_split(N).r0 <= 12 ? 3 : 2) k_line4(const __grid_constant__ GridSet gs, int ni, size_t pstride,
+                                               size_t ostride, int lnp, int nIT, const float2* __restrict__ twg) {
+  constexpr ColSplit S = col_split(N);
+  constexpr int R0 = S.r0, R1 = S.r1, R2 = S.r2, N1 = R1 * R2, RL = R2 > 1 ? R2 : R1;
+  extern __shared__ __align__(16) float2 sm[];
+  float2* tw = sm;
+  const uint32_t Y = smem_addr(sm + even_up(N));
+  const int T = blockDim.x, tid = threadIdx.x, NP = 1 << lnp, W = 2 * NP;
+  const int it = blockIdx.x % nIT, o = blockIdx.x / nIT;
+  const int i0 = it * W, nw = min(W, ni - i0);
+  float2* g = reinterpret_cast<float2*>(gs.p[blockIdx.y]) + (size_t)o * ostride + i0;
+  const uint32_t ps = 16u << lnp;
+  for (int t = tid; t < N; t += T) tw[t] = twg[t];
+  bool first = true;
+#pragma unroll 1
+  for (int e = tid; e < NP * N1 || first; e += T) {
+    const int q = e & (NP - 1), t = e >> lnp;
+    const bool on = e < NP * N1, in0 = on && q < nw, in1 = on && q + NP < nw;
+    C2 v[R0];
+    {
+      const float2* src = g + (size_t)t * pstride + q;
+      const size_t st = (size_t)N1 * pstride;
+#pragma unroll
+      for (int m = 0; m < R0; m++, src += st) {
+        const float2 a = in0 ? src[0] : make_float2(0.f, 0.f), b = in1 ? src[NP] : make_float2(0.f, 0.f);
+        v[m] = {make_float2(a.x, b.x), make_float2(a.y, b.y)};
+      }
+    }
+    DftP<R0, DIR>::run(v);
+    if (first) {          // the table, staged behind the loads
+      __syncthreads();
+      first = false;
+    }
+    if (!on) break;
+    col_twiddle<R0, DIR>(v, tw, t);
+    const uint32_t y = Y + (uint32_t)t * ps + 16u * (uint32_t)q;
+#pragma unroll
+    for (int k = 0; k < R0; k++) sts_c2(y + (uint32_t)(k * N1) * ps, v[k]);
+  }
+  __syncthreads();
+  if constexpr (R2 > 1) {
+#pragma unroll 1
+    for (int e = tid; e < NP * R0 * R2; e += T) {
+      const int q = e & (NP - 1), j = e >> lnp, k0 = j / R2, t = j - k0 * R2;
+      const uint32_t y = Y + (uint32_t)(k0 * N1 + t) * ps + 16u * (uint32_t)q;
+      C2 v[R1];
+#pragma unroll
+      for (int m = 0; m < R1; m++) v[m] = lds_c2(y + (uint32_t)(m * R2) * ps);
+      DftP<R1, DIR>::run(v);
+      col_twiddle<R1, DIR>(v, tw, R0 * t);
+#pragma unroll
+      for (int k = 0; k < R1; k++) sts_c2(y + (uint32_t)(k * R2) * ps, v[k]);
+    }
+    __syncthreads();
+  }
+#pragma unroll 1
+  for (int e = tid; e < NP * (N / RL); e += T) {
+    const int q = e & (NP - 1), b = e >> lnp;
+    const uint32_t y = Y + (uint32_t)(b * RL) * ps + 16u * (uint32_t)q;
+    C2 v[RL];
+#pragma unroll
+    for (int m = 0; m < RL; m++) v[m] = lds_c2(y + (uint32_t)m * ps);
+    DftP<RL, DIR>::run(v);
+    const int k0 = R2 > 1 ? b / R1 : b, rev = R2 > 1 ? k0 + R0 * (b - k0 * R1) : b;
+    float2* dst = g + (size_t)rev * pstride + q;
+    const size_t st = (size_t)(N / RL) * pstride;
+    if (q + NP < nw) {
+#pragma unroll
+      for (int k = 0; k < RL; k++, dst += st) {
+        dst[0] = make_float2(v[k].r.x, v[k].i.x);
+        dst[NP] = make_float2(v[k].r.y, v[k].i.y);
+      }
+    } else if (q < nw) {
+#pragma unroll
+      for (int k = 0; k < RL; k++, dst += st) dst[0] = make_float2(v[k].r.x, v[k].i.x);
+    }
+  }
+}
+
+// The scalar two-pass form of the longer lengths (line4 below says which), one column an item.
 //
 // One tile of W columns (nw of them valid) of the lines through g: point p of column w at
 // g[p pstride + w], read from src[p spstride + w] (g itself, or a staged copy of the tile in
@@ -66,7 +186,7 @@ constexpr size_t line4_smem(int W, int SK) {
 // Forward instances bounded at 256 threads (the register allocation the forward passes were
 // tuned with), inverse ones at 512 (a CTA may take one pass in a single round).
 template <int N1, int N2, int DIR>
-__global__ void __launch_bounds__(DIR > 0 ? 512 : 256) k_line4(const __grid_constant__ GridSet gs, int ni, size_t pstride,
+__global__ void __launch_bounds__(DIR > 0 ? 512 : 256) k_line4s(const __grid_constant__ GridSet gs, int ni, size_t pstride,
                                                size_t ostride, int W, int lw, int nIT, int SK,
                                                const float2* __restrict__ twg, int pf) {
   constexpr int N = N1 * N2;
@@ -168,11 +288,10 @@ __device__ __forceinline__ void xr2c4_rows(const float2* src, float2* dst, int n
 
 // nr rows of half spectra staged in Xs (shared, pitch h + 1) to scaled real rows in g (Xs
 // itself, or global memory; same pitch); the merge step as k_x_c2r (kernels.cu).  Z: rpc * PITCH.
-// Ends with a barrier.  COPY: the real rows also go
-// to Vc (shared, row r at r * h pairs of samples).
-template <int N1, int N2, bool COPY = false>
+// Ends with a barrier.
+template <int N1, int N2>
 __device__ __forceinline__ void xc2r4_staged(const float2* Xs, float2* g, int nr, float scale, const float2* tw,
-                                             const float2* twh, float2* Z, float2* Vc = nullptr) {
+                                             const float2* twh, float2* Z) {
   using L = RowLayout<N1, N2>;
   constexpr int H = L::H, PITCH = L::PITCH;
   constexpr int CN = H + 1;
@@ -215,11 +334,94 @@ __device__ __forceinline__ void xc2r4_staged(const float2* Xs, float2* g, int nr
     for (int k1 = 0; k1 < N2; k1++) {
       const float2 o = make_float2(v[k1].x * scale, v[k1].y * scale);
       X[k2 + N1 * k1] = o;
-      if (COPY) Vc[r * H + k2 + N1 * k1] = o;
     }
     if (k2 == 0) X[H] = make_float2(0.f, 0.f);
   }
   __syncthreads();
+}
+
+// ------------------------------------------------------------------ inverse rows in pairs
+//
+// The inverse row transform of two rows at once (C2, fft_pair.cuh: the merge, both DFTs and the twiddles
+// as packed instructions, one table read for both rows, the exchange between the passes in 16-byte words):
+// 101 -> about 50 instructions a point at h = 270, where the scalar form ran at 60 % of the
+// issue slots.  One buffer serves the staged rows, the exchange words and the real rows: a thread
+// has at most one item per pass, so all reads of a pass are over at the barrier before its writes.
+// Lengths with N1 <= 24 (4 N1 registers of data); longer factors keep xc2r4_staged.
+//
+// B: the rows, pitch h + 1, pair p = rows 2 p, 2 p + 1; word (t, k2) of a pair's exchange buffer at
+// t + k2 WS, an odd stride.  T >= ceil(nr / 2) max(N1, N2).  The real rows are left in B (the caller
+// synchronises).
+template <int N1, int N2>
+struct RowPairs {
+  static constexpr bool ok = N1 <= 24;
+  static constexpr int H = N1 * N2, CN = H + 1, WS = N2 + (N2 % 2 == 0), PITCH = N1 * WS;
+  // float2 of the buffer of np pairs
+  static constexpr int words(int np) { return np * (2 * PITCH > 2 * CN ? 2 * PITCH : 2 * CN); }
+};
+template <int N1, int N2>
+__device__ __forceinline__ void xc2r4_pairs(float2* B, int nr, float scale, const float2* tw, const float2* twh) {
+  using L = RowPairs<N1, N2>;
+  constexpr int H = L::H, CN = L::CN;
+  const int np = (nr + 1) >> 1, tid = threadIdx.x;
+  const uint32_t zb = smem_addr(B);
+  C2 v[N1];
+  const bool on1 = tid < np * N2;
+  const int p1 = tid / N2, t = tid - p1 * N2;
+  if (on1) {
+    const float2* X0 = B + 2 * p1 * CN;
+    const float2* X1 = 2 * p1 + 1 < nr ? X0 + CN : X0;
+#pragma unroll
+    for (int m = 0; m < N1; m++) {
+      // z[k] = (X[k] + conj X[h-k]) + i w^k (X[k] - conj X[h-k]), w = e^{2 pi i / nxp}; a real-output
+      // inverse has no slot for Im X[0], Im X[h]
+      const int k = t + N2 * m;
+      float2 a0 = X0[k], b0 = X0[H - k], a1 = X1[k], b1 = X1[H - k];
+      if (m == 0 && t == 0) a0.y = b0.y = a1.y = b1.y = 0.f;
+      const float2 w = twh[k];
+      const float2 ar = make_float2(a0.x, a1.x), ai = make_float2(a0.y, a1.y);
+      const float2 br = make_float2(b0.x, b1.x), bi = make_float2(b0.y, b1.y);
+      const float2 pr = f2_add(ar, br), pi = f2_sub(ai, bi), mr = f2_sub(ar, br), mi = f2_add(ai, bi);
+      const float2 qr = f2_fma(mi, f2_dup(w.y), f2_mul(mr, f2_dup(w.x)));
+      const float2 qi = f2_fma(mr, f2_dup(-w.y), f2_mul(mi, f2_dup(w.x)));
+      v[m] = {f2_sub(pr, qi), f2_add(pi, qr)};
+    }
+    DftP<N1, 1>::run(v);
+#pragma unroll
+    for (int k2 = 1; k2 < N1; k2++) {
+      const float2 w = tw[t * k2];
+      v[k2] = c2_mul(v[k2], w.x, -w.y);
+    }
+  }
+  __syncthreads();
+  if (on1) {
+#pragma unroll
+    for (int k2 = 0; k2 < N1; k2++) sts_c2(zb + 16u * (uint32_t)(p1 * L::PITCH + t + k2 * L::WS), v[k2]);
+  }
+  __syncthreads();
+  const bool on2 = tid < np * N1;
+  const int p2 = tid / N1, k2 = tid - p2 * N1;
+  C2 u[N2];
+  if (on2) {
+#pragma unroll
+    for (int t2 = 0; t2 < N2; t2++) u[t2] = lds_c2(zb + 16u * (uint32_t)(p2 * L::PITCH + t2 + k2 * L::WS));
+    DftP<N2, 1>::run(u);
+  }
+  __syncthreads();
+  if (on2) {
+    float2* R0 = B + 2 * p2 * CN;
+    const bool two = 2 * p2 + 1 < nr;
+#pragma unroll
+    for (int k1 = 0; k1 < N2; k1++) {
+      const float2 r = f2_mul(u[k1].r, f2_dup(scale)), i = f2_mul(u[k1].i, f2_dup(scale));
+      R0[k2 + N1 * k1] = make_float2(r.x, i.x);
+      if (two) R0[CN + k2 + N1 * k1] = make_float2(r.y, i.y);
+    }
+    if (k2 == 0) {
+      R0[H] = make_float2(0.f, 0.f);
+      if (two) R0[CN + H] = make_float2(0.f, 0.f);
+    }
+  }
 }
 
 // L2 prefetch of the row chunk pf block indices on (x fastest): rows of (h + 1) complex values,
@@ -281,10 +483,6 @@ __device__ __forceinline__ void rows_out(float2* dst, const float2* src, int n, 
   }
 }
 
-// shared layout of the row kernels: nt twiddles (rounded up to an even count, so that the rows
-// start on 16 bytes), the staged rows, the exchange buffer of the two passes
-constexpr int even_up(int n) { return (n + 1) & ~1; }
-
 // The forward rows keep their loads and stores in the passes: pass 1's loads are the first thing a
 // thread does and pass 2 stores runs of N1 points; staged both ways they measured slower (540x540x256:
 // 1.24 against 1.18 ms; staged stores alone the same), the rows' second buffer costing resident CTAs.
@@ -328,7 +526,6 @@ __global__ void __launch_bounds__(256) k_xc2r4(const __grid_constant__ GridSet g
   float2* tw = sm;
   float2* twh = tw + H;
   float2* Xs = sm + 2 * H;
-  float2* Z = Xs + even_up(rpc * CN);
   const int row0 = blockIdx.x * rpc, nr = min(rpc, rows - row0);
   float2* g = reinterpret_cast<float2*>(gs.p[blockIdx.y]) + (size_t)row0 * CN;
   rows_in(Xs, g, nr * CN, al16);
@@ -339,7 +536,8 @@ __global__ void __launch_bounds__(256) k_xc2r4(const __grid_constant__ GridSet g
   }
   cp_async_wait_0();
   __syncthreads();
-  xc2r4_staged<N1, N2>(Xs, Xs, nr, gs.scale[blockIdx.y], tw, twh, Z);
+  if constexpr (RowPairs<N1, N2>::ok) xc2r4_pairs<N1, N2>(Xs, nr, gs.scale[blockIdx.y], tw, twh);
+  else xc2r4_staged<N1, N2>(Xs, Xs, nr, gs.scale[blockIdx.y], tw, twh, Xs + even_up(rpc * CN));
   rows_out(g, Xs, nr * CN, al16);
 }
 
@@ -483,7 +681,7 @@ static inline bool four_step_enabled(int n) { return tuned("four_step", n, 1) !=
 static inline int round_up32(int t) { return std::max(64, (t + 31) / 32 * 32); }
 
 template <int N1, int N2>
-static cudaError_t line4(const GridSet& gs, int ni, size_t pstride, int no, size_t ostride, const float2* tw,
+static cudaError_t line4_scalar(const GridSet& gs, int ni, size_t pstride, int no, size_t ostride, const float2* tw,
                          float sign, cudaStream_t st) {
   constexpr int N = N1 * N2;
   // 8-column tiles; 16 for inverse transforms up to 540 points (measured faster there,
@@ -502,7 +700,7 @@ static cudaError_t line4(const GridSet& gs, int ni, size_t pstride, int no, size
                             tuned(sign < 0.f ? "line4_threads_fwd" : "line4_threads_inv", N, T) / 32 * 32));
   const int nIT = (ni + W - 1) / W;
   const size_t smem = sizeof(float2) * (size_t)N + line4_smem<N1, N2>(W, SK);
-  const void* fn = sign < 0.f ? (const void*)k_line4<N1, N2, -1> : (const void*)k_line4<N1, N2, 1>;
+  const void* fn = sign < 0.f ? (const void*)k_line4s<N1, N2, -1> : (const void*)k_line4s<N1, N2, 1>;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   dim3 grid((unsigned)(nIT * no), gs.n);
@@ -514,9 +712,47 @@ static cudaError_t line4(const GridSet& gs, int ni, size_t pstride, int no, size
     if ((e = resident_grid(fn, T, smem, 1 << 30, &res)) != cudaSuccess) return e;
     pf = std::max(1, res * q / 4);
   }
-  if (sign < 0.f) k_line4<N1, N2, -1><<<grid, T, smem, st>>>(gs, ni, pstride, ostride, W, lw, nIT, SK, tw, pf);
-  else k_line4<N1, N2, 1><<<grid, T, smem, st>>>(gs, ni, pstride, ostride, W, lw, nIT, SK, tw, pf);
+  if (sign < 0.f) k_line4s<N1, N2, -1><<<grid, T, smem, st>>>(gs, ni, pstride, ostride, W, lw, nIT, SK, tw, pf);
+  else k_line4s<N1, N2, 1><<<grid, T, smem, st>>>(gs, ni, pstride, ostride, W, lw, nIT, SK, tw, pf);
   return cudaGetLastError();
+}
+
+template <int N>
+static cudaError_t line4_pairs(const GridSet& gs, int ni, size_t pstride, int no, size_t ostride, const float2* tw,
+                               float sign, cudaStream_t st) {
+  constexpr ColSplit S = col_split(N);
+  // 16-column tiles (rows of 128 bytes); narrower where the grid is
+  int W = std::max(2, std::min(16, tuned(sign < 0.f ? "line4_w_fwd" : "line4_w_inv", N, 16)));
+  while (W > 2 && W / 2 >= ni) W /= 2;
+  int lnp = 0;
+  while ((4 << lnp) <= W) lnp++;
+  W = 2 << lnp;
+  const size_t smem = sizeof(float2) * ((size_t)even_up(N) + (size_t)W * N);
+  // threads: the items of the first stage in as few rounds of at most 256 threads as they take
+  const int items = (W / 2) * (N / S.r0), rounds = (items + 255) / 256;
+  int T = round_up32((items + rounds - 1) / rounds);
+  T = std::max(64, std::min(256, tuned(sign < 0.f ? "line4_threads_fwd" : "line4_threads_inv", N, T) / 32 * 32));
+  const int nIT = (ni + W - 1) / W;
+  const void* fn = sign < 0.f ? (const void*)k_line4<N, -1> : (const void*)k_line4<N, 1>;
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  dim3 grid((unsigned)(nIT * no), gs.n);
+  if (sign < 0.f) k_line4<N, -1><<<grid, T, smem, st>>>(gs, ni, pstride, ostride, lnp, nIT, tw);
+  else k_line4<N, 1><<<grid, T, smem, st>>>(gs, ni, pstride, ostride, lnp, nIT, tw);
+  return cudaGetLastError();
+}
+
+// Pairs up to 270 points: with 250 x-points, 21 grids of 60 planes, 5 % faster or equal at lengths of two
+// factors up to 16, 1.3 to 1.9 times at the lopsided ones (125 = 25 x 5, 250 = 25 x 10) that then
+// take three stages; above, three stages cost more than the scalar form's two (288 to 1024 points:
+// 0.65 to 1.05 of its speed).
+template <int N1, int N2>
+static cudaError_t line4(const GridSet& gs, int ni, size_t pstride, int no, size_t ostride, const float2* tw,
+                         float sign, cudaStream_t st) {
+  if constexpr (N1 * N2 <= 270) {
+    if (!gs.plain || sign > 0.f) return line4_pairs<N1 * N2>(gs, ni, pstride, no, ostride, tw, sign, st);
+  }
+  return line4_scalar<N1, N2>(gs, ni, pstride, no, ostride, tw, sign, st);
 }
 
 // Threads and lines per CTA of a row kernel whose passes have i1 and i2 items per line of c1 and
@@ -552,10 +788,31 @@ static inline bool grids_al16(const GridSet& gs) {
   return a % 16 == 0;
 }
 
+// Row pairs per CTA of xc2r4_pairs: one item per thread and pass, by the same estimate as row_shape.
+template <int N1, int N2>
+static inline int pair_count() {
+  using L = RowPairs<N1, N2>;
+  int best = 1;
+  double least = 1e30;
+  for (int np = 1; np * N1 <= 256; np++) {
+    const size_t smem = sizeof(float2) * (2 * (size_t)L::H + L::words(np)) + 1024;
+    if (np > 1 && smem > 37 * 1024) break;
+    const int T = std::max(64, (np * N1 + 31) / 32 * 32);
+    const int ctas = std::min(32, std::min((int)(227 * 1024 / smem), 65536 / ((4 * N1 + 40) * T)));
+    const double t = (40.0 / std::max(1, ctas) + 2.5 * T / 32) / np;
+    if (t < least * 0.999) {
+      least = t;
+      best = np;
+    }
+  }
+  return best;
+}
+
 template <int N1, int N2>
 static cudaError_t x4(bool fwd, const GridSet& gs, int rows, const float2* tw, const float2* twn, cudaStream_t st) {
   using L = RowLayout<N1, N2>;
   constexpr int H = L::H;
+  constexpr bool kPairs = RowPairs<N1, N2>::ok;
   // twiddle tables staged in shared memory (schedule key x4_stage_fwd) or read from global memory
   const int stage = !fwd || tuned("x4_stage_fwd", H, 1) != 0;
   const size_t fixed = sizeof(float2) * 2 * (size_t)H * stage;
@@ -566,9 +823,17 @@ static cudaError_t x4(bool fwd, const GridSet& gs, int rows, const float2* tw, c
   RowShape rs{128, 128 / (N1 / 2 + 1)};
   if (!fwd || rs.lines < 1 || 2 * rs.lines * N2 < rs.T)
     rs = row_shape(N2, N1, fwd ? N1 / 2 + 1 : N1, fwd ? 2 * N2 : N2, fixed, per, fwd ? 1 : 2);
-  const int T = std::max(64, std::min(256, tuned(fwd ? "x4_threads_fwd" : "x4_threads_inv", H, rs.T) / 32 * 32));
-  const int rpc = std::max(1, std::min(64, tuned(fwd ? "x4_rpc_fwd" : "x4_rpc_inv", H, rs.lines)));
-  const size_t smem = fixed + per * rpc + sizeof(float2);
+  int rpc = std::max(1, std::min(64, tuned(fwd ? "x4_rpc_fwd" : "x4_rpc_inv", H, rs.lines)));
+  int T = std::max(64, std::min(256, tuned(fwd ? "x4_threads_fwd" : "x4_threads_inv", H, rs.T) / 32 * 32));
+  size_t smem = fixed + per * rpc + sizeof(float2);
+  if constexpr (kPairs) {
+    if (!fwd) {
+      const int np = std::max(1, std::min(256 / N1, tuned("x4_rpc_inv", H, 2 * pair_count<N1, N2>()) / 2));
+      rpc = 2 * np;
+      T = std::max(64, std::max((np * N1 + 31) / 32 * 32, std::min(256, tuned("x4_threads_inv", H, 64) / 32 * 32)));
+      smem = fixed + sizeof(float2) * RowPairs<N1, N2>::words(np);
+    }
+  }
   const void* fn = fwd ? (const void*)k_xr2c4<N1, N2> : (const void*)k_xc2r4<N1, N2>;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;

@@ -456,7 +456,8 @@ static cudaError_t launch_x(bool fwd, const GridSet& gs, int nxp, int rows, cons
                             const float2* twn, cudaStream_t st, int* nlaunch) {
   const bool even = (nxp & 1) == 0;
   const int n = even ? nxp / 2 : nxp;
-  if (four_step_supported(n)) return launch_x4(fwd, gs, nxp, rows, tw, twn, st, nlaunch);
+  // odd forward rows of a plain set keep the full-length transform of each row
+  if (four_step_supported(n) && (even || !fwd || !gs.plain)) return launch_x4(fwd, gs, nxp, rows, tw, twn, st, nlaunch);
   if (even && pipe_enabled()) {
     // rows per unit and threads: about 8 points per thread (schedule keys x_ppt, x_rpc)
     const int ppt = std::max(1, tuned("x_ppt", n, 8));

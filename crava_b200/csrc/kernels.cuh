@@ -26,6 +26,7 @@ struct GridSet {
   const float* src[kMaxGrids];
   float scale[kMaxGrids];
   int n;
+  int plain = 0;   // 1: forward transforms in the scalar kernels' order of roundings (zpass.cuh says why)
 };
 
 // Per-kz operator tables of one block (device pointers), see the host-side builder.
@@ -57,6 +58,8 @@ struct ZParams {
   int D, PS, swz;              // tile layout (pencil.cuh): slot of the diagonal, bytes per position,
                                // positions swapped within fours in the per-bin steps
   int vec;                     // 1: pairs of bins move as 16-byte words
+  int logW, GT;                // k_zpass: log2 W, slots per z-transform call (3 SB <= GT)
+  LinePlan zp;                 // k_zpass: the z transform's stages
   ZPlan z;
   int nth, nsim;
   int separable;               // 1: prior from cxy/ct factors, 0: from spectral grids
@@ -257,6 +260,10 @@ cudaError_t launch_line_fft(const GridSet& gs, int ni, int n, size_t pstride, in
 bool pencil_shape(ZParams& zp, int* threads);
 cudaError_t launch_pencil(const ZParams& zp, int threads, cudaStream_t st, int* nlaunch);
 size_t pencil_smem_bytes(int W, int nzp, int nth, int SB);
+// zpass.cu: the same with the scalar z transforms, for residual spectra; zpass_shape as pencil_shape
+bool zpass_shape(ZParams& zp, int* threads);
+cudaError_t launch_zpass(const ZParams& zp, int threads, cudaStream_t st, int* nlaunch);
+size_t zpass_smem_bytes(int W, int nzp, int nth, int GT, int SB);
 // Float layout of one position's row of the eigen tables: kw (2n floats), Lam (n), then per
 // angle l a row of V (2n floats) and Q_l (6) + H_l (9); sections padded to 4 floats so the
 // kernel reads them as float4 groups and streams one angle's row at a time.

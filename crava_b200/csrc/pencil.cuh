@@ -280,21 +280,6 @@ __device__ __forceinline__ int pencil_kz_dev(const ZPlan& z, int p) {
 
 // ------------------------------------------------------------------ per-bin algebra, eigen form
 
-constexpr int pad4(int x) { return (x + 3) / 4 * 4; }
-
-// Section of N floats (N % 4 == 0) of the row of position p: group g at e[g * stride].
-template <int N>
-__device__ __forceinline__ void ldrow(float (&out)[N], const float4* __restrict__ e, int stride) {
-#pragma unroll
-  for (int g = 0; g < N / 4; g++) {
-    const float4 v = __ldg(e + g * stride);
-    out[4 * g] = v.x;
-    out[4 * g + 1] = v.y;
-    out[4 * g + 2] = v.z;
-    out[4 * g + 3] = v.w;
-  }
-}
-
 __device__ __forceinline__ float rcp_approx(float x) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -313,10 +298,12 @@ struct PairPost {
 __device__ __forceinline__ C2 a_mu(const ZParams& P, int l, const C2 (&m)[3]) {
   return c2_fma(P.A[l][2], m[2], c2_fma(P.A[l][1], m[1], c2_scale(m[0], P.A[l][0])));
 }
-// x - kw y
+// x - k y, the product rounded before the difference: residuals are differences of large numbers, and
+// zpass.cuh forms them in this order too
 __device__ __forceinline__ C2 c2_submul(C2 x, float kr, float ki, C2 y) {
-  return {f2_fma(f2_dup(ki), y.i, f2_fma(f2_dup(-kr), y.r, x.r)),
-          f2_fma(f2_dup(-ki), y.r, f2_fma(f2_dup(-kr), y.i, x.i))};
+  const float2 r = f2_fma(f2_dup(kr), y.r, f2_mul(f2_dup(-ki), y.i));
+  const float2 i = f2_fma(f2_dup(kr), y.i, f2_mul(f2_dup(ki), y.r));
+  return {f2_sub(x.r, r), f2_sub(x.i, i)};
 }
 
 // mu_post and S_post of the two bins of one z position from that position's row e (float4 groups

@@ -153,4 +153,21 @@ __device__ __forceinline__ bool chol_ref(float2 (&a)[N][N]) {
   return true;
 }
 
+// ------------------------------------------------------------------ eigen tables
+
+constexpr int pad4(int x) { return (x + 3) / 4 * 4; }
+
+// Section of N floats (N % 4 == 0) of the row of position p: group g at e[g * stride].
+template <int N>
+__device__ __forceinline__ void ldrow(float (&out)[N], const float4* __restrict__ e, int stride) {
+#pragma unroll
+  for (int g = 0; g < N / 4; g++) {
+    const float4 v = __ldg(e + g * stride);
+    out[4 * g] = v.x;
+    out[4 * g + 1] = v.y;
+    out[4 * g + 2] = v.z;
+    out[4 * g + 3] = v.w;
+  }
+}
+
 }  // namespace crava
