@@ -523,18 +523,25 @@ class Job:
 
     def download_outputs(self) -> dict:
         blk = self.blk
-        out = {"mean": np.stack([self.download(ROLE_POST_MEAN, a) for a in range(3)])}
-        cov = np.stack([self.download(ROLE_POST_COV, q) for q in range(6)])
+
+        # one array per output, the grids downloaded into it: no copies, and numpy backs arrays of
+        # some megabytes with huge pages, which a fresh buffer per grid does not reach
+        def grids(role, n):
+            a = np.empty((n,) + self.shape, dtype=np.float32)
+            for q in range(n):
+                self.download(role, q, a[q])
+            return a
+
+        out = {"mean": grids(ROLE_POST_MEAN, 3)}
+        cov = grids(ROLE_POST_COV, 6)
         if self.flags & FLAG_SPECTRAL_COV:
             out["cov_spec"] = cov.view(np.complex64)
         else:
             out["cov"] = cov
         if self.nsim:
-            out["sims"] = np.stack([self.download(ROLE_SIM, q) for q in range(3 * self.nsim)]).reshape(
-                (self.nsim, 3) + self.shape)
+            out["sims"] = grids(ROLE_SIM, 3 * self.nsim).reshape((self.nsim, 3) + self.shape)
         if self.flags & FLAG_KEEP_RESIDUAL:
-            out["resid_spec"] = np.stack([self.download(ROLE_RESIDUAL, l).view(np.complex64)
-                                          for l in range(blk.ntheta)])
+            out["resid_spec"] = grids(ROLE_RESIDUAL, blk.ntheta).view(np.complex64)
         return out
 
     def close(self):
