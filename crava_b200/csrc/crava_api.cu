@@ -1007,7 +1007,7 @@ float inv_scale(size_t N, bool cov) {
 // batched launches.
 crava_status fwd_xy(crava_ctx* ctx, const std::vector<const float*>& src, const std::vector<float*>& g,
                     const std::vector<float>& sc, int nxp, int nyp, int nzp, bool with_z, cudaStream_t st,
-                    bool plain = false) {
+                    bool plain = false, unsigned long long* zero = nullptr) {
   if (g.empty()) return CRAVA_OK;
   Plan *px, *pn, *py, *pz;
   crava_status s;
@@ -1017,6 +1017,7 @@ crava_status fwd_xy(crava_ctx* ctx, const std::vector<const float*>& src, const 
   for (size_t b = 0; b < g.size(); b += kMaxGrids) {
     GridSet gs;
     gs.plain = plain;
+    gs.zero = b == 0 ? zero : nullptr;
     gs.n = (int)std::min(g.size() - b, (size_t)kMaxGrids);
     for (int q = 0; q < gs.n; q++) { gs.p[q] = g[b + q]; gs.src[q] = src[b + q]; gs.scale[q] = sc[b + q]; }
     {
@@ -2460,7 +2461,6 @@ crava_status crava_job_run(crava_job* job, void* stream) {
   const crava_job_desc& d = job->d;
   cudaStream_t st = (cudaStream_t)stream;
   CUDA_TRY(cudaSetDevice(ctx->device));
-  CUDA_TRY(cudaMemsetAsync(job->counters, 0, kNumCounters * sizeof(unsigned long long), st));
   const bool grids = d.prior_mode == CRAVA_PRIOR_GRIDS;
   const float fs = fwd_scale(job->N);
   crava_status s;
@@ -2471,8 +2471,10 @@ crava_status crava_job_run(crava_job* job, void* stream) {
     std::vector<float> sc;
     for (int l = 0; l < d.ntheta; l++) { src.push_back(job->in_data[l]); g.push_back(job->data[l]); sc.push_back(fs); }
     for (int a = 0; a < 3; a++) { src.push_back(job->in_mean[a]); g.push_back(job->mean[a]); sc.push_back(fs); }
-    // residual spectra keep the scalar transforms' roundings (zpass.cuh)
-    if ((s = fwd_xy(ctx, src, g, sc, d.nxp, d.nyp, d.nzp, false, st, (d.flags & CRAVA_FLAG_KEEP_RESIDUAL) != 0))) return s;
+    // residual spectra keep the scalar transforms' roundings (zpass.cuh); the first kernel clears the counters
+    if ((s = fwd_xy(ctx, src, g, sc, d.nxp, d.nyp, d.nzp, false, st, (d.flags & CRAVA_FLAG_KEEP_RESIDUAL) != 0,
+                    job->counters)))
+      return s;
   }
   if (grids) {
     std::vector<const float*> src;

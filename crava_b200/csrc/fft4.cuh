@@ -74,6 +74,8 @@ __global__ void __launch_bounds__(256, col_split(N).r0 <= 10 ? 4 : col_split(N).
   const int i0 = it * W, nw = min(W, ni - i0);
   float2* g = reinterpret_cast<float2*>(gs.p[blockIdx.y]) + (size_t)o * ostride + i0;
   const uint32_t ps = 16u << lnp;
+  dep_wait();
+  dep_launch();
   for (int t = tid; t < N; t += T) tw[t] = twg[t];
   bool first = true;
 #pragma unroll 1
@@ -192,6 +194,8 @@ __global__ void __launch_bounds__(DIR > 0 ? 512 : 256) k_line4s(const __grid_con
   constexpr int N = N1 * N2;
   extern __shared__ float2 sm[];
   float2* tw = sm;
+  dep_wait();
+  dep_launch();
   for (int t = threadIdx.x; t < N; t += blockDim.x) tw[t] = twg[t];
   const int it = blockIdx.x % nIT, o = blockIdx.x / nIT;
   const int i0 = it * W, nw = min(W, ni - i0);
@@ -487,6 +491,11 @@ __device__ __forceinline__ void rows_out(float2* dst, const float2* src, int n, 
 // thread does and pass 2 stores runs of N1 points; staged both ways they measured slower (540x540x256:
 // 1.24 against 1.18 ms; staged stores alone the same), the rows' second buffer costing resident CTAs.
 //
+// the counters a job clears with its first transform
+__device__ __forceinline__ void x_clear(const GridSet& gs) {
+  if (gs.zero && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < kNumCounters) gs.zero[threadIdx.x] = 0;
+}
+
 // stage != 0: the twiddle tables are copied into shared memory first; 0: the passes read
 // them from global memory (L1-resident: every CTA of the launch reads the same 2 h values),
 // and the CTA's first barrier and the table copy go away.
@@ -498,6 +507,9 @@ __global__ void __launch_bounds__(256) k_xr2c4(const __grid_constant__ GridSet g
   extern __shared__ float2 sm[];
   const float2 *tw = twg, *twh = twn;
   float2* Z = sm;
+  dep_wait();
+  dep_launch();
+  x_clear(gs);
   if (pf > 0) x4_prefetch<true>(gs, rows, rpc, H + 1, pf);
   if (stage) {
     float2* t1 = sm;
@@ -528,6 +540,8 @@ __global__ void __launch_bounds__(256) k_xc2r4(const __grid_constant__ GridSet g
   float2* Xs = sm + 2 * H;
   const int row0 = blockIdx.x * rpc, nr = min(rpc, rows - row0);
   float2* g = reinterpret_cast<float2*>(gs.p[blockIdx.y]) + (size_t)row0 * CN;
+  dep_wait();
+  dep_launch();
   rows_in(Xs, g, nr * CN, al16);
   if (pf > 0) x4_prefetch<false>(gs, rows, rpc, CN, pf);
   for (int t = threadIdx.x; t < H; t += blockDim.x) {
@@ -563,6 +577,9 @@ __global__ void __launch_bounds__(256) k_xr2c4o(const __grid_constant__ GridSet 
   const int T = blockDim.x, tid = threadIdx.x;
   const int row0 = blockIdx.x * 2 * lpc, nr = min(2 * lpc, rows - row0), nl = (nr + 1) / 2;
   const size_t o = (size_t)row0 * CN;
+  dep_wait();
+  dep_launch();
+  x_clear(gs);
   rows_in(Xs, reinterpret_cast<const float2*>(gs.src[blockIdx.y]) + o, nr * CN, al16);
   for (int t = tid; t < N; t += T) tw[t] = twg[t];
   cp_async_wait_0();
@@ -619,6 +636,8 @@ __global__ void __launch_bounds__(256) k_xc2r4o(const __grid_constant__ GridSet 
   const int T = blockDim.x, tid = threadIdx.x;
   const int row0 = blockIdx.x * 2 * lpc, nr = min(2 * lpc, rows - row0), nl = (nr + 1) / 2;
   float2* g = reinterpret_cast<float2*>(gs.p[blockIdx.y]) + (size_t)row0 * CN;
+  dep_wait();
+  dep_launch();
   rows_in(Xs, g, nr * CN, al16);
   for (int t = tid; t < N; t += T) tw[t] = twg[t];
   cp_async_wait_0();
@@ -712,9 +731,9 @@ static cudaError_t line4_scalar(const GridSet& gs, int ni, size_t pstride, int n
     if ((e = resident_grid(fn, T, smem, 1 << 30, &res)) != cudaSuccess) return e;
     pf = std::max(1, res * q / 4);
   }
-  if (sign < 0.f) k_line4s<N1, N2, -1><<<grid, T, smem, st>>>(gs, ni, pstride, ostride, W, lw, nIT, SK, tw, pf);
-  else k_line4s<N1, N2, 1><<<grid, T, smem, st>>>(gs, ni, pstride, ostride, W, lw, nIT, SK, tw, pf);
-  return cudaGetLastError();
+  const size_t bytes = sizeof(float2) * (size_t)gs.n * ni * N * no;
+  return sign < 0.f ? launch_dep(bytes, k_line4s<N1, N2, -1>, grid, T, smem, st, gs, ni, pstride, ostride, W, lw, nIT, SK, tw, pf)
+                    : launch_dep(bytes, k_line4s<N1, N2, 1>, grid, T, smem, st, gs, ni, pstride, ostride, W, lw, nIT, SK, tw, pf);
 }
 
 template <int N>
@@ -737,9 +756,9 @@ static cudaError_t line4_pairs(const GridSet& gs, int ni, size_t pstride, int no
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   dim3 grid((unsigned)(nIT * no), gs.n);
-  if (sign < 0.f) k_line4<N, -1><<<grid, T, smem, st>>>(gs, ni, pstride, ostride, lnp, nIT, tw);
-  else k_line4<N, 1><<<grid, T, smem, st>>>(gs, ni, pstride, ostride, lnp, nIT, tw);
-  return cudaGetLastError();
+  const size_t bytes = sizeof(float2) * (size_t)gs.n * ni * N * no;
+  return sign < 0.f ? launch_dep(bytes, k_line4<N, -1>, grid, T, smem, st, gs, ni, pstride, ostride, lnp, nIT, tw)
+                    : launch_dep(bytes, k_line4<N, 1>, grid, T, smem, st, gs, ni, pstride, ostride, lnp, nIT, tw);
 }
 
 // Pairs up to 270 points: with 250 x-points, 21 grids of 60 planes, 5 % faster or equal at lengths of two
@@ -848,9 +867,9 @@ static cudaError_t x4(bool fwd, const GridSet& gs, int rows, const float2* tw, c
   }
   // every chunk starts at an even row, or two rows' bytes do not matter ((h + 1) even)
   const int al16 = grids_al16(gs) && (rpc % 2 == 0 || (H + 1) % 2 == 0);
-  if (fwd) k_xr2c4<N1, N2><<<grid, T, smem, st>>>(gs, rows, rpc, tw, twn, stage, pf);
-  else k_xc2r4<N1, N2><<<grid, T, smem, st>>>(gs, rows, rpc, tw, twn, al16, pf);
-  return cudaGetLastError();
+  const size_t bytes = sizeof(float2) * (size_t)gs.n * rows * (H + 1);
+  return fwd ? launch_dep(bytes, k_xr2c4<N1, N2>, grid, T, smem, st, gs, rows, rpc, tw, twn, stage, pf)
+             : launch_dep(bytes, k_xc2r4<N1, N2>, grid, T, smem, st, gs, rows, rpc, tw, twn, al16, pf);
 }
 
 // odd nxp = N1 N2: rows taken in pairs
@@ -866,9 +885,9 @@ static cudaError_t x4_odd(bool fwd, const GridSet& gs, int rows, const float2* t
   if (e != cudaSuccess) return e;
   dim3 grid((unsigned)((rows + 2 * rs.lines - 1) / (2 * rs.lines)), gs.n);
   const int al16 = grids_al16(gs);
-  if (fwd) k_xr2c4o<N1, N2><<<grid, rs.T, smem, st>>>(gs, rows, rs.lines, tw, al16);
-  else k_xc2r4o<N1, N2><<<grid, rs.T, smem, st>>>(gs, rows, rs.lines, tw, al16);
-  return cudaGetLastError();
+  const size_t bytes = sizeof(float) * (size_t)gs.n * rows * (N + 1);
+  return fwd ? launch_dep(bytes, k_xr2c4o<N1, N2>, grid, rs.T, smem, st, gs, rows, rs.lines, tw, al16)
+             : launch_dep(bytes, k_xc2r4o<N1, N2>, grid, rs.T, smem, st, gs, rows, rs.lines, tw, al16);
 }
 
 }  // namespace crava

@@ -49,6 +49,7 @@ __global__ void __launch_bounds__(512, 2) k_x_r2c(const __grid_constant__ GridSe
   const float scale = gs.scale[blockIdx.y];
   const int row0 = blockIdx.x * rpc;
   const int nr = min(rpc, rows - row0);
+  if (gs.zero && blockIdx.x == 0 && blockIdx.y == 0 && tid < kNumCounters) gs.zero[tid] = 0;
   for (int t = tid; t < n; t += T) tw[t] = twg[t];
   if (even)
     for (int t = tid; t < nxp / 2; t += T) twh[t] = twn[t];
@@ -240,6 +241,7 @@ __global__ void __launch_bounds__(512, 2) k_x_r2c_pipe(const __grid_constant__ G
   float2* const tile0 = twh + h;
   float2* const tile1 = tile0 + rpc * h;
   float2* scr = tile1 + rpc * h;
+  if (gs.zero && blockIdx.x == 0 && tid < kNumCounters) gs.zero[tid] = 0;
   for (int t = tid; t < h; t += T) {
     tw[t] = twg[t];
     twh[t] = twn[t];

@@ -9,6 +9,32 @@
 
 namespace crava {
 
+// Launches whose kernels follow one another in a stream overlap the next one's launch with the last one's
+// end (programmatic dependent launch) where the grids they work on hold less than kDepBytes: there the
+// launch gaps are a good part of the pass (32x30x40: 33 -> 23 us, 64x64x128 with 26 MB: 76 -> 66).
+// Larger ones run slower that way (105x135x125 with 16 realisations, 400 MB: 0.91 -> 1.00 ms), the
+// waiting CTAs taking room from the last wave.  dep_wait, before a kernel touches memory that another
+// may have written or still reads, waits until the grids before it are over; dep_launch lets the next
+// grid's CTAs take their places.
+constexpr size_t kDepBytes = 64u << 20;
+template <class... P, class... A>
+inline cudaError_t launch_dep(size_t bytes, void (*fn)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st,
+                              const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = bytes < kDepBytes ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, fn, args...);
+}
+__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Schedule table: tile shapes and kernel choices by name and size (n), from the schedule
 // file the library loads at first use (schedules.txt beside the library, written by
 // crava_b200/autotune.py; CRAVA_SCHEDULES names another file) or set through
@@ -21,11 +47,13 @@ constexpr int kMaxSim = 16;     // realisations per job launch
 
 // Grids of one batched transform launch.  p[] are the grids transformed in place;
 // for the forward x pass src[] are the real inputs it reads (src[q] == p[q] is in place).
+constexpr int kNumCounters = 5;
 struct GridSet {
   float* p[kMaxGrids];
   const float* src[kMaxGrids];
   float scale[kMaxGrids];
   int n;
+  unsigned long long* zero = nullptr;   // forward x pass: kNumCounters words it clears
   int plain = 0;   // 1: forward transforms in the scalar kernels' order of roundings (zpass.cuh says why)
 };
 
@@ -99,7 +127,6 @@ struct ZParams {
                                    // [3] bins re-factorised in FP64 [4] pencil tiles whose
                                    // input spectra are not finite
 };
-constexpr int kNumCounters = 5;
 
 // Local-noise shrinkage (localnoise.cu): per-trace maps of the posterior and realisations
 // from the local noise scales; the matrices are job constants computed on the host.

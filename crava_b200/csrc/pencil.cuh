@@ -500,6 +500,8 @@ __global__ void __launch_bounds__(512, 1) k_pencil(const __grid_constant__ ZPara
   const size_t kstride = (size_t)P.nyp * P.cnxp;
   const size_t base = (size_t)j * P.cnxp + i0;
 
+  dep_wait();
+  dep_launch();
   // ---- inputs, natural kz order; x-bins beyond the grid are zero-filled
   for (int e = tid; e < NZ << lnp; e += T) {
     const int q = e & (NP - 1), w = 2 * q, k = e >> lnp;
@@ -885,8 +887,8 @@ inline cudaError_t launch_pencil_t(const ZParams& zp, int threads, cudaStream_t 
   auto fn = k_pencil<NTH, MODE, R0, R1>;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  fn<<<dim3((unsigned)(zp.nIT * zp.nyp)), threads, smem, st>>>(zp);
-  return cudaGetLastError();
+  const size_t bytes = sizeof(float2) * (size_t)(12 + zp.nth + 3 * zp.nsim) * zp.cnxp * zp.nyp * zp.nzp;
+  return launch_dep(bytes, fn, dim3((unsigned)(zp.nIT * zp.nyp)), threads, smem, st, zp);
 }
 template <int NTH>
 inline cudaError_t launch_pencil_m(const ZParams& zp, int threads, cudaStream_t st) {
