@@ -162,7 +162,7 @@ struct ProfRec {
 
 namespace {
 // Per-block device tables: the per-kz operator tables of the prior and wavelet model (with
-// the separable factors and the eigen tables of pencil.cu) and the lateral correlation
+// the separable factors and the eigen tables of pencil.cuh) and the lateral correlation
 // spectrum.  They sit in the job's pool, or in an entry of the context's resident cache
 // shared by every job with the same model (crava_ctx_set_table_cache).
 struct KzSet {
@@ -301,10 +301,10 @@ struct crava_job {
   uint8_t* inv = nullptr;
   float2* cxy = nullptr;     // SEPARABLE
   float2* ct = nullptr;
-  float4* eig = nullptr;     // SEPARABLE: eigen tables of the in-place pencil kernel (pencil.cu)
-  bool eig_ok = false;       //   built and applicable: crava_job_run launches k_pencil
+  float4* eig = nullptr;     // SEPARABLE: eigen tables of the pencil pass (pencil.cuh)
+  bool eig_ok = false;       //   built and applicable: the pass takes the eigen form
   int n_inv_rows = 0;        //   inverted kz
-  std::string eig_why;       //   why the general kernel runs instead
+  std::string eig_why;       //   why it takes the Cholesky form instead
   float* cxy_grid = nullptr; // staging for the corr_xy transform
   float* fill_xy = nullptr;  // GRIDS: corrXY and circCorrT for crava_job_fill_prior
   float* fill_t = nullptr;
@@ -1956,7 +1956,7 @@ crava_status kz_set_build(const crava_job_desc& d, const std::vector<double>& A,
   std::vector<float2> ct(d.nzp);
   for (int kz = 0; kz < d.nzp; kz++) ct[kz] = make_float2((float)C[kz].real(), sym ? 0.f : (float)C[kz].imag());
   CUDA_TRY(up(k.ct, ct.data(), sizeof(float2) * d.nzp));
-  // the eigen form of the per-bin posterior (pencil.cu) where it applies
+  // the eigen form of the per-bin posterior (pencil.cuh) where it applies
   if (!k.eig) k.eig_why = "no separable prior";
   else if (!sym) k.eig_why = "circular temporal correlation not symmetric";
   else if (d.fp64_threshold > 0.f) k.eig_why = "FP64 re-factorisation requested";
@@ -2404,7 +2404,7 @@ namespace {
 // probabilities of crava_job_set_facies: the x transform and the evaluation in one pass
 // (launch_x4_facies) where the x length has a four-step split and the schedule key
 // facies_fused (n = nxp/2) is 1, else the x transform and then the facies pass.  The default
-// is the two passes: at 540x540x256 the one-pass form took 5.4 ms against 0.5 + 2.3 ms, its
+// is the two passes: at 540x540x256 the one-pass form took 5.4 ms against 0.5 + 2.3 ms (2.3 since halved), its
 // density gathers (L2-latency bound) running at the transform kernel's occupancy (8 warps
 // per SM against about 40 in the facies pass).
 crava_status inv_mean_facies(crava_ctx* ctx, crava_job* job, float ps, cudaStream_t st) {
