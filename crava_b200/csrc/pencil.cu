@@ -67,8 +67,14 @@ size_t pencil_smem_bytes(int W, int nzp, int nth, int SB) {
   return 8 * (size_t)even_up_z(nzp) + 96 + 2 * (size_t)((nzp + 7) & ~7) + (size_t)tile_ps(W, nth, SB) * nzp;
 }
 
-// CTAs that share an SM at T threads (128 registers each) and `smem` bytes.
-static int resident(size_t smem, int T) { return std::min((int)(227 * 1024 / (smem + 1024)), 512 / T); }
+// CTAs whose tiles of `smem` bytes share an SM: 228 KB, of which each takes 1 KB and its static shared
+// memory (64 bytes at most) besides, in units of 128 bytes.  A tile at the cap of 227 KB is one.
+constexpr size_t kStaticSmem = 64;
+static int tiles_per_sm(size_t smem) {
+  return std::max(1, (int)(228 * 1024 / ((smem + kStaticSmem + 127) / 128 * 128 + 1024)));
+}
+// ... and at T threads (128 registers each).
+static int resident(size_t smem, int T) { return std::max(1, std::min(tiles_per_sm(smem), 512 / T)); }
 
 // The tile.  Two or more CTAs of 128..256 threads on an SM overlap one's copies and barriers with the
 // other's arithmetic (270x270x256, 5 angles, 4 realisations: W 8, 512 threads 1.30 ms; W 4, two of
@@ -77,7 +83,7 @@ static int resident(size_t smem, int T) { return std::min((int)(227 * 1024 / (sm
 // threads busy).  Relative costs as measured at 64 to 320 points, 1 to 16 realisations; a shape
 // whose tiles fill the last wave badly pays for it (64x64x128: W 8 39 us, W 4 31).
 bool pencil_shape(ZParams& zp, int* threads) {
-  const size_t cap = 227 * 1024 - 64;   // the kernel's static shared memory comes on top
+  const size_t cap = 227 * 1024 - kStaticSmem;
   const int key = zp.nzp * 16 + zp.nth, least = zp.nsim ? 1 : 0, most = std::min(zp.nsim, 4);
   if (!pencil_plan(zp.nzp, zp.z)) return false;
   const int tw = tuned("pencil_w", key, 0), ts = tuned("pencil_sb", key, -1), tt = tuned("pencil_threads", key, 0);
@@ -91,7 +97,7 @@ bool pencil_shape(ZParams& zp, int* threads) {
       if (ts >= 0 && b > std::max(least, std::min(most, ts))) continue;
       const size_t smem = pencil_smem_bytes(w, zp.nzp, zp.nth, b);
       if (smem > cap) continue;
-      const int fit = std::min(4, (int)(227 * 1024 / (smem + 1024)));
+      const int fit = std::min(4, tiles_per_sm(smem));
       int t = fit >= 2 ? 512 / fit / 32 * 32 : 512;
       t = std::max(64, std::min(t, (zp.nzp * w / 2 + 31) / 32 * 32));   // a pair of bins each
       const int ctas = resident(smem, t);
