@@ -288,12 +288,6 @@ __device__ __forceinline__ int pencil_kz_dev(const ZPlan& z, int p) {
 
 // ------------------------------------------------------------------ per-bin algebra, eigen form
 
-__device__ __forceinline__ float rcp_approx(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-
 // A pair of bins between the posterior and the realisations: mu_post, and S_post as its real
 // diagonal 00 11 22 and its entries 01 02 12.
 struct PairPost {
@@ -353,10 +347,7 @@ __device__ __forceinline__ void pair_posterior_eig(const ZParams& P, const float
            f2_fma(f2_dup(vi), d[m].r, f2_fma(f2_dup(vr), d[m].i, r.i))};
     }
     const float2 den = f2_fma(lam, f2_dup(Lm[l]), make_float2(1.f, 1.f));
-    // 1 / den (den >= 1): the hardware reciprocal and one Newton step
-    const float2 x0 = make_float2(rcp_approx(den.x), rcp_approx(den.y));
-    const float2 x1 = f2_fma(x0, f2_fma(f2_neg(den), x0, make_float2(1.f, 1.f)), x0);
-    const float2 f = f2_mul(lam, x1);
+    const float2 f = f2_mul(lam, make_float2(__frcp_rn(den.x), __frcp_rn(den.y)));
     const C2 sl = {f2_mul(r.r, f), f2_mul(r.i, f)};
     const float2 nw = f2_neg(f2_mul(lam, f));
     // mu_post += conj(Q_l.) s_l;  S_post -= w_l H_l, H_l = (|Q_l0|^2, |Q_l1|^2, |Q_l2|^2,

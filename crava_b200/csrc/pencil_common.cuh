@@ -10,12 +10,6 @@
 
 namespace crava {
 
-__device__ __forceinline__ float rsqrt_approx(float x) {
-  float r;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-
 // ------------------------------------------------------------------ noise (product mode)
 
 // Philox-4x32 (Salmon, Moraes, Dror, Shaw, SC'11) with 7 rounds, which the authors
@@ -43,9 +37,9 @@ __device__ __forceinline__ uint4 philox4x32_7(uint4 c, uint2 k) {
 // (the largest |normal| is sqrt(2 ln 2^27) = 6.1) and the angle 2 pi ((b + 1/2) / 2^16 - 1/2), with the
 // hardware approximations of log, sine and cosine: their absolute errors (about 2^-21 on
 // these ranges) are far below what the normals' statistics can show.  The two bins' arithmetic is
-// packed; b / 2^16 comes from the mantissa bits of [1, 2) without a conversion, and the square
-// root from the reciprocal one with a Newton step (no branch for special values: its
-// argument is kept positive).
+// packed, with the operations and roundings of device_noise3 (zpass.cuh), so that a bin's draw does not
+// depend on the kernel that makes it; b / 2^16 comes from the mantissa bits of [1, 2) without a
+// conversion.
 __device__ __forceinline__ void pair_noise(const ZParams& P, int s, int i, int j, int k, C2 (&z)[3]) {
   const int last = P.cnxp - 1;
   uint64_t bin[2];
@@ -66,6 +60,8 @@ __device__ __forceinline__ void pair_noise(const ZParams& P, int s, int i, int j
       }
     }
   }
+  constexpr float kH = 0.70710678118654752f;
+  const float2 h = make_float2(self[0] ? 1.0f : kH, self[1] ? 1.0f : kH);
   const uint2 key = make_uint2((uint32_t)P.seed, (uint32_t)(P.seed >> 32));
   uint4 r[2];
 #pragma unroll
@@ -84,34 +80,22 @@ __device__ __forceinline__ void pair_noise(const ZParams& P, int s, int i, int j
     const uint32_t a1 = (c == 0 ? r[1].x : c == 1 ? r[1].y : r[1].z) >> 6;
     const float2 u1 = f2_mul(f2_add(make_float2((float)a0, (float)a1), f2_dup(0.5f)), f2_dup(1.4901161193847656e-08f));
     const float2 t = f2_mul(make_float2(__logf(u1.x), __logf(u1.y)), f2_dup(-2.0f));
-    const float2 x = make_float2(fmaxf(t.x, 1e-30f), fmaxf(t.y, 1e-30f));
-    const float2 q = make_float2(rsqrt_approx(x.x), rsqrt_approx(x.y));
-    float2 rad = f2_mul(x, q);
-    rad = f2_fma(f2_mul(q, f2_dup(0.5f)), f2_fma(f2_neg(rad), rad, x), rad);
-    rad = f2_mul(rad, f2_dup(0.70710678118654752f));
+    const float2 rad = make_float2(sqrtf(t.x), sqrtf(t.y));
     // (1 + b / 2^16) - (3/2 - 2^-17), exact
     const float2 u2 = f2_add(make_float2(__uint_as_float(b[c][0]), __uint_as_float(b[c][1])), f2_dup(-1.49999237060546875f));
     const float2 ang = f2_mul(u2, f2_dup(6.283185307179586f));   // in (-pi, pi)
     float2 sn, cs;
     __sincosf(ang.x, &sn.x, &cs.x);
     __sincosf(ang.y, &sn.y, &cs.y);
-    z[c] = {f2_mul(rad, cs), f2_mul(rad, sn)};
+    z[c] = {f2_mul(f2_mul(rad, cs), h), f2_mul(f2_mul(rad, sn), h)};
   }
   if (edge) {
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-      if (self[0]) {
-        z[c].r.x *= 1.41421356237309505f;
-        z[c].i.x = 0.f;
-      } else if (conj[0]) {
-        z[c].i.x = -z[c].i.x;
-      }
-      if (self[1]) {
-        z[c].r.y *= 1.41421356237309505f;
-        z[c].i.y = 0.f;
-      } else if (conj[1]) {
-        z[c].i.y = -z[c].i.y;
-      }
+      if (self[0]) z[c].i.x = 0.f;
+      else if (conj[0]) z[c].i.x = -z[c].i.x;
+      if (self[1]) z[c].i.y = 0.f;
+      else if (conj[1]) z[c].i.y = -z[c].i.y;
     }
   }
 }
