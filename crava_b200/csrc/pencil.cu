@@ -85,6 +85,7 @@ static int resident(size_t smem, int T) { return std::max(1, std::min(tiles_per_
 bool pencil_shape(ZParams& zp, int* threads) {
   const size_t cap = 227 * 1024 - kStaticSmem;
   const int key = zp.nzp * 16 + zp.nth, least = zp.nsim ? 1 : 0, most = std::min(zp.nsim, 4);
+  const int per = zp.eig ? 2 : 1;       // bins per thread of the per-bin step
   if (!pencil_plan(zp.nzp, zp.z)) return false;
   const int tw = tuned("pencil_w", key, 0), ts = tuned("pencil_sb", key, -1), tt = tuned("pencil_threads", key, 0);
   int W = 0, SB = 0, T = 0;
@@ -99,7 +100,7 @@ bool pencil_shape(ZParams& zp, int* threads) {
       if (smem > cap) continue;
       const int fit = std::min(4, tiles_per_sm(smem));
       int t = fit >= 2 ? 512 / fit / 32 * 32 : 512;
-      t = std::max(64, std::min(t, (zp.nzp * w / 2 + 31) / 32 * 32));   // a pair of bins each
+      t = std::max(64, std::min(t, (zp.nzp * w / per + 31) / 32 * 32));
       const int ctas = resident(smem, t);
       const long long tiles = (long long)((zp.cnxp + w - 1) / w) * zp.nyp, slots = 148LL * ctas;
       const double fill = (double)tiles / ((tiles + slots - 1) / slots * slots);
@@ -135,6 +136,24 @@ bool pencil_shape(ZParams& zp, int* threads) {
   zp.PS = tile_ps(W, zp.nth, SB);
   zp.swz = zp.NP == 4 && zp.nzp % 4 == 0;
   const int items = zp.nzp * zp.NP;
+  // The Cholesky forms on a block whose tiles are all resident at once: a tile's time is its rounds of
+  // bins, each as long as a factorisation, so the threads of an SM go to the r tiles that it gets where that
+  // saves a round (48x50x72, 6 angles, 350 tiles of 288 bins: 160 threads instead of 128, the pass 37 -> 33 us, with
+  // FP64 96 -> 70).  Tiles that are not all resident keep their neighbours' company: 400 tiles of 512 threads
+  // instead of 128 took 76 us instead of 62.
+  const long long tiles = (long long)zp.nIT * zp.nyp;
+  const int fit = std::min(4, tiles_per_sm(pencil_smem_bytes(W, zp.nzp, zp.nth, SB)));
+  if (!zp.eig && tiles <= 148LL * fit) {
+    int least = 1 << 30;
+    for (int r = fit; r >= (int)((tiles + 147) / 148); r--) {
+      const int t = std::max(64, std::min(512 / r / 32 * 32, (zp.nzp * W + 31) / 32 * 32));
+      const int rounds = (zp.nzp * W + t - 1) / t;
+      if (rounds < least) {
+        least = rounds;
+        T = t;
+      }
+    }
+  }
   if (tt > 0) T = std::max(64, std::min(512, tt / 32 * 32));
   // two bits per item of a thread hold the failed factorisations: at most 16 items each
   T = std::max(T, std::min(512, (items / 16 + 31) / 32 * 32));

@@ -441,7 +441,7 @@ __device__ __forceinline__ void pair_llh(float2 (&sd)[3], C2 (&so)[3], int fail)
 // ------------------------------------------------------------------ the kernel
 //
 // Shared memory: tw [nzp] (float2), the grid pointers of one batch of output lines (12), perm
-// [nzp] (uint16: kz of a position), then the tile, PS bytes per position.  With NP = W / 2 pairs:
+// [nzp] (uint16: kz of a position; position of a kz in the Cholesky forms), then the tile, PS bytes per position.  With NP = W / 2 pairs:
 //   slot s, pair q         16-byte word s NP + q
 //   inputs                 data 0 .. nth-1, mean nth .. nth+2
 //   after the per-bin step SB realisations' spectra 0 .. 3 SB - 1, mu_post 3 SB .. 3 SB + 2,
@@ -471,6 +471,14 @@ __device__ __forceinline__ void diag_put(uint32_t pos, const ZParams& P, int q, 
     sts1(x + 4u, 0.f);
     sts1(x + 12u, 0.f);
   }
+}
+// ... of the pair's bin u alone
+__device__ __forceinline__ void diag_put1(uint32_t pos, const ZParams& P, int q, int u, float d0, float d1, float d2) {
+  const uint32_t w = pos + 16u * (uint32_t)(P.D * P.NP);
+  sts2(w + 16u * (uint32_t)q + 8u * (uint32_t)u, make_float2(d0, d1));
+  const uint32_t x = w + 16u * (uint32_t)(P.NP + (q >> 1)) + 4u * (uint32_t)(q & 1) + 8u * (uint32_t)u;
+  sts1(x, d2);
+  if (P.NP == 1) sts1(x + 4u, 0.f);
 }
 __device__ __forceinline__ void diag_get(uint32_t pos, const ZParams& P, int q, float2 (&d)[3]) {
   const uint32_t w = pos + 16u * (uint32_t)(P.D * P.NP);
@@ -525,7 +533,8 @@ __global__ void __launch_bounds__(512, 1) k_pencil(const __grid_constant__ ZPara
   if (tid < 4) cnt[tid] = 0;
   for (int t = tid; t < NZ; t += T) {
     sts2(s_tw + 8u * (uint32_t)t, __ldg(P.twz + t));
-    const_cast<uint16_t*>(perm)[t] = (uint16_t)pencil_kz_dev(P.z, t);
+    const int kz = pencil_kz_dev(P.z, t);
+    const_cast<uint16_t*>(perm)[MODE == kEig ? t : kz] = (uint16_t)(MODE == kEig ? kz : t);
   }
   cp_async_wait_0();
   __syncthreads();
@@ -538,7 +547,8 @@ __global__ void __launch_bounds__(512, 1) k_pencil(const __grid_constant__ ZPara
   zs.gap = 0;
   z_forward<R0, R1>(P.z, zs);
   // a NaN or Inf in any input grid reaches every bin through the transforms
-  if (tid == 0 && P.counters) {
+  // (read by the thread whose per-bin step takes that bin first)
+  if (tid == (MODE == kEig ? 0 : wlo) && P.counters) {
     float s = 0.f;
 #pragma unroll
     for (int g = 0; g < GIN; g++) {
@@ -554,25 +564,140 @@ __global__ void __launch_bounds__(512, 1) k_pencil(const __grid_constant__ ZPara
   const uint32_t s_post = 16u * (uint32_t)((3 * SB) << lnp);   // byte offset of mu_post in a position
   unsigned long long n_zero_bins = 0, n_inv = 0, n_fail = 0, n_fp64 = 0;
   unsigned int failed = 0;                                    // two bits per item of this thread
-  auto pos_of = [&](int b) {
-    const int p = b >> lnp;
-    return P.swz ? (p & ~3) | ((p & 1) << 1) | ((p >> 1) & 1) : p;
+  // Position and kz of the m-th round.  The eigen form takes the positions in order; the Cholesky forms the
+  // kz in order: the kz that are not inverted and the bins that FP64 does again come in runs, which whole
+  // warps then skip or take, where digit-reversed every warp holds a few (200x216x200, prior grids: 0.80 -> 0.74 ms,
+  // with FP64 0.82 -> 0.75; 60x50x128, FP64: 74 -> 62 us).
+  auto locate = [&](int m, int& p, int& kz) {
+    if constexpr (MODE == kEig) {
+      p = P.swz ? (m & ~3) | ((m & 1) << 1) | ((m >> 1) & 1) : m;
+      kz = perm[p];
+    } else {
+      kz = m;
+      p = perm[m];
+    }
   };
-  {
+  if constexpr (MODE != kEig) {
+    // The Cholesky forms: a bin, not a pair, per thread and round.  A factorisation is a serial chain, longer by
+    // several times where it is done again in FP64, and on a small block the chains of one tile are the time
+    // of the pass (28x27x45, 5 angles, FP64: 73 us with a pair's two chains in one thread, 52 so).  Lane u of a
+    // pair's words is its bin u: the two threads of a pair share words, but no float.
+#pragma unroll 1
+    for (int b = tid; b < 2 * items; b += T) {
+      const int u = b & 1, q = (b >> 1) & (NP - 1), w = 2 * q + u;
+      int p, kz;
+      locate(b >> (1 + lnp), p, kz);
+      const uint32_t pos = tile + (uint32_t)(p * PS), sl = pos + 16u * (uint32_t)q + 4u * (uint32_t)u;
+      const bool in = w >= wlo && w < nw;
+      const size_t gi = base + (size_t)kz * kstride + w;
+      float2 m1[3], d1[NTH];
+#pragma unroll
+      for (int l = 0; l < NTH; l++) {
+        const uint32_t x = sl + 16u * (uint32_t)(l << lnp);
+        d1[l] = make_float2(lds1(x), lds1(x + 8u));
+      }
+#pragma unroll
+      for (int a = 0; a < 3; a++) {
+        const uint32_t x = sl + 16u * (uint32_t)((NTH + a) << lnp);
+        m1[a] = make_float2(lds1(x), lds1(x + 8u));
+      }
+      float S[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, lam = 0.f, rho = 0.f;
+      if (in) {
+        if (P.separable) {
+          const float2 cx = __ldg(P.cxy + base + w), c_t = __ldg(P.ct + kz);
+          rho = fabsf(cx.x * c_t.x - cx.y * c_t.y);
+#pragma unroll
+          for (int c = 0; c < 6; c++) S[c] = P.pv[c] * rho;
+          lam = fabsf(cx.x);
+        } else {
+          // getNextParameterCovariance: |Re/pv| pv (no division when pv == 0); a base prior's
+          // pairs share |Re/pv| of the one spectrum transformed (pv[0] != 0)
+          if (P.base_prior) {
+            const float r0 = fabsf(P.cov[0][gi].x / P.pv[0]);
+#pragma unroll
+            for (int c = 0; c < 6; c++) S[c] = r0 * P.pv[c];
+          } else {
+#pragma unroll
+            for (int c = 0; c < 6; c++) {
+              float re = P.cov[c][gi].x;
+              const float pv = P.pv[c];
+              if (pv != 0.f) re = re / pv;
+              S[c] = fabsf(re) * pv;
+            }
+          }
+          lam = fabsf(P.errspec[gi].x);
+        }
+      }
+      BinOut bo;
+      bool ok = false;
+      if (in && P.kz.inv[kz] != 0) {
+        n_inv++;
+        ok = P.septab ? bin_posterior<NTH, true>(P, kz, S, lam, rho, m1, d1, bo)
+                      : bin_posterior<NTH, false>(P, kz, S, lam, rho, m1, d1, bo);
+        if constexpr (MODE == kCholFp64) {
+          if (ok) {
+            float ratio = 1.f;
+#pragma unroll
+            for (int a = 0; a < 3; a++)
+              if (S[a] > 0.f) ratio = fminf(ratio, bo.sp[a].x / S[a]);
+            if (bo.cond > P.fp64_threshold || ratio * P.fp64_threshold < 1.f) {
+              // the data are still in their slots: restart from them
+              float2 d64[NTH];
+#pragma unroll
+              for (int l = 0; l < NTH; l++) {
+                const uint32_t x = sl + 16u * (uint32_t)(l << lnp);
+                d64[l] = make_float2(lds1(x), lds1(x + 8u));
+              }
+              if (bin_posterior_fp64<NTH>(P, kz, S, lam, m1, d64, bo)) {
+                n_fp64++;
+#pragma unroll
+                for (int l = 0; l < NTH; l++) d1[l] = d64[l];
+              }
+            }
+          }
+        }
+        if (!ok) n_fail++;
+      }
+      if (!ok) {
+#pragma unroll
+        for (int a = 0; a < 3; a++) bo.mu[a] = m1[a];
+#pragma unroll
+        for (int c = 0; c < 6; c++) bo.sp[c] = make_float2(S[c], 0.f);
+      }
+      if (P.keep_resid && in) {
+#pragma unroll
+        for (int l = 0; l < NTH; l++) P.data[l][gi] = d1[l];
+      }
+#pragma unroll
+      for (int a = 0; a < 3; a++) {
+        const uint32_t xm = sl + s_post + 16u * (uint32_t)(a << lnp), xs = sl + s_post + 16u * (uint32_t)((3 + a) << lnp);
+        sts1(xm, bo.mu[a].x);
+        sts1(xm + 8u, bo.mu[a].y);
+        sts1(xs, bo.sp[3 + a].x);
+        sts1(xs + 8u, bo.sp[3 + a].y);
+      }
+      diag_put1(pos, P, q, u, bo.sp[0].x, bo.sp[1].x, bo.sp[2].x);
+    }
+    __syncthreads();
+  }
+  // The eigen form, two bins a thread.  Then, in every form, S_post is factored once for all realisations; the
+  // covariance output is rebuilt as L L^H
+  if (MODE == kEig || P.nsim > 0) {
     int n = 0;
 #pragma unroll 1
     for (int b = tid; b < items; b += T, n++) {
-      const int q = b & (NP - 1), p = pos_of(b), kz = perm[p];
-      const uint32_t pos = tile + (uint32_t)(p * PS), sl = pos + 16u * (uint32_t)q;
+      const int q = b & (NP - 1);
+      int p, kz;
+      locate(b >> lnp, p, kz);
+      const uint32_t pos = tile + (uint32_t)(p * PS), sl = pos + 16u * (uint32_t)q, so = sl + s_post;
       const bool in0 = 2 * q >= wlo && 2 * q < nw, in1 = 2 * q + 1 < nw;
-      const size_t gidx = base + (size_t)kz * kstride + 2 * q;
-      C2 mu[3], d[NTH];
-#pragma unroll
-      for (int l = 0; l < NTH; l++) d[l] = lds_c2(sl + 16u * (uint32_t)(l << lnp));
-#pragma unroll
-      for (int a = 0; a < 3; a++) mu[a] = lds_c2(sl + 16u * (uint32_t)((NTH + a) << lnp));
       PairPost o;
       if constexpr (MODE == kEig) {
+        C2 mu[3], d[NTH];
+#pragma unroll
+        for (int l = 0; l < NTH; l++) d[l] = lds_c2(sl + 16u * (uint32_t)(l << lnp));
+#pragma unroll
+        for (int a = 0; a < 3; a++) mu[a] = lds_c2(sl + 16u * (uint32_t)((NTH + a) << lnp));
         float2 lam, rho;
         {
           const float ctk = __ldg(P.ct + kz).x;
@@ -582,119 +707,28 @@ __global__ void __launch_bounds__(512, 1) k_pencil(const __grid_constant__ ZPara
           rho = make_float2(fabsf(c0 * ctk), fabsf(c1 * ctk));
         }
         pair_posterior_eig<NTH>(P, P.eig + p, lam, rho, mu, d, o);
-      } else {
-        const bool inv = P.kz.inv[kz] != 0;
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-          float S[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, lam = 0.f, rho = 0.f;
-          const bool in = u ? in1 : in0;
-          if (in) {
-            if (P.separable) {
-              const float2 cx = __ldg(P.cxy + base + 2 * q + u), c_t = __ldg(P.ct + kz);
-              rho = fabsf(cx.x * c_t.x - cx.y * c_t.y);
-#pragma unroll
-              for (int c = 0; c < 6; c++) S[c] = P.pv[c] * rho;
-              lam = fabsf(cx.x);
-            } else {
-              // getNextParameterCovariance: |Re/pv| pv (no division when pv == 0); a base prior's
-              // pairs share |Re/pv| of the one spectrum transformed (pv[0] != 0)
-              const size_t gi = gidx + u;
-              if (P.base_prior) {
-                const float r0 = fabsf(P.cov[0][gi].x / P.pv[0]);
-#pragma unroll
-                for (int c = 0; c < 6; c++) S[c] = r0 * P.pv[c];
-              } else {
-#pragma unroll
-                for (int c = 0; c < 6; c++) {
-                  float re = P.cov[c][gi].x;
-                  const float pv = P.pv[c];
-                  if (pv != 0.f) re = re / pv;
-                  S[c] = fabsf(re) * pv;
-                }
-              }
-              lam = fabsf(P.errspec[gi].x);
-            }
-          }
-          float2 m1[3], d1[NTH];
-#pragma unroll
-          for (int a = 0; a < 3; a++) m1[a] = u ? make_float2(mu[a].r.y, mu[a].i.y) : make_float2(mu[a].r.x, mu[a].i.x);
-#pragma unroll
-          for (int l = 0; l < NTH; l++) d1[l] = u ? make_float2(d[l].r.y, d[l].i.y) : make_float2(d[l].r.x, d[l].i.x);
-          BinOut bo;
-          bool ok = false;
-          if (inv && in) {
-            n_inv++;
-            ok = P.septab ? bin_posterior<NTH, true>(P, kz, S, lam, rho, m1, d1, bo)
-                          : bin_posterior<NTH, false>(P, kz, S, lam, rho, m1, d1, bo);
-            if constexpr (MODE == kCholFp64) {
-              if (ok) {
-                float ratio = 1.f;
-#pragma unroll
-                for (int a = 0; a < 3; a++)
-                  if (S[a] > 0.f) ratio = fminf(ratio, bo.sp[a].x / S[a]);
-                if (bo.cond > P.fp64_threshold || ratio * P.fp64_threshold < 1.f) {
-                  float2 d64[NTH];
-#pragma unroll
-                  for (int l = 0; l < NTH; l++)
-                    d64[l] = u ? make_float2(d[l].r.y, d[l].i.y) : make_float2(d[l].r.x, d[l].i.x);
-                  if (bin_posterior_fp64<NTH>(P, kz, S, lam, m1, d64, bo)) {
-                    n_fp64++;
-#pragma unroll
-                    for (int l = 0; l < NTH; l++) d1[l] = d64[l];
-                  }
-                }
-              }
-            }
-            if (!ok) n_fail++;
-          }
-          if (!ok) {
-#pragma unroll
-            for (int a = 0; a < 3; a++) bo.mu[a] = m1[a];
-#pragma unroll
-            for (int c = 0; c < 6; c++) bo.sp[c] = make_float2(S[c], 0.f);
-          }
-#pragma unroll
-          for (int a = 0; a < 3; a++) {
-            if (u == 0) {
-              o.mu[a].r.x = bo.mu[a].x;
-              o.mu[a].i.x = bo.mu[a].y;
-              o.sd[a].x = bo.sp[a].x;
-              o.so[a].r.x = bo.sp[3 + a].x;
-              o.so[a].i.x = bo.sp[3 + a].y;
-            } else {
-              o.mu[a].r.y = bo.mu[a].x;
-              o.mu[a].i.y = bo.mu[a].y;
-              o.sd[a].y = bo.sp[a].x;
-              o.so[a].r.y = bo.sp[3 + a].x;
-              o.so[a].i.y = bo.sp[3 + a].y;
-            }
-          }
-          if (P.keep_resid && in) {
-#pragma unroll
-            for (int l = 0; l < NTH; l++) P.data[l][gidx + u] = d1[l];
-          }
-        }
-      }
-      if constexpr (MODE == kEig) {
         if (P.keep_resid) {
+          const size_t gidx = base + (size_t)kz * kstride + 2 * q;
 #pragma unroll
           for (int l = 0; l < NTH; l++) {
             if (in0) P.data[l][gidx] = make_float2(d[l].r.x, d[l].i.x);
             if (in1) P.data[l][gidx + 1] = make_float2(d[l].r.y, d[l].i.y);
           }
         }
+      } else {
+        diag_get(pos, P, q, o.sd);
+#pragma unroll
+        for (int a = 0; a < 3; a++) o.so[a] = lds_c2(so + 16u * (uint32_t)((3 + a) << lnp));
       }
-      // S_post is factored once for all realisations; the covariance output is rebuilt as L L^H
       if (P.nsim > 0) {
         const int fail = pair_factor(o);
         failed |= (unsigned int)fail << (2 * n);
         if ((fail & 1) && in0) n_zero_bins++;
         if ((fail & 2) && in1) n_zero_bins++;
       }
-      const uint32_t so = sl + s_post;
 #pragma unroll
       for (int a = 0; a < 3; a++) {
-        sts_c2(so + 16u * (uint32_t)(a << lnp), o.mu[a]);
+        if constexpr (MODE == kEig) sts_c2(so + 16u * (uint32_t)(a << lnp), o.mu[a]);
         sts_c2(so + 16u * (uint32_t)((3 + a) << lnp), o.so[a]);
       }
       diag_put(pos, P, q, o.sd);
@@ -719,7 +753,9 @@ __global__ void __launch_bounds__(512, 1) k_pencil(const __grid_constant__ ZPara
     int n = 0;
 #pragma unroll 1
     for (int b = tid; b < items; b += T, n++) {
-      const int q = b & (NP - 1), p = pos_of(b), kz = perm[p];
+      const int q = b & (NP - 1);
+      int p, kz;
+      locate(b >> lnp, p, kz);
       const uint32_t pos = tile + (uint32_t)(p * PS), sl = pos + 16u * (uint32_t)q, so = sl + s_post;
       const int fail = (failed >> (2 * n)) & 3;
       float2 ld[3];
@@ -783,10 +819,12 @@ __global__ void __launch_bounds__(512, 1) k_pencil(const __grid_constant__ ZPara
   if (P.cov_spectral) {
     if (tid < 3) outp[tid] = (unsigned long long)(uintptr_t)P.mean[tid];
     for (int b = tid; b < items; b += T) {
-      const int q = b & (NP - 1), p = b >> lnp;
+      const int q = b & (NP - 1);
+      int p, kz;
+      locate(b >> lnp, p, kz);
       const uint32_t pos = tile + (uint32_t)(p * PS), so = pos + 16u * (uint32_t)q + s_post;
       const bool in0 = 2 * q >= wlo && 2 * q < nw, in1 = 2 * q + 1 < nw;
-      const size_t gidx = base + (size_t)perm[p] * kstride + 2 * q;
+      const size_t gidx = base + (size_t)kz * kstride + 2 * q;
       float2 sd[3];
       diag_get(pos, P, q, sd);
 #pragma unroll
@@ -889,15 +927,22 @@ inline cudaError_t launch_pencil_t(const ZParams& zp, int threads, cudaStream_t 
   const size_t bytes = sizeof(float2) * (size_t)(12 + zp.nth + 3 * zp.nsim) * zp.cnxp * zp.nyp * zp.nzp;
   return launch_dep(bytes, fn, dim3((unsigned)(zp.nIT * zp.nyp)), threads, smem, st, zp);
 }
+// the lengths whose split is inlined (pencil_plan gives the same)
+template <int NTH, int MODE>
+inline cudaError_t launch_pencil_z(const ZParams& zp, int threads, cudaStream_t st) {
+  switch (zp.nzp) {
+#define CRAVA_CASE(N, R0, R1) \
+  case N: return launch_pencil_t<NTH, MODE, R0, R1>(zp, threads, st);
+    CRAVA_Z_INLINED(CRAVA_CASE)
+#undef CRAVA_CASE
+    default: return launch_pencil_t<NTH, MODE, 0, 0>(zp, threads, st);
+  }
+}
 template <int NTH>
 inline cudaError_t launch_pencil_m(const ZParams& zp, int threads, cudaStream_t st) {
-  if (zp.fp64_threshold > 0.f) return launch_pencil_t<NTH, kCholFp64, 0, 0>(zp, threads, st);
-  if (!zp.eig) return launch_pencil_t<NTH, kChol, 0, 0>(zp, threads, st);
-  // the z lengths of the benchmark blocks inline their split (pencil_plan gives the same)
-  if (zp.nzp == 256) return launch_pencil_t<NTH, kEig, 16, 16>(zp, threads, st);
-  if (zp.nzp == 320) return launch_pencil_t<NTH, kEig, 20, 16>(zp, threads, st);
-  if (zp.nzp == 128) return launch_pencil_t<NTH, kEig, 16, 8>(zp, threads, st);
-  return launch_pencil_t<NTH, kEig, 0, 0>(zp, threads, st);
+  if (zp.fp64_threshold > 0.f) return launch_pencil_z<NTH, kCholFp64>(zp, threads, st);
+  if (!zp.eig) return launch_pencil_z<NTH, kChol>(zp, threads, st);
+  return launch_pencil_z<NTH, kEig>(zp, threads, st);
 }
 
 // launchers by angle count (pencil_n12.cu, pencil_n34.cu, pencil_n56.cu, pencil_n78.cu): one
