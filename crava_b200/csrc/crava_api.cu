@@ -657,7 +657,7 @@ void build_kz_tables(const crava_job_desc& d, std::vector<float2>& kw, std::vect
 // Jobs whose pencil pass is the scalar one (zpass.cuh): residual spectra kept, at the z lengths where
 // pencil.cuh's transform has another order of roundings.
 bool pencil_scalar(const crava_job_desc* d) {
-  return (d->flags & CRAVA_FLAG_KEEP_RESIDUAL) && d->nzp != 128 && d->nzp != 256 && d->nzp != 320;
+  return (d->flags & CRAVA_FLAG_KEEP_RESIDUAL) && !z_inlined(d->nzp);
 }
 
 // Eigen tables of a separable-prior job: bytes on the device (0 for other priors).

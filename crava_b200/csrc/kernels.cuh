@@ -80,6 +80,12 @@ bool pencil_plan(int n, ZPlan& z);
 // and the 5 x 2^6 that blocks are usually padded to.  The calls of the general stages cost a tenth of the instructions
 // (pencil.cuh) and more of a small block's latency (64x60x320, prior grids: 178 against 140 us).
 #define CRAVA_Z_INLINED(X) X(128, 16, 8) X(256, 16, 16) X(320, 20, 16)
+constexpr bool z_inlined(int nzp) {
+#define CRAVA_CASE(N, R0, R1) if (nzp == N) return true;
+  CRAVA_Z_INLINED(CRAVA_CASE)
+#undef CRAVA_CASE
+  return false;
+}
 // kz at position p of a line after the forward stages (in place, digits reversed)
 int pencil_kz(const ZPlan& z, int p);
 

@@ -163,7 +163,8 @@ bool pencil_shape(ZParams& zp, int* threads) {
 
 cudaError_t launch_pencil(const ZParams& zp, int threads, cudaStream_t st, int* nlaunch) {
   if (zp.NP < 1 || zp.W != 2 * zp.NP || (1 << zp.logNP) != zp.NP || threads < 64 || threads > 512 ||
-      zp.SB < (zp.nsim ? 1 : 0) || zp.SB > 4 || zp.nzp * zp.NP > 16 * threads)
+      zp.SB < (zp.nsim ? 1 : 0) || zp.SB > 4 || zp.nzp * zp.NP > 16 * threads ||
+      (zp.keep_resid && !z_inlined(zp.nzp)))
     return cudaErrorInvalidValue;
   if (nlaunch) (*nlaunch)++;
   switch (zp.nth) {

@@ -311,7 +311,7 @@ __device__ __forceinline__ C2 c2_submul(C2 x, float kr, float ki, C2 y) {
 // mu_post and S_post of the two bins of one z position from that position's row e (float4 groups
 // at stride nzp, laid out as EigLayout: the angles' rows are streamed one at a time), and with
 // RES the residuals in d.
-template <int NTH>
+template <int NTH, bool RES>
 __device__ __forceinline__ void pair_posterior_eig(const ZParams& P, const float4* __restrict__ e, float2 lam,
                                                    float2 rho, const C2 (&mu)[3], C2 (&d)[NTH], PairPost& o) {
   constexpr int VP = pad4(2 * NTH), OKW = 0, OL = VP, OR = OL + pad4(NTH), RS = VP + 16;
@@ -363,7 +363,7 @@ __device__ __forceinline__ void pair_posterior_eig(const ZParams& P, const float
   }
   // residual d - K mu_post = y - K (mu_post - mu) (the data spectrum itself where the row is zero:
   // kz not inverted)
-  if (P.keep_resid) {
+  if (RES && P.keep_resid) {
     float kw[VP];
     ldrow(kw, e + (OKW / 4) * st, st);
     C2 dm[3];
@@ -494,6 +494,7 @@ __global__ void __launch_bounds__(512, 1) k_pencil(const __grid_constant__ ZPara
   extern __shared__ __align__(16) unsigned char smb[];
   __shared__ unsigned long long cnt[4];
   constexpr int GIN = NTH + 3;
+  constexpr bool kResid = R0 != 0;   // residual spectra at the other lengths are zpass.cuh's
   const int NZ = P.nzp, NP = P.NP, lnp = P.logNP, W = 2 * NP, SB = P.SB, PS = P.PS;
   const int T = blockDim.x, tid = threadIdx.x;
   const uint32_t s_tw = smem_addr(smb), s_out = s_tw + 8u * (uint32_t)even_up_z(NZ), s_perm = s_out + 96u;
@@ -664,10 +665,11 @@ __global__ void __launch_bounds__(512, 1) k_pencil(const __grid_constant__ ZPara
 #pragma unroll
         for (int c = 0; c < 6; c++) bo.sp[c] = make_float2(S[c], 0.f);
       }
-      if (P.keep_resid && in) {
+      if constexpr (kResid)
+        if (P.keep_resid && in) {
 #pragma unroll
-        for (int l = 0; l < NTH; l++) P.data[l][gi] = d1[l];
-      }
+          for (int l = 0; l < NTH; l++) P.data[l][gi] = d1[l];
+        }
 #pragma unroll
       for (int a = 0; a < 3; a++) {
         const uint32_t xm = sl + s_post + 16u * (uint32_t)(a << lnp), xs = sl + s_post + 16u * (uint32_t)((3 + a) << lnp);
@@ -706,15 +708,16 @@ __global__ void __launch_bounds__(512, 1) k_pencil(const __grid_constant__ ZPara
           lam = make_float2(fabsf(c0), fabsf(c1));
           rho = make_float2(fabsf(c0 * ctk), fabsf(c1 * ctk));
         }
-        pair_posterior_eig<NTH>(P, P.eig + p, lam, rho, mu, d, o);
-        if (P.keep_resid) {
-          const size_t gidx = base + (size_t)kz * kstride + 2 * q;
+        pair_posterior_eig<NTH, kResid>(P, P.eig + p, lam, rho, mu, d, o);
+        if constexpr (kResid)
+          if (P.keep_resid) {
+            const size_t gidx = base + (size_t)kz * kstride + 2 * q;
 #pragma unroll
-          for (int l = 0; l < NTH; l++) {
-            if (in0) P.data[l][gidx] = make_float2(d[l].r.x, d[l].i.x);
-            if (in1) P.data[l][gidx + 1] = make_float2(d[l].r.y, d[l].i.y);
+            for (int l = 0; l < NTH; l++) {
+              if (in0) P.data[l][gidx] = make_float2(d[l].r.x, d[l].i.x);
+              if (in1) P.data[l][gidx + 1] = make_float2(d[l].r.y, d[l].i.y);
+            }
           }
-        }
       } else {
         diag_get(pos, P, q, o.sd);
 #pragma unroll

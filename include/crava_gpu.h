@@ -80,7 +80,9 @@ enum {
 enum {
   CRAVA_FLAG_HOST_NOISE = 1,   /* realisation noise uploaded by the caller (parity with a
                                   sequential generator such as the reference RandomGen)   */
-  CRAVA_FLAG_KEEP_RESIDUAL = 2, /* keep the residual spectra for CRAVA_ROLE_RESIDUAL         */
+  CRAVA_FLAG_KEEP_RESIDUAL = 2, /* keep the residual spectra for CRAVA_ROLE_RESIDUAL; such a
+                                   job transforms in another order of operations, so that the
+                                   other outputs differ from a plain job's in their last bits */
   CRAVA_FLAG_SPECTRAL_COV = 4,  /* leave the posterior covariance in the Fourier domain, as
                                    the reference holds it between computePostMeanResidAndFFTCov
                                    and invFFTCovGrids (src/avoinversion.cpp:1071-1077,
