@@ -448,27 +448,31 @@ __device__ __forceinline__ void x4_prefetch(const GridSet& gs, int rows, int rpc
 // A chunk of rows is one contiguous run of global memory.  It comes in by 16-byte cp.async and
 // its results, written over it in shared memory, leave by one bulk copy (cp.async.bulk, issued by
 // one thread), so the passes spend no instructions on global addresses and every global access is
-// a full line.  al16: the chunk starts on a 16-byte boundary (the grid is 16-byte aligned and the
-// chunk starts at an even row: two rows are a multiple of 16 bytes whatever nxp is); without it
-// both ways move 8-byte words.
+// a full line.  al: 16 where the chunk starts on a 16-byte boundary (the grid is 16-byte aligned and the
+// chunk starts at an even row: two rows are a multiple of 16 bytes whatever nxp is); 8 otherwise: both
+// ways move 8-byte words; 4 where the real input of an odd length starts off an 8-byte boundary, which needs
+// no more than a float's alignment (its rows were never read as pairs): 4-byte words in.
 
 // n 8-byte words from src to dst (shared, 16-byte aligned); the caller commits and waits.
-__device__ __forceinline__ void rows_in(float2* dst, const float2* src, int n, bool al16) {
+__device__ __forceinline__ void rows_in(float2* dst, const float2* src, int n, int al) {
   const uint32_t d = smem_addr(dst);
-  if (al16) {
+  if (al == 16) {
     const int n2 = n >> 1;
     for (int e = threadIdx.x; e < n2; e += blockDim.x) cp_async16(d + 16u * (uint32_t)e, src + 2 * e);
     if ((n & 1) && threadIdx.x == 0) cp_async8(d + 8u * (uint32_t)(n - 1), src + n - 1);
-  } else {
+  } else if (al == 8) {
     for (int e = threadIdx.x; e < n; e += blockDim.x) cp_async8(d + 8u * (uint32_t)e, src + e);
+  } else {
+    const float* f = reinterpret_cast<const float*>(src);
+    for (int e = threadIdx.x; e < 2 * n; e += blockDim.x) cp_async4(d + 4u * (uint32_t)e, f + e);
   }
   cp_async_commit();
 }
 
 // n 8-byte words from src (shared, 16-byte aligned, written by this CTA's threads, no barrier
 // since) to dst.  Returns when shared memory may be given back.
-__device__ __forceinline__ void rows_out(float2* dst, const float2* src, int n, bool al16) {
-  if (al16) {
+__device__ __forceinline__ void rows_out(float2* dst, const float2* src, int n, int al) {
+  if (al == 16) {
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -533,7 +537,7 @@ __global__ void __launch_bounds__(256) k_xr2c4(const __grid_constant__ GridSet g
 template <int N1, int N2>
 __global__ void __launch_bounds__(256) k_xc2r4(const __grid_constant__ GridSet gs, int rows, int rpc,
                                                const float2* __restrict__ twg, const float2* __restrict__ twn,
-                                               int al16, int pf) {
+                                               int al, int pf) {
   constexpr int H = N1 * N2, CN = H + 1;
   extern __shared__ __align__(16) float2 sm[];
   float2* tw = sm;
@@ -543,7 +547,7 @@ __global__ void __launch_bounds__(256) k_xc2r4(const __grid_constant__ GridSet g
   float2* g = reinterpret_cast<float2*>(gs.p[blockIdx.y]) + (size_t)row0 * CN;
   dep_wait();
   dep_launch();
-  rows_in(Xs, g, nr * CN, al16);
+  rows_in(Xs, g, nr * CN, al);
   if (pf > 0) x4_prefetch<false>(gs, rows, rpc, CN, pf);
   for (int t = threadIdx.x; t < H; t += blockDim.x) {
     tw[t] = twg[t];
@@ -553,7 +557,7 @@ __global__ void __launch_bounds__(256) k_xc2r4(const __grid_constant__ GridSet g
   __syncthreads();
   if constexpr (RowPairs<N1, N2>::ok) xc2r4_pairs<N1, N2>(Xs, nr, gs.scale[blockIdx.y], tw, twh);
   else xc2r4_staged<N1, N2>(Xs, Xs, nr, gs.scale[blockIdx.y], tw, twh, Xs + even_up(rpc * CN));
-  rows_out(g, Xs, nr * CN, al16);
+  rows_out(g, Xs, nr * CN, al);
 }
 
 // ------------------------------------------------------------------ rows, odd nxp
@@ -568,7 +572,7 @@ __global__ void __launch_bounds__(256) k_xc2r4(const __grid_constant__ GridSet g
 // Rows in global and staged memory have N + 1 floats; the last is written as zero.
 template <int N1, int N2>
 __global__ void __launch_bounds__(256) k_xr2c4o(const __grid_constant__ GridSet gs, int rows, int lpc,
-                                                const float2* __restrict__ twg, int al16) {
+                                                const float2* __restrict__ twg, int al) {
   using L = RowLayout<N1, N2>;
   constexpr int N = N1 * N2, CN = (N + 1) / 2, NPI = N1 / 2 + 1;
   extern __shared__ __align__(16) float2 sm[];
@@ -581,7 +585,7 @@ __global__ void __launch_bounds__(256) k_xr2c4o(const __grid_constant__ GridSet 
   dep_wait();
   dep_launch();
   x_clear(gs);
-  rows_in(Xs, reinterpret_cast<const float2*>(gs.src[blockIdx.y]) + o, nr * CN, al16);
+  rows_in(Xs, reinterpret_cast<const float2*>(gs.src[blockIdx.y]) + o, nr * CN, al);
   for (int t = tid; t < N; t += T) tw[t] = twg[t];
   cp_async_wait_0();
   __syncthreads();
@@ -622,12 +626,12 @@ __global__ void __launch_bounds__(256) k_xr2c4o(const __grid_constant__ GridSet 
       if (two) XA[CN + k0] = make_float2(hs * (p.y + m.y), hs * (m.x - p.x));
     }
   }
-  rows_out(reinterpret_cast<float2*>(gs.p[blockIdx.y]) + o, Xs, nr * CN, al16);
+  rows_out(reinterpret_cast<float2*>(gs.p[blockIdx.y]) + o, Xs, nr * CN, al);
 }
 
 template <int N1, int N2>
 __global__ void __launch_bounds__(256) k_xc2r4o(const __grid_constant__ GridSet gs, int rows, int lpc,
-                                                const float2* __restrict__ twg, int al16) {
+                                                const float2* __restrict__ twg, int al) {
   using L = RowLayout<N1, N2>;
   constexpr int N = N1 * N2, CN = (N + 1) / 2;
   extern __shared__ __align__(16) float2 sm[];
@@ -639,7 +643,7 @@ __global__ void __launch_bounds__(256) k_xc2r4o(const __grid_constant__ GridSet 
   float2* g = reinterpret_cast<float2*>(gs.p[blockIdx.y]) + (size_t)row0 * CN;
   dep_wait();
   dep_launch();
-  rows_in(Xs, g, nr * CN, al16);
+  rows_in(Xs, g, nr * CN, al);
   for (int t = tid; t < N; t += T) tw[t] = twg[t];
   cp_async_wait_0();
   __syncthreads();
@@ -680,7 +684,7 @@ __global__ void __launch_bounds__(256) k_xc2r4o(const __grid_constant__ GridSet 
       if (two) a[2 * N + 1] = 0.f;
     }
   }
-  rows_out(g, Xs, nr * CN, al16);
+  rows_out(g, Xs, nr * CN, al);
 }
 
 static inline cudaError_t resident_grid(const void* fn, int T, size_t smem, int units, int* grid) {
@@ -802,10 +806,11 @@ static inline RowShape row_shape(int i1, int c1, int i2, int c2, size_t fixed, s
   return best;
 }
 
-static inline bool grids_al16(const GridSet& gs) {
+// the alignment that every grid of the set has, inputs (of a forward transform) included: 16, 8 or 4
+static inline int grids_align(const GridSet& gs, bool fwd) {
   uintptr_t a = 0;
-  for (int q = 0; q < gs.n; q++) a |= reinterpret_cast<uintptr_t>(gs.p[q]) | reinterpret_cast<uintptr_t>(gs.src[q]);
-  return a % 16 == 0;
+  for (int q = 0; q < gs.n; q++) a |= reinterpret_cast<uintptr_t>(gs.p[q]) | (fwd ? reinterpret_cast<uintptr_t>(gs.src[q]) : 0);
+  return a % 16 == 0 ? 16 : a % 8 == 0 ? 8 : 4;
 }
 
 // Row pairs per CTA of xc2r4_pairs: one item per thread and pass, by the same estimate as row_shape.
@@ -867,10 +872,10 @@ static cudaError_t x4(bool fwd, const GridSet& gs, int rows, const float2* tw, c
     pf = std::max(1, res * q / 4);
   }
   // every chunk starts at an even row, or two rows' bytes do not matter ((h + 1) even)
-  const int al16 = grids_al16(gs) && (rpc % 2 == 0 || (H + 1) % 2 == 0);
+  const int al = std::min(grids_align(gs, fwd), rpc % 2 == 0 || (H + 1) % 2 == 0 ? 16 : 8);
   const size_t bytes = sizeof(float2) * (size_t)gs.n * rows * (H + 1);
   return fwd ? launch_dep(bytes, k_xr2c4<N1, N2>, grid, T, smem, st, gs, rows, rpc, tw, twn, stage, pf)
-             : launch_dep(bytes, k_xc2r4<N1, N2>, grid, T, smem, st, gs, rows, rpc, tw, twn, al16, pf);
+             : launch_dep(bytes, k_xc2r4<N1, N2>, grid, T, smem, st, gs, rows, rpc, tw, twn, al, pf);
 }
 
 // odd nxp = N1 N2: rows taken in pairs
@@ -885,10 +890,10 @@ static cudaError_t x4_odd(bool fwd, const GridSet& gs, int rows, const float2* t
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   dim3 grid((unsigned)((rows + 2 * rs.lines - 1) / (2 * rs.lines)), gs.n);
-  const int al16 = grids_al16(gs);
+  const int al = grids_align(gs, fwd);
   const size_t bytes = sizeof(float) * (size_t)gs.n * rows * (N + 1);
-  return fwd ? launch_dep(bytes, k_xr2c4o<N1, N2>, grid, rs.T, smem, st, gs, rows, rs.lines, tw, al16)
-             : launch_dep(bytes, k_xc2r4o<N1, N2>, grid, rs.T, smem, st, gs, rows, rs.lines, tw, al16);
+  return fwd ? launch_dep(bytes, k_xr2c4o<N1, N2>, grid, rs.T, smem, st, gs, rows, rs.lines, tw, al)
+             : launch_dep(bytes, k_xc2r4o<N1, N2>, grid, rs.T, smem, st, gs, rows, rs.lines, tw, al);
 }
 
 }  // namespace crava

@@ -26,14 +26,14 @@ __global__ void __launch_bounds__(256) k_xc2r4_facies(const __grid_constant__ Fa
     tw[t] = twg[t];
     twh[t] = twn[t];
   }
-  for (int a = 0; a < 3; a++) rows_in(V + a * bw, reinterpret_cast<const float2*>(F.mean[a]) + (size_t)row0 * CN, nr * CN, false);
+  for (int a = 0; a < 3; a++) rows_in(V + a * bw, reinterpret_cast<const float2*>(F.mean[a]) + (size_t)row0 * CN, nr * CN, 8);
   cp_async_wait_0();
   __syncthreads();
   for (int a = 0; a < 3; a++) {
     float2* B = V + a * bw;
     if constexpr (RowPairs<N1, N2>::ok) xc2r4_pairs<N1, N2>(B, nr, F.scale, tw, twh);
     else xc2r4_staged<N1, N2>(B, B, nr, F.scale, tw, twh, V + 3 * bw);
-    rows_out(reinterpret_cast<float2*>(F.mean[a]) + (size_t)row0 * CN, B, nr * CN, false);
+    rows_out(reinterpret_cast<float2*>(F.mean[a]) + (size_t)row0 * CN, B, nr * CN, 8);
     __syncthreads();
   }
   const float* Vf = reinterpret_cast<const float*>(V);
