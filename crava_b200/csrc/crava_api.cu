@@ -209,8 +209,9 @@ struct crava_ctx {
   long long kt_n[KT_COUNT] = {};
   // stream-ordered scratch of the facies, local-noise and prior calls: a memory pool of the context's own that keeps up to
   // kScratchKeep between calls (the default pool gives its memory back at every synchronisation,
-  // and mapping it again took up to milliseconds); destroyed with the context, emptied when a job
-  // finds no memory
+  // and mapping it again took up to milliseconds); destroyed with the context, emptied when any other
+  // allocation of the context finds no memory (alloc_or_trim)
+  std::mutex scratch_mu;
   cudaMemPool_t scratch = nullptr;
   std::mutex stage_mu;         // device staging grid of the host-grid transforms
   float* stage = nullptr;
@@ -232,21 +233,46 @@ namespace {
 constexpr uint64_t kScratchKeep = 256ull << 20;
 
 cudaError_t scratch_alloc(crava_ctx* ctx, void** p, size_t bytes, cudaStream_t st) {
+  cudaMemPool_t pool = nullptr;
   {
-    std::lock_guard<std::mutex> lk(ctx->mu);
+    std::lock_guard<std::mutex> lk(ctx->scratch_mu);
     if (!ctx->scratch) {
       cudaMemPoolProps pr = {};
       pr.allocType = cudaMemAllocationTypePinned;
       pr.location.type = cudaMemLocationTypeDevice;
       pr.location.id = ctx->device;
-      cudaError_t e = cudaMemPoolCreate(&ctx->scratch, &pr);
+      cudaError_t e = cudaMemPoolCreate(&pool, &pr);
       if (e != cudaSuccess) return e;
       uint64_t keep = kScratchKeep;
-      e = cudaMemPoolSetAttribute(ctx->scratch, cudaMemPoolAttrReleaseThreshold, &keep);
-      if (e != cudaSuccess) return e;
+      e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+      if (e != cudaSuccess) {
+        cudaMemPoolDestroy(pool);
+        return e;
+      }
+      ctx->scratch = pool;
     }
+    pool = ctx->scratch;
   }
-  return cudaMallocFromPoolAsync(p, bytes, ctx->scratch, st);
+  return cudaMallocFromPoolAsync(p, bytes, pool, st);
+}
+
+void scratch_give_back(crava_ctx* ctx) {
+  std::lock_guard<std::mutex> lk(ctx->scratch_mu);
+  if (ctx->scratch) cudaMemPoolTrimTo(ctx->scratch, 0);
+}
+
+// alloc(), once more without the kept scratch if it finds no memory
+template <class F>
+cudaError_t alloc_or_trim(crava_ctx* ctx, F alloc) {
+  cudaError_t e = alloc();
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  scratch_give_back(ctx);
+  return alloc();
+}
+template <class T>
+cudaError_t device_alloc(crava_ctx* ctx, T** p, size_t bytes) {
+  return alloc_or_trim(ctx, [&] { return cudaMalloc((void**)p, bytes); });
 }
 
 void cache_evict_locked(crava_ctx* ctx, size_t want, cudaStream_t st);
@@ -381,7 +407,7 @@ crava_status get_plan(crava_ctx* ctx, int n, Plan** out, bool allow16) {
     double ang = 2.0 * M_PI * (double)t / (double)n;
     tw[t] = make_float2((float)std::cos(ang), (float)(-std::sin(ang)));
   }
-  CUDA_TRY(cudaMalloc(&p.tw, sizeof(float2) * n));
+  CUDA_TRY(device_alloc(ctx, &p.tw, sizeof(float2) * n));
   CUDA_TRY(cudaMemcpy(p.tw, tw.data(), sizeof(float2) * n, cudaMemcpyHostToDevice));
   auto res = ctx->plans.emplace(key, p);
   *out = &res.first->second;
@@ -1099,7 +1125,7 @@ crava_status io_buffers(crava_ctx* ctx) {
     if (!ctx->io_host[b]) CUDA_TRY(cudaHostAlloc((void**)&ctx->io_host[b], kIoChunk, cudaHostAllocDefault));
     if (!ctx->io_ev[b]) CUDA_TRY(cudaEventCreateWithFlags(&ctx->io_ev[b], cudaEventDisableTiming));
   }
-  if (!ctx->io_dev) CUDA_TRY(cudaMalloc(&ctx->io_dev, 2 * kIoChunk));
+  if (!ctx->io_dev) CUDA_TRY(device_alloc(ctx, &ctx->io_dev, 2 * kIoChunk));
   return CRAVA_OK;
 }
 
@@ -1573,7 +1599,7 @@ crava_status crava_grid_write_segy(crava_ctx* ctx, const char* path, const float
   const size_t hb = align256(nrec * 240), tb = align256(nrec * sizeof(SegyTrace));
   cudaError_t e = cudaSuccess;
   if (nrec) {
-    e = cudaMallocAsync((void**)&dmem, hb + tb, st);
+    e = alloc_or_trim(ctx, [&] { return cudaMallocAsync((void**)&dmem, hb + tb, st); });
     if (e == cudaSuccess) e = cudaMemcpyAsync(dmem, hdr.data(), nrec * 240, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(dmem + hb, trs.data(), nrec * sizeof(SegyTrace), cudaMemcpyHostToDevice, st);
   }
@@ -2087,7 +2113,7 @@ crava_status cache_acquire(crava_ctx* ctx, const std::string& key, size_t bytes,
   CacheEntry* e = new CacheEntry();
   e->key = key;
   e->bytes = bytes;
-  cudaError_t ce = cudaMallocAsync((void**)&e->mem, bytes, st);
+  cudaError_t ce = alloc_or_trim(ctx, [&] { return cudaMallocAsync((void**)&e->mem, bytes, st); });
   crava_status s = ce == cudaSuccess ? build(e->mem, *e) : fail(CRAVA_ENOMEM, "table cache allocation");
   if (!s && cudaEventCreateWithFlags(&e->ready, cudaEventDisableTiming) != cudaSuccess) s = CRAVA_ECUDA;
   if (!s && cudaEventRecord(e->ready, st) != cudaSuccess) s = CRAVA_ECUDA;
@@ -2184,12 +2210,7 @@ crava_status job_create_impl(crava_ctx* ctx, const crava_job_desc* desc, cudaStr
   auto pool_alloc = [&] {
     return async ? cudaMallocAsync((void**)&j->pool, need, st) : cudaMalloc(&j->pool, need);
   };
-  cudaError_t e = injected ? cudaErrorMemoryAllocation : pool_alloc();
-  if (e != cudaSuccess && !injected && ctx->scratch) {   // the kept scratch gives way to a job
-    cudaGetLastError();
-    cudaMemPoolTrimTo(ctx->scratch, 0);
-    e = pool_alloc();
-  }
+  const cudaError_t e = alloc_or_trim(ctx, [&] { return injected ? cudaErrorMemoryAllocation : pool_alloc(); });
   if (e != cudaSuccess) {
     cudaGetLastError();
     j->pool = nullptr;
@@ -2902,7 +2923,7 @@ crava_status crava_job_set_wavelet_grids(crava_job* job, int angle, const float*
   }
   CUDA_TRY(cudaSetDevice(job->ctx->device));
   if (!job->wgrid) {
-    CUDA_TRY(cudaMalloc(&job->wgrid, sizeof(float) * 2 * d.ntheta * nxy));
+    CUDA_TRY(device_alloc(job->ctx, &job->wgrid, sizeof(float) * 2 * d.ntheta * nxy));
     std::vector<float> init(2 * d.ntheta * nxy, 0.f);
     std::fill(init.begin() + d.ntheta * nxy, init.end(), 1.f);
     CUDA_TRY(cudaMemcpy(job->wgrid, init.data(), sizeof(float) * init.size(), cudaMemcpyHostToDevice));
@@ -2969,7 +2990,7 @@ crava_status crava_job_set_wavelet_3d(crava_job* job, const crava_wavelet3d_desc
   const size_t o_par = align256(sizeof(double) * nth * nxy);
   const size_t o_glob = o_par + align256(sizeof(float4) * nth * nxy);
   if (!job->w3mem) {
-    CUDA_TRY(cudaMalloc(&job->w3mem, o_glob + sizeof(float2) * nth * cn));
+    CUDA_TRY(device_alloc(job->ctx, &job->w3mem, o_glob + sizeof(float2) * nth * cn));
     job->w3mult = (double*)job->w3mem;
     job->w3par = (float4*)((char*)job->w3mem + o_par);
     job->w3glob = (float2*)((char*)job->w3mem + o_glob);
@@ -2986,7 +3007,7 @@ crava_status crava_job_set_wavelet_3d(crava_job* job, const crava_wavelet3d_desc
   } else {
     if (!job->wspec) {
       const std::vector<float2> ws = wavelet_spectra(d);
-      CUDA_TRY(cudaMalloc(&job->wspec, sizeof(float2) * ws.size()));
+      CUDA_TRY(device_alloc(job->ctx, &job->wspec, sizeof(float2) * ws.size()));
       CUDA_TRY(cudaMemcpy(job->wspec, ws.data(), sizeof(float2) * ws.size(), cudaMemcpyHostToDevice));
     }
     F.wamp = job->wspec;
@@ -3008,7 +3029,7 @@ crava_status crava_job_set_wavelet_3d(crava_job* job, const crava_wavelet3d_desc
   // the maps and surfaces, staged in one temporary allocation
   const size_t o_gy = align256(sizeof(float) * nxy), o_a = 2 * o_gy, o_h = o_a + align256(sizeof(float) * nth * nij);
   void* tmp = nullptr;
-  CUDA_TRY(cudaMalloc(&tmp, o_h + sizeof(float) * nth * nij));
+  CUDA_TRY(device_alloc(job->ctx, &tmp, o_h + sizeof(float) * nth * nij));
   char* tb = (char*)tmp;
   cudaError_t e = cudaSuccess;
   if (w->grad_x && e == cudaSuccess) e = cudaMemcpy(tb, w->grad_x, sizeof(float) * nxy, cudaMemcpyHostToDevice);
@@ -3053,7 +3074,7 @@ crava_status crava_job_residual_synthetics(crava_job* job, void* stream) {
   } else {
     if (!job->wspec) {
       const std::vector<float2> w = wavelet_spectra(d);
-      CUDA_TRY(cudaMalloc(&job->wspec, sizeof(float2) * w.size()));
+      CUDA_TRY(device_alloc(job->ctx, &job->wspec, sizeof(float2) * w.size()));
       CUDA_TRY(cudaMemcpy(job->wspec, w.data(), sizeof(float2) * w.size(), cudaMemcpyHostToDevice));
     }
     tp.wamp = job->wspec;
@@ -3118,7 +3139,7 @@ static crava_status fft_host(crava_ctx* ctx, float* hgrid, int nxp, int nyp, int
     if (ctx->stage) CUDA_TRY(cudaFree(ctx->stage));
     ctx->stage = nullptr;
     ctx->stage_bytes = 0;
-    CUDA_TRY(cudaMalloc(&ctx->stage, bytes));
+    CUDA_TRY(device_alloc(ctx, &ctx->stage, bytes));
     ctx->stage_bytes = bytes;
   }
   CUDA_TRY(cudaMemcpy(ctx->stage, hgrid, bytes, cudaMemcpyHostToDevice));
@@ -4022,7 +4043,7 @@ crava_status crava_job_set_facies(crava_job* job, const crava_facies_desc* corne
   const int nc = 1 << nang, nf = corners->nfacies;
   size_t bytes = align256(sizeof(float) * t.size());
   for (int c = 0; c < nc; c++) bytes += align256(facies_packed_bytes(hc.box[c], nf));
-  CUDA_TRY(cudaMalloc((void**)&job->fac_mem, bytes));
+  CUDA_TRY(device_alloc(job->ctx, &job->fac_mem, bytes));
   char* p = job->fac_mem;
   float* dt = (float*)p;
   p += align256(sizeof(float) * t.size());
