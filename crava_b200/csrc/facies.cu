@@ -37,9 +37,8 @@ __global__ void k_facies_prob_corners(const float* __restrict__ vp, const float*
       const float v[3] = {vp[g0 + i], vs[g0 + i], rho[g0 + i]};
       float val[kMaxFacies];
       const float sum = facies_voxel(v, i, j, nx, ny, C, nf, pr, undef_sum, val);
-      const FaciesQuot quot(sum);
-      for (int f = 0; f < nf; f++) out.p[f][e] = quot(val[f]);
-      out.p[nf][e] = quot(undef_sum);
+      for (int f = 0; f < nf; f++) out.p[f][e] = val[f] / sum;
+      out.p[nf][e] = undef_sum / sum;
       if (seis_lh) seis_lh[e] = sum;
     }
   }
@@ -51,7 +50,7 @@ __global__ void k_facies_prob_corners(const float* __restrict__ vp, const float*
 struct FaciesSingle {
   const float4* dens;
   int nb[3];
-  double vmin[3], idv[3];
+  double vmin[3], dv[3];
 };
 __global__ void __launch_bounds__(256) k_facies_prob_single(const float* __restrict__ vp, const float* __restrict__ vs,
                                                             const float* __restrict__ rho, int nx, int ny, int nz,
@@ -74,9 +73,9 @@ __global__ void __launch_bounds__(256) k_facies_prob_single(const float* __restr
       }
       int a1, a2, b1, b2, c1, c2;
       float wj, wk, wl;
-      axis_weights(__ldg(vp + g0 + i), C.vmin[0], C.idv[0], C.nb[0], a1, a2, wj);
-      axis_weights(__ldg(vs + g0 + i), C.vmin[1], C.idv[1], C.nb[1], b1, b2, wk);
-      axis_weights(__ldg(rho + g0 + i), C.vmin[2], C.idv[2], C.nb[2], c1, c2, wl);
+      axis_weights(__ldg(vp + g0 + i), C.vmin[0], C.dv[0], C.nb[0], a1, a2, wj);
+      axis_weights(__ldg(vs + g0 + i), C.vmin[1], C.dv[1], C.nb[1], b1, b2, wk);
+      axis_weights(__ldg(rho + g0 + i), C.vmin[2], C.dv[2], C.nb[2], c1, c2, wl);
       const float uj = 1.0f - wj, uk = 1.0f - wk, ul = 1.0f - wl;
       const float w8[8] = {uj * uk * ul, uj * uk * wl, uj * wk * ul, uj * wk * wl,
                            wj * uk * ul, wj * uk * wl, wj * wk * ul, wj * wk * wl};
@@ -101,11 +100,10 @@ __global__ void __launch_bounds__(256) k_facies_prob_single(const float* __restr
         d[f] = f < nf ? pr.p[f] * (d[f] > 0.f ? d[f] : 0.f) : 0.f;
         if (f < nf) sum += d[f];
       }
-      const FaciesQuot quot(sum);
 #pragma unroll
       for (int f = 0; f < 4; f++)
-        if (f < nf) out.p[f][e] = quot(d[f]);
-      out.p[nf][e] = quot(undef_sum);
+        if (f < nf) out.p[f][e] = d[f] / sum;
+      out.p[nf][e] = undef_sum / sum;
       if (seis_lh) seis_lh[e] = sum;
     }
   }
@@ -304,7 +302,7 @@ cudaError_t launch_facies_eval(const float* vp, const float* vs, const float* rh
     for (int d = 0; d < 3; d++) {
       F.nb[d] = hc.box[0].nb[d];
       F.vmin[d] = hc.box[0].vmin[d];
-      F.idv[d] = 1.0 / hc.box[0].dv[d];
+      F.dv[d] = hc.box[0].dv[d];
     }
     k_facies_prob_single<<<blocks, dim3(32, 8), 0, st>>>(vp, vs, rho, nx, ny, nz, rnxp_in, nyp_in, rnxp_out, F, nf, pr,
                                                          undef_sum, po, seis_lh);
@@ -335,7 +333,7 @@ FaciesCorners facies_corners(const FaciesCornersHost& hc) {
     for (int d = 0; d < 3; d++) {
       C.box[c].nb[d] = hc.box[c].nb[d];
       C.box[c].vmin[d] = hc.box[c].vmin[d];
-      C.box[c].idv[d] = 1.0 / hc.box[c].dv[d];
+      C.box[c].dv[d] = hc.box[c].dv[d];
     }
     C.box[c].rs = hc.box[c].rs;
     C.box[c].fstride = hc.box[c].fstride;

@@ -11,13 +11,13 @@ namespace crava {
 
 constexpr float kRMissing = -99999.0f;
 
-// Box of one density volume: bins (nb), lower edges (vmin) and inverse widths (idv) along
+// Box of one density volume: bins (nb), lower edges (vmin) and bin widths (dv) along
 // vp, vs, rho; density cube f at dens + f*fstride, element (j, k, l) at
 // j + rs*k + rs*nb[1]*l (rs = row stride, FFTGrid-padded or dense).
 struct FaciesBox {
   int nb[3];
   double vmin[3];
-  double idv[3];
+  double dv[3];
   int rs;
   size_t fstride;
 };
@@ -30,33 +30,16 @@ struct FaciesCorners {
 };
 
 // Index along one axis as Simbox::getInterpolationIndexes (value at bin centres, in
-// double as the reference, by the reciprocal width) and the clamping of findDensity: below the first
-// centre or beyond the last the value of the edge bin is used.
-__device__ __forceinline__ void axis_weights(float v, double vmin, double idv, int nb, int& i1, int& i2, float& w) {
-  const double f = ((double)v - vmin) * idv - 0.5;
+// double as the reference) and the clamping of findDensity: below the first centre or
+// beyond the last the value of the edge bin is used.
+__device__ __forceinline__ void axis_weights(float v, double vmin, double dv, int nb, int& i1, int& i2, float& w) {
+  const double f = ((double)v - vmin) / dv - 0.5;
   const int i = (int)floor(f);
   const bool lo = i < 0, hi = i >= nb - 1;
   i1 = lo ? 0 : hi ? nb - 1 : i;
   i2 = lo || hi ? i1 : i + 1;
   w = lo || hi ? 0.f : (float)(f - (double)i);
 }
-
-// n / sum for several n: one reciprocal and a correction step each, the division itself for zero, tiny,
-// infinite or NaN sums.
-struct FaciesQuot {
-  float sum, inv;
-  bool plain;
-  __device__ __forceinline__ explicit FaciesQuot(float s) {
-    sum = s;
-    inv = __frcp_rn(s);
-    plain = s > 1e-30f && s < 1e30f;
-  }
-  __device__ __forceinline__ float operator()(float n) const {
-    if (!plain) return n / sum;
-    const float q = __fmul_rn(n, inv);
-    return __fmaf_rn(__fmaf_rn(-q, sum, n), inv, q);
-  }
-};
 
 // 32 bytes of read-only global memory, 32-byte aligned, in one load
 __device__ __forceinline__ void ldg_pair(const float4* p, float4& a, float4& b) {
@@ -94,7 +77,7 @@ __device__ __forceinline__ float facies_voxel(const float (&v)[3], int i, int j,
     int a1[3], a2[3];
     float w[3];
 #pragma unroll
-    for (int d = 0; d < 3; d++) axis_weights(v[d], box.vmin[d], box.idv[d], box.nb[d], a1[d], a2[d], w[d]);
+    for (int d = 0; d < 3; d++) axis_weights(v[d], box.vmin[d], box.dv[d], box.nb[d], a1[d], a2[d], w[d]);
     const size_t sk = (size_t)box.nb[0], sl = (size_t)box.nb[0] * box.nb[1];
     const float wj = w[0], wk = w[1], wl = w[2];
     const bool edge = a1[0] == a2[0];     // beyond the first or last bin centre: its own value twice
