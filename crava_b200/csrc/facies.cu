@@ -22,12 +22,12 @@ __global__ void k_facies_prob_corners(const float* __restrict__ vp, const float*
                                       const float* __restrict__ rho, int nx, int ny, int nz, int rnxp_in, int nyp_in,
                                       int rnxp_out, const __grid_constant__ FaciesCorners C, int nf, FaciesPrior pr,
                                       float undef_sum, FaciesOut out, float* __restrict__ seis_lh) {
-  // a warp per row (32-bit index arithmetic), eight rows per CTA
+  // a warp per row (32-bit index arithmetic), eight rows per CTA; blockIdx.y takes a part of the rows
   const int rows = ny * nz;
   for (int r = blockIdx.x * blockDim.y + threadIdx.y; r < rows; r += gridDim.x * blockDim.y) {
     const int k = r / ny, j = r - k * ny;
     const size_t e0 = (size_t)rnxp_out * r, g0 = (size_t)rnxp_in * ((size_t)j + (size_t)nyp_in * k);
-    for (int i = threadIdx.x; i < rnxp_out; i += blockDim.x) {
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < rnxp_out; i += gridDim.y * blockDim.x) {
       const size_t e = e0 + i;
       if (i >= nx) {
         for (int f = 0; f <= nf; f++) out.p[f][e] = kRMissing;
@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(256) k_facies_prob_single(const float* __restr
   for (int r = blockIdx.x * blockDim.y + threadIdx.y; r < rows; r += gridDim.x * blockDim.y) {
     const int k = r / ny, j = r - k * ny;
     const size_t e0 = (size_t)rnxp_out * r, g0 = (size_t)rnxp_in * ((size_t)j + (size_t)nyp_in * k);
-    for (int i = threadIdx.x; i < rnxp_out; i += blockDim.x) {
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < rnxp_out; i += gridDim.y * blockDim.x) {
       const size_t e = e0 + i;
       if (i >= nx) {
         for (int f = 0; f <= nf; f++) out.p[f][e] = kRMissing;
@@ -295,7 +295,10 @@ cudaError_t launch_facies_eval(const float* vp, const float* vs, const float* rh
   for (int f = 0; f < nf; f++) pr.p[f] = prior[f];
   for (int f = 0; f <= nf; f++) po.p[f] = out[f];
   const FaciesCorners C = facies_corners(hc);
-  const int blocks = (int)std::min<size_t>(((size_t)ny * nz + 7) / 8, 148 * 32);
+  // a few long rows (a section of 4000 traces has 2 per slice) are shared by several warps each, until eight CTAs an
+  // SM have work (4000x2x40, 6 facies: 449 -> 58 us; 2000x1x200: 260 -> 64)
+  dim3 blocks((unsigned)std::min<size_t>(((size_t)ny * nz + 7) / 8, 148 * 32));
+  blocks.y = (unsigned)std::max(1, std::min((rnxp_out + 31) / 32, (148 * 8 + (int)blocks.x - 1) / (int)blocks.x));
   if (hc.nang == 0 && nf <= 4 && (size_t)hc.box[0].nb[0] * hc.box[0].nb[1] * hc.box[0].nb[2] < (1u << 30)) {
     FaciesSingle F;
     F.dens = hc.packed[0];

@@ -1,6 +1,7 @@
 """Facies probabilities at the edges of their arithmetic, in both kernels (up to four facies in registers, more in
 the general form): quotients below the normal range rounded as IEEE division rounds them, voxels exactly on
-a bin centre beside a cell that must not count, parameters that are not finite, and axes of one bin."""
+a bin centre beside a cell that must not count, parameters that are not finite, axes of one bin, and shapes
+of few long or many short rows."""
 import numpy as np
 import pytest
 
@@ -112,3 +113,18 @@ def test_one_bin_axes_and_values_that_are_not_finite(ctx, nf, nb):
     assert np.max(np.abs(lh - tot) / tot) < 2e-6
     for f in range(nf):
         assert np.max(np.abs(p[f] - val[f] / tot)) < 2e-6, f
+
+
+@pytest.mark.parametrize("nf", [3, 6])
+@pytest.mark.parametrize("dims", [(1000, 2, 3), (301, 1, 1), (2, 70, 90), (31, 9, 1), (33, 1, 300)])
+def test_rows_of_every_length(ctx, dims, nf):
+    """Few long rows are shared by warps, short ones leave lanes idle: every voxel once, none beyond."""
+    nx, ny, nz = dims
+    rng = np.random.default_rng(nx + nf)
+    dens = rng.uniform(0.1, 1.0, (nf, 4, 4, 4)).astype(np.float32)
+    cell = rng.integers(0, 4, (3, nz, ny, nx))
+    p, lh = prob(ctx, dens, *UNIT, np.ones(nf, np.float32), 0.0, cell.astype(np.float32) + np.float32(0.5))
+    at = dens[:, cell[2], cell[1], cell[0]]
+    tot = at.astype(np.float64).sum(axis=0)
+    assert np.max(np.abs(lh - tot) / tot) < 2e-6
+    assert np.max(np.abs(p[:nf] - at / tot)) < 2e-6
