@@ -3946,6 +3946,7 @@ crava_status facies_setup(const crava_facies_desc* corners, int nang, const floa
     hc.box[c].fstride = (size_t)density_row * corners[c].nbins[1] * corners[c].nbins[2];
     hc.dens[c] = d_density[c];
   }
+  hc.pairs = facies_pairs(hc, fd->nfacies);
   const size_t nxy = (size_t)nx * ny;
   t.assign((size_t)nang * nxy, 0.f);
   for (int a = 0; a < nang; a++) {
@@ -3988,13 +3989,13 @@ crava_status crava_facies_prob_local_noise(crava_ctx* ctx, const crava_facies_de
   hc.t = dt;
   // facies-interleaved copies of the volumes for the lookups
   size_t pbytes = 0;
-  for (int c = 0; c < nc; c++) pbytes += align256(facies_packed_bytes(hc.box[c], fd->nfacies));
+  for (int c = 0; c < nc; c++) pbytes += align256(facies_packed_bytes(hc.box[c], fd->nfacies, hc.pairs));
   char* pk = nullptr;
   CUDA_TRY(scratch_alloc(ctx, (void**)&pk, pbytes, st));
   size_t off = 0;
   for (int c = 0; c < nc; c++) {
     hc.packed[c] = (float4*)(pk + off);
-    off += align256(facies_packed_bytes(hc.box[c], fd->nfacies));
+    off += align256(facies_packed_bytes(hc.box[c], fd->nfacies, hc.pairs));
   }
   // undefSum = p_undefined / (bins of the first density volume), as the reference
   const float undef_sum = fd->p_undefined / (float)(fd->nbins[0] * fd->nbins[1] * fd->nbins[2]);
@@ -4042,14 +4043,14 @@ crava_status crava_job_set_facies(crava_job* job, const crava_facies_desc* corne
     return s;
   const int nc = 1 << nang, nf = corners->nfacies;
   size_t bytes = align256(sizeof(float) * t.size());
-  for (int c = 0; c < nc; c++) bytes += align256(facies_packed_bytes(hc.box[c], nf));
+  for (int c = 0; c < nc; c++) bytes += align256(facies_packed_bytes(hc.box[c], nf, hc.pairs));
   CUDA_TRY(device_alloc(job->ctx, &job->fac_mem, bytes));
   char* p = job->fac_mem;
   float* dt = (float*)p;
   p += align256(sizeof(float) * t.size());
   for (int c = 0; c < nc; c++) {
     hc.packed[c] = (float4*)p;
-    p += align256(facies_packed_bytes(hc.box[c], nf));
+    p += align256(facies_packed_bytes(hc.box[c], nf, hc.pairs));
   }
   if (!t.empty()) CUDA_TRY(cudaMemcpy(dt, t.data(), sizeof(float) * t.size(), cudaMemcpyHostToDevice));
   hc.t = nang > 0 ? dt : nullptr;

@@ -52,6 +52,7 @@ struct FaciesSingle {
   int nb[3];
   double vmin[3], dv[3];
 };
+template <bool PAIRS>
 __global__ void __launch_bounds__(256) k_facies_prob_single(const float* __restrict__ vp, const float* __restrict__ vs,
                                                             const float* __restrict__ rho, int nx, int ny, int nz,
                                                             int rnxp_in, int nyp_in, int rnxp_out,
@@ -83,8 +84,13 @@ __global__ void __launch_bounds__(256) k_facies_prob_single(const float* __restr
       float4 x[8];
 #pragma unroll
       for (int q = 0; q < 4; q++) {
-        ldg_pair(C.dens + 2 * (size_t)cell[q], x[q], x[4 + q]);
-        if (a1 == a2) x[4 + q] = x[q];
+        if constexpr (PAIRS) {
+          ldg_pair(C.dens + 2 * (size_t)cell[q], x[q], x[4 + q]);
+          if (a1 == a2) x[4 + q] = x[q];
+        } else {
+          x[q] = __ldg(C.dens + cell[q]);
+          x[4 + q] = __ldg(C.dens + cell[q] + (a2 - a1));
+        }
       }
       float d[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -109,9 +115,10 @@ __global__ void __launch_bounds__(256) k_facies_prob_single(const float* __restr
   }
 }
 
-// Packs one density volume: cell (j, k, l) <- the nf facies values max(0, dens_f) of (j, k, l) and of
-// (j + 1, k, l) (the last bin's own again), four per float4 (zero beyond nf), the pair of a group of
+// Packs one density volume: cell (j, k, l) <- the nf facies values max(0, dens_f) of (j, k, l) and, in pairs,
+// of (j + 1, k, l) (the last bin's own again), four per float4 (zero beyond nf), the pair of a group of
 // four side by side; dens_f at src + f * fstride + j + rs (k + nb1 l).
+template <bool PAIRS>
 __global__ void k_facies_pack(const float* __restrict__ src, int nb0, int nb1, int nb2, int rs, size_t fstride,
                               int nf, float4* __restrict__ dst) {
   const int nf4 = (nf + 3) / 4;
@@ -125,7 +132,7 @@ __global__ void k_facies_pack(const float* __restrict__ src, int nb0, int nb1, i
     const int kk = (int)(kl % nb1), l = (int)(kl / nb1);
     const size_t o = (size_t)rs * ((size_t)kk + (size_t)nb1 * l);
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
+    for (int h = 0; h < (PAIRS ? 2 : 1); h++) {
       const int jh = min(j + h, nb0 - 1);
       float x[4];
 #pragma unroll
@@ -133,7 +140,7 @@ __global__ void k_facies_pack(const float* __restrict__ src, int nb0, int nb1, i
         const int f = 4 * g + u;
         x[u] = f < nf ? fmaxf(0.f, __ldg(src + fstride * f + o + jh)) : 0.f;
       }
-      dst[2 * cidx + h] = make_float4(x[0], x[1], x[2], x[3]);
+      dst[(PAIRS ? 2 : 1) * cidx + h] = make_float4(x[0], x[1], x[2], x[3]);
     }
   }
 }
@@ -307,8 +314,8 @@ cudaError_t launch_facies_eval(const float* vp, const float* vs, const float* rh
       F.vmin[d] = hc.box[0].vmin[d];
       F.dv[d] = hc.box[0].dv[d];
     }
-    k_facies_prob_single<<<blocks, dim3(32, 8), 0, st>>>(vp, vs, rho, nx, ny, nz, rnxp_in, nyp_in, rnxp_out, F, nf, pr,
-                                                         undef_sum, po, seis_lh);
+    (hc.pairs ? k_facies_prob_single<true> : k_facies_prob_single<false>)<<<blocks, dim3(32, 8), 0, st>>>(
+        vp, vs, rho, nx, ny, nz, rnxp_in, nyp_in, rnxp_out, F, nf, pr, undef_sum, po, seis_lh);
     return cudaGetLastError();
   }
   k_facies_prob_corners<<<blocks, dim3(32, 8), 0, st>>>(vp, vs, rho, nx, ny, nz, rnxp_in, nyp_in, rnxp_out, C, nf, pr,
@@ -322,8 +329,8 @@ cudaError_t launch_facies_pack(const FaciesCornersHost& hc, int nf, cudaStream_t
   for (int c = 0; c < (1 << hc.nang); c++) {
     const size_t units = (size_t)hc.box[c].nb[0] * hc.box[c].nb[1] * hc.box[c].nb[2] * nf4;
     const int pb = (int)std::min<size_t>((units + 255) / 256, 148 * 8);
-    k_facies_pack<<<pb, 256, 0, st>>>(hc.dens[c], hc.box[c].nb[0], hc.box[c].nb[1], hc.box[c].nb[2], hc.box[c].rs,
-                                      hc.box[c].fstride, nf, hc.packed[c]);
+    (hc.pairs ? k_facies_pack<true> : k_facies_pack<false>)<<<pb, 256, 0, st>>>(
+        hc.dens[c], hc.box[c].nb[0], hc.box[c].nb[1], hc.box[c].nb[2], hc.box[c].rs, hc.box[c].fstride, nf, hc.packed[c]);
   }
   return cudaGetLastError();
 }
@@ -331,6 +338,7 @@ cudaError_t launch_facies_pack(const FaciesCornersHost& hc, int nf, cudaStream_t
 FaciesCorners facies_corners(const FaciesCornersHost& hc) {
   FaciesCorners C;
   C.nang = hc.nang;
+  C.pairs = hc.pairs;
   C.t = hc.t;
   for (int c = 0; c < (1 << hc.nang); c++) {
     for (int d = 0; d < 3; d++) {
@@ -345,8 +353,15 @@ FaciesCorners facies_corners(const FaciesCornersHost& hc) {
   return C;
 }
 
-size_t facies_packed_bytes(const FaciesBoxHost& b, int nf) {
-  return 2 * sizeof(float4) * (size_t)b.nb[0] * b.nb[1] * b.nb[2] * ((nf + 3) / 4);
+size_t facies_packed_bytes(const FaciesBoxHost& b, int nf, bool pairs) {
+  return (pairs ? 2 : 1) * sizeof(float4) * (size_t)b.nb[0] * b.nb[1] * b.nb[2] * ((nf + 3) / 4);
+}
+
+// 128 MB: the L2 holds 126.  4 volumes of 128 MB in all are faster in pairs, 16 of 256 MB are not (facies.cuh).
+bool facies_pairs(const FaciesCornersHost& hc, int nf) {
+  size_t bytes = 0;
+  for (int c = 0; c < (1 << hc.nang); c++) bytes += facies_packed_bytes(hc.box[c], nf, true);
+  return bytes <= 128u << 20;
 }
 
 cudaError_t launch_spec_mul(float2* a, const float2* b, size_t n, cudaStream_t st) {

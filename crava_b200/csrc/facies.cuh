@@ -24,6 +24,7 @@ struct FaciesBox {
 
 struct FaciesCorners {
   int nang;                          // angles with a noise scale: 2^nang corner volumes
+  int pairs;                         // cells packed in pairs
   const float* t;                    // nang x ny x nx relative noise scales in [0, 1]
   FaciesBox box[1 << kMaxFaciesAngles];
   const float4* dens[1 << kMaxFaciesAngles];   // packed volumes (k_facies_pack)
@@ -53,12 +54,14 @@ __device__ __forceinline__ void ldg_pair(const float4* p, float4& a, float4& b) 
 // sum_c prod_a (t_a or 1 - t_a by bit a of c) * trilinear_c, t_a the trace's relative noise
 // scale of angle a (calculateFaciesProb, :1961-1977).  nang = 0 is the single volume.
 //
-// The volumes are read packed (k_facies_pack): cell (j, k, l) of corner c holds, per group of four
-// facies, 32 bytes: the clamped densities of (j, k, l) and of (j + 1, k, l), so that a voxel makes
-// four 32-byte loads per volume and group and computes the cell indexes once per volume.  The
-// lookups are bound by the L1's one line a clock for scattered lanes: eight 16-byte loads took
-// 0.66 ms at 270x270x256 and one volume of 100x100x50, four 32-byte ones 0.63.  The float operations
-// per facies are the reference's, in its order.
+// The volumes are read packed (k_facies_pack): cell (j, k, l) of corner c holds, per group of four facies, the
+// clamped densities of (j, k, l) in 16 bytes or, packed in pairs, those of (j, k, l) and (j + 1, k, l) in
+// 32, so that a voxel makes four 32-byte loads per volume and group instead of eight, and computes the cell indexes
+// once per volume.  The lookups are bound by the L1's one line a clock for scattered lanes where the
+// volumes sit in the L2 (facies_pairs; with the packing, volumes of 100x100x50, eight against four loads: 270x270x256, one
+// volume, 3 facies 647 -> 428 us, 6 facies 1495 -> 1067; 200x200x100, 4 volumes, 6 facies, 128 MB in pairs 1568 -> 1270),
+// and by the bytes beyond it (16 volumes, 3 facies, 256 MB in pairs 3512 -> 3640, 6 facies 5843 -> 8856).  The
+// float operations per facies are the reference's, in its order.
 //
 // facies_voxel: the densities of voxel (i, j) of trace row j at the parameters v, prior-
 // weighted: val[f] = prior_f max(0, dens_f) and the returned sum = undef_sum + sum_f val[f]
@@ -93,10 +96,17 @@ __device__ __forceinline__ float facies_voxel(const float (&v)[3], int i, int j,
     for (int g = 0; g < nf4; g++) {
       float d[4] = {0.f, 0.f, 0.f, 0.f};
       float4 x[8];
+      const size_t next = edge ? 0 : nf4;
 #pragma unroll
       for (int q = 0; q < 4; q++) {
-        ldg_pair(P4 + 2 * (cell[q] * nf4 + g), x[q], x[4 + q]);
-        if (edge) x[4 + q] = x[q];
+        const size_t at = cell[q] * nf4 + g;
+        if (C.pairs) {
+          ldg_pair(P4 + 2 * at, x[q], x[4 + q]);
+          if (edge) x[4 + q] = x[q];
+        } else {
+          x[q] = __ldg(P4 + at);
+          x[4 + q] = __ldg(P4 + at + next);
+        }
       }
 #pragma unroll
       for (int q = 0; q < 8; q++) {

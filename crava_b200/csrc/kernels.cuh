@@ -351,12 +351,15 @@ struct SegyPack {
 cudaError_t launch_segy_pack(const SegyPack& P, size_t r0, int nr, uint32_t* out, cudaStream_t st);
 struct FaciesCornersHost {
   int nang;
+  bool pairs;                                     // cells packed in pairs (facies_pairs)
   const float* t;                                 // device, nang x ny x nx
   FaciesBoxHost box[1 << kMaxFaciesAngles];
   const float* dens[1 << kMaxFaciesAngles];       // device density volume of each corner
   float4* packed[1 << kMaxFaciesAngles];          // device scratch of facies_packed_bytes each
 };
-size_t facies_packed_bytes(const FaciesBoxHost& b, int nf);
+size_t facies_packed_bytes(const FaciesBoxHost& b, int nf, bool pairs);
+// whether the volumes of hc.box are packed in pairs: while they then fit the L2
+bool facies_pairs(const FaciesCornersHost& hc, int nf);
 // the probabilities from volumes already packed (launch_facies_prob_corners = pack + eval)
 cudaError_t launch_facies_eval(const float* vp, const float* vs, const float* rho, int nx, int ny, int nz, int rnxp_in,
                                int nyp_in, int rnxp_out, const FaciesCornersHost& hc, int nf, const float* prior,
