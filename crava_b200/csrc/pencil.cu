@@ -103,6 +103,9 @@ bool pencil_shape(ZParams& zp, int* threads) {
       t = std::max(64, std::min(t, (zp.nzp * w / per + 31) / 32 * 32));
       const int ctas = resident(smem, t);
       const long long tiles = (long long)((zp.cnxp + w - 1) / w) * zp.nyp, slots = 148LL * ctas;
+      // eight bins only where they leave two tiles for every SM: a small block is as fast as one tile, and half
+      // as wide a tile is faster (20x20x40, 2 angles, 16 realisations, 40 tiles of 8 bins: 105 us, 60 of 4: 54)
+      if (w == 8 && tw <= 0 && tiles < 2 * 148) break;
       const double fill = (double)tiles / ((tiles + slots - 1) / slots * slots);
       double c = w == 8 ? 1.0 : w == 4 ? 1.02 : 1.35;
       if (zp.nsim > 1) c *= b == 1 ? 1.05 : b == 4 && w == 8 ? 1.03 : 1.0;
@@ -136,18 +139,20 @@ bool pencil_shape(ZParams& zp, int* threads) {
   zp.PS = tile_ps(W, zp.nth, SB);
   zp.swz = zp.NP == 4 && zp.nzp % 4 == 0;
   const int items = zp.nzp * zp.NP;
-  // The Cholesky forms on a block whose tiles are all resident at once: a tile's time is its rounds of
-  // bins, each as long as a factorisation, so the threads of an SM go to the r tiles that it gets where that
-  // saves a round (48x50x72, 6 angles, 350 tiles of 288 bins: 160 threads instead of 128, the pass 37 -> 33 us, with
-  // FP64 96 -> 70).  Tiles that are not all resident keep their neighbours' company: 400 tiles of 512 threads
-  // instead of 128 took 76 us instead of 62.
+  // A block whose tiles are all resident at once: a tile's time is its rounds of pairs (of bins in the Cholesky
+  // forms, each as long as a factorisation) and of transform items, so the threads of an SM go to the r tiles that it
+  // gets where that saves a round (24x36x42, 8 realisations, 144 tiles: the job 60.6 us at 96 threads, 46.5 at 192;
+  // 24x24x128: 62.9 at 256, 53.8 at 384; 48x50x72, 6 angles, FP64, 350 tiles of 288 bins: the pass 96 -> 70 us at 160
+  // instead of 128).  Not so many that some tiles wait (48x48x48, 336 tiles: 80.3 at 128, 103.6 at 192).
   const long long tiles = (long long)zp.nIT * zp.nyp;
   const int fit = std::min(4, tiles_per_sm(pencil_smem_bytes(W, zp.nzp, zp.nth, SB)));
-  if (!zp.eig && tiles <= 148LL * fit) {
+  if (tiles <= 148LL * fit) {
+    const int lines = std::max(3 * SB, std::max(zp.nth + 3, 8)) * zp.NP;
+    const int work = std::max(zp.nzp * W / per, lines * (zp.nzp / zp.z.radix[zp.z.ns - 1]));
     int least = 1 << 30;
     for (int r = fit; r >= (int)((tiles + 147) / 148); r--) {
-      const int t = std::max(64, std::min(512 / r / 32 * 32, (zp.nzp * W + 31) / 32 * 32));
-      const int rounds = (zp.nzp * W + t - 1) / t;
+      const int t = std::max(64, std::min(512 / r / 32 * 32, (work + 31) / 32 * 32));
+      const int rounds = (work + t - 1) / t;
       if (rounds < least) {
         least = rounds;
         T = t;

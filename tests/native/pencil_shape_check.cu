@@ -1,16 +1,29 @@
 // Runs pencil_shape of the built library over every z length, angle count and realisation count that a
 // job may have, on narrow and wide blocks, and checks what launch_pencil and the kernel ask of a shape.
-// No device is used.  Arguments: the schedule's threads per CTA (0: none).  Prints "<shapes> <bad>".
+// No device is used.  Prints "<shapes> <bad>"; with arguments nxp nyp nzp nth nsim eig, the shape of that job:
+// "<W> <SB> <T> <tiles>".
 #include <cstdio>
 #include <cstdlib>
 
 #include "kernels.cuh"
 
-extern "C" int crava_tuning_set(const char* key, int n, int value);
-
 int main(int argc, char** argv) {
   using namespace crava;
-  const int want = argc > 1 ? std::atoi(argv[1]) : 0;
+  if (argc > 6) {
+    ZParams zp = {};
+    zp.nxp = std::atoi(argv[1]);
+    zp.cnxp = zp.nxp / 2 + 1;
+    zp.nyp = std::atoi(argv[2]);
+    zp.nzp = std::atoi(argv[3]);
+    zp.nth = std::atoi(argv[4]);
+    zp.nsim = std::atoi(argv[5]);
+    alignas(16) static float4 table;
+    zp.eig = std::atoi(argv[6]) ? &table : nullptr;
+    int T = 0;
+    if (!pencil_shape(zp, &T)) return 1;
+    std::printf("%d %d %d %d\n", zp.W, zp.SB, T, zp.nIT * zp.nyp);
+    return 0;
+  }
   long shapes = 0, bad = 0;
   for (int nzp = 2; nzp <= 1024; nzp++) {
     int m = nzp;
@@ -18,7 +31,6 @@ int main(int argc, char** argv) {
       while (m % p == 0) m /= p;
     if (m != 1) continue;
     for (int nth = 1; nth <= kMaxTheta; nth++) {
-      if (want) crava_tuning_set("pencil_threads", nzp * 16 + nth, want);
       for (int nsim = 0; nsim <= kMaxSim; nsim++)
         for (int side : {2, 31, 540, 4096}) {
           ZParams zp = {};
