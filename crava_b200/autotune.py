@@ -13,11 +13,11 @@ fastest value.  The keys swept, with their size key n:
   line4_w_fwd, line4_w_inv   n = N     four-step column transforms: columns per tile
   line4_threads_fwd, line4_threads_inv  four-step column transforms: threads per CTA (n = N;
                                         at most 256 forward, 512 inverse)
-  x4_stage_fwd, x4_stage_inv           four-step row transforms: 1 = twiddle tables staged in
-                                        shared memory, 0 = read from global memory (n = nxp/2)
+  x4_stage_fwd   n = nxp/2             forward row transforms: 1 = twiddle tables staged in
+                                        shared memory, 0 = read from global memory
   x4_threads_fwd, x4_threads_inv       four-step row transforms: threads per CTA
                  n = nxp/2
-  x4_rpc_fwd, x4_rpc_inv  n = nxp/2    rows per CTA (defaults threads / (N1/2 + 1), threads / N1)
+  x4_rpc_fwd, x4_rpc_inv  n = nxp/2    rows per CTA (defaults from the passes' items)
   line4_pf_fwd, line4_pf_inv (n = N),  L2 prefetch of the tiles (rows) that many quarters of
   x4_pf_fwd, x4_pf_inv (n = nxp/2)     the resident CTAs ahead; 0 = off
 
@@ -114,6 +114,8 @@ def tune_workload(name, w, reps, entries, log):
     log.append(f"# workload {name}: {nxp}x{nyp}x{nzp}, {nth} angles, {job.nsim} realisations")
     # pencil pass: the realisation batch and threads of every tile width; an entry is kept only
     # where it beats the built-in shape (pencil_shape in pencil.cu), which also weighs the lateral size
+    for key in ("pencil_w", "pencil_sb", "pencil_threads"):
+        api.tuning_set(key, pk, -1)
     base = time_classes(ctx, job, stream, reps).get("zpass", 0.0)
     best = (base, {})
     for w in (8, 4, 2):
@@ -128,34 +130,39 @@ def tune_workload(name, w, reps, entries, log):
         if best[1]:
             entries[(key, pk)] = best[1][key]
     log.append(f"# pencil shape {pk}: built-in {base:.3f} ms, best {best[0]:.3f} ms")
-    # four-step column (y) and row (x) transforms
+    # four-step column (y) and row (x) transforms; columns of up to 270 points go in pairs, in tiles of at
+    # most 16 by at most 256 threads and without a prefetch (line4 in fft4.cuh)
+    pairs = nyp <= 270
     for key, tkey, cls in (("line4_w_fwd", "line4_threads_fwd", ["line_fwd"]),
                            ("line4_w_inv", "line4_threads_inv", ["line_inv"])):
-        b = sweep(ctx, job, stream, reps, key, nyp, [4, 8, 16, 32], cls, log)
+        b = sweep(ctx, job, stream, reps, key, nyp, [4, 8, 16] if pairs else [4, 8, 16, 32], cls, log)
         if b:
             entries[(key, nyp)] = b[0]
-        tv = [128, 160, 192, 224, 256] + ([320, 384, 448, 512] if tkey.endswith("inv") else [])
+        tv = [128, 160, 192, 224, 256] + ([320, 384, 448, 512] if tkey.endswith("inv") and not pairs else [])
         b = sweep(ctx, job, stream, reps, tkey, nyp, tv, cls, log)
         if b:
             entries[(tkey, nyp)] = b[0]
+        if pairs:
+            continue
         pkey = "line4_pf_fwd" if tkey.endswith("fwd") else "line4_pf_inv"
         b = sweep(ctx, job, stream, reps, pkey, nyp, [0, 2, 4], cls, log)
         if b:
             entries[(pkey, nyp)] = b[0]
     if nxp % 2 == 0:
         h = nxp // 2
-        for key, skey, cls in (("x4_threads_fwd", "x4_stage_fwd", ["x_r2c"]),
-                               ("x4_threads_inv", "x4_stage_inv", ["x_c2r"])):
+        for key, skey, cls in (("x4_threads_fwd", "x4_stage_fwd", ["x_r2c"]), ("x4_threads_inv", None, ["x_c2r"])):
             best = None
-            for stage in (1, 0):
-                api.tuning_set(skey, h, stage)
+            for stage in (1, 0) if skey else (1,):
+                if skey:
+                    api.tuning_set(skey, h, stage)
                 b = sweep(ctx, job, stream, reps, key, h, [64, 96, 128, 160, 192, 256], cls, log)
                 if b and (best is None or b[1] < best[2]):
                     best = (stage, b[0], b[1])
             if best:
-                api.tuning_set(skey, h, best[0])
+                if skey:
+                    api.tuning_set(skey, h, best[0])
+                    entries[(skey, h)] = best[0]
                 api.tuning_set(key, h, best[1])
-                entries[(skey, h)] = best[0]
                 entries[(key, h)] = best[1]
             rkey = key.replace("threads", "rpc")   # rows per CTA
             b = sweep(ctx, job, stream, reps, rkey, h, [2, 4, 6, 8, 12], cls, log)
@@ -196,9 +203,8 @@ def main():
         f.write("# key n value   (n: see crava_b200/autotune.py; -1 = every size)\n")
         for (k, n), v in sorted(entries.items()):
             f.write(f"{k} {n} {v}\n")
-        f.write("# sweep log (device ms of the kernel class the key controls, per run)\n")
-        for l in log:
-            f.write(l + "\n")
+    for l in log:      # device ms of the kernel class the key controls, per run
+        print(l)
     print(f"wrote {args.out}: {len(entries)} entries")
 
 

@@ -147,6 +147,7 @@ int tuned(const char* key, int n, int fallback) {
 }  // namespace crava
 
 // Per-kernel-class CUDA-event timing (off unless crava_ctx_set_profiling enables it).
+// The class numbers are part of crava_ctx_kernel_times: 5 and 6 are kept, though no kernel is of those classes.
 enum { KT_X_R2C = 0, KT_LINE_FWD = 1, KT_ZPASS = 2, KT_LINE_INV = 3, KT_X_C2R = 4, KT_XY_FWD = 5, KT_XY_INV = 6,
        KT_THICK_DIVIDE = 7, KT_THICK_FILL = 8, KT_LOCAL_NOISE = 9, KT_FACIES = 10, KT_FILL_PRIOR = 11,
        KT_COUNT = 12 };

@@ -495,7 +495,6 @@ inline cudaError_t launch_zpass_t(const ZParams& zp, int threads, cudaStream_t s
 
 // the general kernel's launchers by angle count (zpass_n12.cu, zpass_n34.cu, zpass_n56.cu,
 // zpass_n78.cu): one translation unit per pair so that they compile side by side
-cudaError_t launch_zpass_nth(const ZParams& zp, int threads, cudaStream_t st);
 cudaError_t launch_zpass_n12(const ZParams& zp, int threads, cudaStream_t st);
 cudaError_t launch_zpass_n34(const ZParams& zp, int threads, cudaStream_t st);
 cudaError_t launch_zpass_n56(const ZParams& zp, int threads, cudaStream_t st);
