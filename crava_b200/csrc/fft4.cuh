@@ -569,6 +569,8 @@ __global__ void __launch_bounds__(256) k_xc2r4(const __grid_constant__ GridSet g
 //            Z[N-k] for all its k (as xr2c4_rows)
 //   inverse  Z[k] = A[k] + i B[k] (k <= N/2), Z[N-k] = conj A[k] + i conj B[k], formed where pass 1
 //            loads it; Im A[0] and Im B[0] have no slot in a real-output transform
+// A row so carries the rounding of the larger of its pair: a zero row beside a large one comes back as some 1e-7 of
+// that one, as the y and z transforms leave every line within 1e-7 of its largest point.
 // Rows in global and staged memory have N + 1 floats; the last is written as zero.
 template <int N1, int N2>
 __global__ void __launch_bounds__(256) k_xr2c4o(const __grid_constant__ GridSet gs, int rows, int lpc,

@@ -36,7 +36,8 @@
 //
 // The diagonal of S_post is real: the pair's second bin goes into the imaginary part of the first
 // one's line, which halves its share of the inverse transform (9 output spectra cost 7.5 lines) and
-// of the tile; the two are told apart after the transform by S(z) = conj S(-z).
+// of the tile; the two are told apart after the transform by S(z) = conj S(-z), each with the rounding of the
+// larger (1e-7 of it: what the x transform that follows makes of a line's points in any case).
 //
 // What bounds it: the latency of packed chains, shared memory and barriers at 16 warps an SM (128
 // registers, the tile in most of the shared memory), not HBM.  Against the scalar kernels with one
