@@ -242,14 +242,17 @@ cudaError_t scratch_alloc(crava_ctx* ctx, void** p, size_t bytes, cudaStream_t s
       pr.allocType = cudaMemAllocationTypePinned;
       pr.location.type = cudaMemLocationTypeDevice;
       pr.location.id = ctx->device;
+      // a capture in its global mode refuses the creation, which touches no stream
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      cudaThreadExchangeStreamCaptureMode(&mode);
       cudaError_t e = cudaMemPoolCreate(&pool, &pr);
-      if (e != cudaSuccess) return e;
       uint64_t keep = kScratchKeep;
-      e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-      if (e != cudaSuccess) {
-        cudaMemPoolDestroy(pool);
-        return e;
+      if (e == cudaSuccess) {
+        e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        if (e != cudaSuccess) cudaMemPoolDestroy(pool);
       }
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      if (e != cudaSuccess) return e;
       ctx->scratch = pool;
     }
     pool = ctx->scratch;
