@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(256, col_split(N).r0 <= 10 ? 4 : col_split(N).
   }
 }
 
-// The scalar two-pass form of the longer lengths (line4 below says which), one column an item.
+// The scalar two-pass form of the other lengths (col_pairs below says which), one column an item.
 //
 // One tile of W columns (nw of them valid) of the lines through g: point p of column w at
 // g[p pstride + w], read from src[p spstride + w] (g itself, or a staged copy of the tile in
@@ -706,13 +706,13 @@ static inline bool four_step_enabled(int n) { return tuned("four_step", n, 1) !=
 
 static inline int round_up32(int t) { return std::max(64, (t + 31) / 32 * 32); }
 
-template <int N1, int N2>
+template <int N1, int N2, int DIR>
 static cudaError_t line4_scalar(const GridSet& gs, int ni, size_t pstride, int no, size_t ostride, const float2* tw,
-                         float sign, cudaStream_t st) {
+                         cudaStream_t st) {
   constexpr int N = N1 * N2;
   // 8-column tiles; 16 for inverse transforms up to 540 points (measured faster there,
   // slower at 768)
-  int W = std::max(1, tuned(sign < 0.f ? "line4_w_fwd" : "line4_w_inv", N, (sign > 0.f && N <= 540) ? 16 : 8));
+  int W = std::max(1, tuned(DIR < 0 ? "line4_w_fwd" : "line4_w_inv", N, (DIR > 0 && N <= 540) ? 16 : 8));
   while (W > 1 && W / 2 >= ni) W /= 2;
   int lw = 0;
   while ((1 << lw) < W) lw++;
@@ -722,33 +722,32 @@ static cudaError_t line4_scalar(const GridSet& gs, int ni, size_t pstride, int n
   // schedule may set up to 512 (a whole number of warps), e.g. so that one pass runs in a
   // single round
   int T = std::min(256, round_up32(W * std::max(N1, N2)));
-  T = std::max(64, std::min(sign < 0.f ? 256 : 512,
-                            tuned(sign < 0.f ? "line4_threads_fwd" : "line4_threads_inv", N, T) / 32 * 32));
+  T = std::max(64, std::min(DIR < 0 ? 256 : 512,
+                            tuned(DIR < 0 ? "line4_threads_fwd" : "line4_threads_inv", N, T) / 32 * 32));
   const int nIT = (ni + W - 1) / W;
   const size_t smem = sizeof(float2) * (size_t)N + line4_smem<N1, N2>(W, SK);
-  const void* fn = sign < 0.f ? (const void*)k_line4s<N1, N2, -1> : (const void*)k_line4s<N1, N2, 1>;
+  const auto fn = k_line4s<N1, N2, DIR>;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   dim3 grid((unsigned)(nIT * no), gs.n);
   // L2 line prefetch ahead of the tiles: schedule keys line4_pf_fwd / line4_pf_inv, the distance in
   // quarters of the resident tiles (0 = off)
   int pf = 0;
-  if (const int q = tuned(sign < 0.f ? "line4_pf_fwd" : "line4_pf_inv", N, 0)) {
+  if (const int q = tuned(DIR < 0 ? "line4_pf_fwd" : "line4_pf_inv", N, 0)) {
     int res = 0;
-    if ((e = resident_grid(fn, T, smem, 1 << 30, &res)) != cudaSuccess) return e;
+    if ((e = resident_grid((const void*)fn, T, smem, 1 << 30, &res)) != cudaSuccess) return e;
     pf = std::max(1, res * q / 4);
   }
   const size_t bytes = sizeof(float2) * (size_t)gs.n * ni * N * no;
-  return sign < 0.f ? launch_dep(bytes, k_line4s<N1, N2, -1>, grid, T, smem, st, gs, ni, pstride, ostride, W, lw, nIT, SK, tw, pf)
-                    : launch_dep(bytes, k_line4s<N1, N2, 1>, grid, T, smem, st, gs, ni, pstride, ostride, W, lw, nIT, SK, tw, pf);
+  return launch_dep(bytes, fn, grid, T, smem, st, gs, ni, pstride, ostride, W, lw, nIT, SK, tw, pf);
 }
 
-template <int N>
+template <int N, int DIR>
 static cudaError_t line4_pairs(const GridSet& gs, int ni, size_t pstride, int no, size_t ostride, const float2* tw,
-                               float sign, cudaStream_t st) {
+                               cudaStream_t st) {
   constexpr ColSplit S = col_split(N);
   // 16-column tiles (rows of 128 bytes); narrower where the grid is
-  int W = std::max(2, std::min(16, tuned(sign < 0.f ? "line4_w_fwd" : "line4_w_inv", N, 16)));
+  int W = std::max(2, std::min(16, tuned(DIR < 0 ? "line4_w_fwd" : "line4_w_inv", N, 16)));
   while (W > 2 && W / 2 >= ni) W /= 2;
   int lnp = 0;
   while ((4 << lnp) <= W) lnp++;
@@ -757,28 +756,36 @@ static cudaError_t line4_pairs(const GridSet& gs, int ni, size_t pstride, int no
   // threads: the items of the first stage in as few rounds of at most 256 threads as they take
   const int items = (W / 2) * (N / S.r0), rounds = (items + 255) / 256;
   int T = round_up32((items + rounds - 1) / rounds);
-  T = std::max(64, std::min(256, tuned(sign < 0.f ? "line4_threads_fwd" : "line4_threads_inv", N, T) / 32 * 32));
+  T = std::max(64, std::min(256, tuned(DIR < 0 ? "line4_threads_fwd" : "line4_threads_inv", N, T) / 32 * 32));
   const int nIT = (ni + W - 1) / W;
-  const void* fn = sign < 0.f ? (const void*)k_line4<N, -1> : (const void*)k_line4<N, 1>;
+  const auto fn = k_line4<N, DIR>;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   dim3 grid((unsigned)(nIT * no), gs.n);
   const size_t bytes = sizeof(float2) * (size_t)gs.n * ni * N * no;
-  return sign < 0.f ? launch_dep(bytes, k_line4<N, -1>, grid, T, smem, st, gs, ni, pstride, ostride, lnp, nIT, tw)
-                    : launch_dep(bytes, k_line4<N, 1>, grid, T, smem, st, gs, ni, pstride, ostride, lnp, nIT, tw);
+  return launch_dep(bytes, fn, grid, T, smem, st, gs, ni, pstride, ostride, lnp, nIT, tw);
 }
 
-// Pairs up to 270 points: with 250 x-points, 21 grids of 60 planes, 5 % faster or equal at lengths of two
-// factors up to 16, 1.3 to 1.9 times at the lopsided ones (125 = 25 x 5, 250 = 25 x 10) that then
-// take three stages; above, three stages cost more than the scalar form's two (288 to 1024 points:
-// 0.65 to 1.05 of its speed).
+// Which columns go in pairs; time of the scalar form over the pairs', 21 grids of 60 planes of 250 x-points:
+//   scalar split with a factor above 20   forward 1.34-1.92, inverse 1.33-1.76 (125, 147, 175, 189, 243, 250 points),
+//                                         at most 270 points: above, three stages cost more than two wide ones
+//   else forward, to 240 points           1.00-1.11 (252 = 18 x 14 against 7 x 6 x 6: 0.78; 256 0.99, 270 1.00, 280 0.93)
+//   else inverse, to 180 points           1.00-1.23 (192 0.98, 196 0.94, 216 0.93, 240 0.97, 252 0.69, 256 0.96)
+constexpr bool col_pairs(int n1, int n, int dir) { return n1 > 20 ? n <= 270 : n <= (dir < 0 ? 240 : 180); }
+
+// Residual spectra keep the scalar form's order of roundings in their forward transforms (GridSet.plain).
 template <int N1, int N2>
 static cudaError_t line4(const GridSet& gs, int ni, size_t pstride, int no, size_t ostride, const float2* tw,
                          float sign, cudaStream_t st) {
-  if constexpr (N1 * N2 <= 270) {
-    if (!gs.plain || sign > 0.f) return line4_pairs<N1 * N2>(gs, ni, pstride, no, ostride, tw, sign, st);
+  constexpr int N = N1 * N2;
+  if (sign > 0.f) {
+    if constexpr (col_pairs(N1, N, 1)) return line4_pairs<N, 1>(gs, ni, pstride, no, ostride, tw, st);
+    else return line4_scalar<N1, N2, 1>(gs, ni, pstride, no, ostride, tw, st);
   }
-  return line4_scalar<N1, N2>(gs, ni, pstride, no, ostride, tw, sign, st);
+  if constexpr (col_pairs(N1, N, -1)) {
+    if (!gs.plain) return line4_pairs<N, -1>(gs, ni, pstride, no, ostride, tw, st);
+  }
+  return line4_scalar<N1, N2, -1>(gs, ni, pstride, no, ostride, tw, st);
 }
 
 // Threads and lines per CTA of a row kernel whose passes have i1 and i2 items per line of c1 and
