@@ -14,7 +14,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libcrava_gpu.so")
-SOURCES = ["crava_api.cu", "kernels.cu", "fft4.cu", "fft4_p1.cu", "fft4_p2.cu", "fft4_p3.cu", "fft4_p4.cu", "fft4_p5.cu", "fft4_p6.cu", "zpass.cu", "zpass_n12.cu", "zpass_n34.cu", "zpass_n56.cu", "zpass_n78.cu", "pencil.cu", "pencil_n12.cu", "pencil_n34.cu", "pencil_n56.cu", "pencil_n78.cu", "localnoise.cu", "gridio.cu", "facies.cu", "thick.cu", "prior.cu", "segy.cu"]
+SOURCES = ["crava_api.cu", "kernels.cu", "fft4.cu", "fft4_p1.cu", "fft4_p2.cu", "fft4_p3.cu", "fft4_p4.cu", "fft4_p5.cu", "fft4_p6.cu", "zpass.cu", "zpass_n12.cu", "zpass_n34.cu", "zpass_n56.cu", "zpass_n78.cu", "pencil.cu", "pencil_n12.cu", "pencil_n34.cu", "pencil_n56.cu", "pencil_n78.cu", "pencil_c12.cu", "pencil_c34.cu", "pencil_c56.cu", "pencil_c78.cu", "localnoise.cu", "gridio.cu", "facies.cu", "thick.cu", "prior.cu", "segy.cu"]
 HEADERS = ["fft_core.cuh", "fft2.cuh", "fft4.cuh", "kernels.cuh", "fft_pair.cuh", "pencil_common.cuh", "pencil_bin.cuh", "pencil.cuh", "zpass.cuh", "facies.cuh", "fft4_facies.cuh", "ibm_float.h"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]

@@ -1,5 +1,5 @@
 // Plan, tile shape and launch of the pencil pass (kernel in pencil.cuh, instantiated by angle
-// count in pencil_n12.cu, pencil_n34.cu, pencil_n56.cu and pencil_n78.cu).
+// count in pencil_n*.cu and pencil_c*.cu).
 #include "pencil.cuh"
 
 #include <algorithm>
@@ -172,11 +172,12 @@ cudaError_t launch_pencil(const ZParams& zp, int threads, cudaStream_t st, int* 
       (zp.keep_resid && !z_inlined(zp.nzp)))
     return cudaErrorInvalidValue;
   if (nlaunch) (*nlaunch)++;
+  const bool chol = zp.fp64_threshold > 0.f || !zp.eig;
   switch (zp.nth) {
-    case 1: case 2: return launch_pencil_n12(zp, threads, st);
-    case 3: case 4: return launch_pencil_n34(zp, threads, st);
-    case 5: case 6: return launch_pencil_n56(zp, threads, st);
-    case 7: case 8: return launch_pencil_n78(zp, threads, st);
+    case 1: case 2: return chol ? launch_pencil_c12(zp, threads, st) : launch_pencil_n12(zp, threads, st);
+    case 3: case 4: return chol ? launch_pencil_c34(zp, threads, st) : launch_pencil_n34(zp, threads, st);
+    case 5: case 6: return chol ? launch_pencil_c56(zp, threads, st) : launch_pencil_n56(zp, threads, st);
+    case 7: case 8: return chol ? launch_pencil_c78(zp, threads, st) : launch_pencil_n78(zp, threads, st);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -942,18 +942,23 @@ inline cudaError_t launch_pencil_z(const ZParams& zp, int threads, cudaStream_t 
     default: return launch_pencil_t<NTH, MODE, 0, 0>(zp, threads, st);
   }
 }
+// FP64 re-factorisation or none
 template <int NTH>
-inline cudaError_t launch_pencil_m(const ZParams& zp, int threads, cudaStream_t st) {
-  if (zp.fp64_threshold > 0.f) return launch_pencil_z<NTH, kCholFp64>(zp, threads, st);
-  if (!zp.eig) return launch_pencil_z<NTH, kChol>(zp, threads, st);
-  return launch_pencil_z<NTH, kEig>(zp, threads, st);
+inline cudaError_t launch_pencil_chol(const ZParams& zp, int threads, cudaStream_t st) {
+  return zp.fp64_threshold > 0.f ? launch_pencil_z<NTH, kCholFp64>(zp, threads, st)
+                                 : launch_pencil_z<NTH, kChol>(zp, threads, st);
 }
 
-// launchers by angle count (pencil_n12.cu, pencil_n34.cu, pencil_n56.cu, pencil_n78.cu): one
-// translation unit per pair so that they compile side by side
+// launchers by angle count: the eigen form in pencil_n12.cu .. pencil_n78.cu, the Cholesky forms in
+// pencil_c12.cu .. pencil_c78.cu.  The units compile side by side, and a process loads the whole of one at its first
+// launch: with the forms in one unit, a process's first job took 31 ms at 540x540x256 and 28 at 250x250x200, apart 21 and 15.
 cudaError_t launch_pencil_n12(const ZParams& zp, int threads, cudaStream_t st);
 cudaError_t launch_pencil_n34(const ZParams& zp, int threads, cudaStream_t st);
 cudaError_t launch_pencil_n56(const ZParams& zp, int threads, cudaStream_t st);
 cudaError_t launch_pencil_n78(const ZParams& zp, int threads, cudaStream_t st);
+cudaError_t launch_pencil_c12(const ZParams& zp, int threads, cudaStream_t st);
+cudaError_t launch_pencil_c34(const ZParams& zp, int threads, cudaStream_t st);
+cudaError_t launch_pencil_c56(const ZParams& zp, int threads, cudaStream_t st);
+cudaError_t launch_pencil_c78(const ZParams& zp, int threads, cudaStream_t st);
 
 }  // namespace crava
