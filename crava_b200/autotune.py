@@ -130,7 +130,7 @@ def tune_workload(name, w, reps, entries, log):
         if best[1]:
             entries[(key, pk)] = best[1][key]
     log.append(f"# pencil shape {pk}: built-in {base:.3f} ms, best {best[0]:.3f} ms")
-    # four-step column (y) and row (x) transforms; columns of up to 270 points may go in pairs (col_pairs in
+    # four-step column (y) and row (x) transforms; columns of up to 270 points may go in pairs (line4 in
     # fft4.cuh), in tiles of at most 16 by at most 256 threads and without a prefetch
     pairs = nyp <= 270
     for key, tkey, cls in (("line4_w_fwd", "line4_threads_fwd", ["line_fwd"]),

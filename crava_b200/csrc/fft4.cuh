@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(256, col_split(N).r0 <= 10 ? 4 : col_split(N).
   }
 }
 
-// The scalar two-pass form of the other lengths (col_pairs below says which), one column an item.
+// The scalar two-pass form of the other lengths (line4 below says which), one column an item.
 //
 // One tile of W columns (nw of them valid) of the lines through g: point p of column w at
 // g[p pstride + w], read from src[p spstride + w] (g itself, or a staged copy of the tile in
@@ -756,6 +756,11 @@ static cudaError_t line4_pairs(const GridSet& gs, int ni, size_t pstride, int no
   // threads: the items of the first stage in as few rounds of at most 256 threads as they take
   const int items = (W / 2) * (N / S.r0), rounds = (items + 255) / 256;
   int T = round_up32((items + rounds - 1) / rounds);
+  // one warp more where it saves both other stages a round (252 = 7 x 6 x 6: 160 threads 176 us, 192 135, inverse, 21 grids)
+  if constexpr (S.r2 > 1) {
+    const int i1 = (W / 2) * (N / S.r1), i2 = (W / 2) * (N / S.r2), up = T + 32;
+    if (up <= 256 && (i1 - 1) / up < (i1 - 1) / T && (i2 - 1) / up < (i2 - 1) / T) T = up;
+  }
   T = std::max(64, std::min(256, tuned(DIR < 0 ? "line4_threads_fwd" : "line4_threads_inv", N, T) / 32 * 32));
   const int nIT = (ni + W - 1) / W;
   const auto fn = k_line4<N, DIR>;
@@ -766,26 +771,24 @@ static cudaError_t line4_pairs(const GridSet& gs, int ni, size_t pstride, int no
   return launch_dep(bytes, fn, grid, T, smem, st, gs, ni, pstride, ostride, lnp, nIT, tw);
 }
 
-// Which columns go in pairs; time of the scalar form over the pairs', 21 grids of 60 planes of 250 x-points:
-//   scalar split with a factor above 20   forward 1.34-1.92, inverse 1.33-1.76 (125, 147, 175, 189, 243, 250 points),
-//                                         at most 270 points: above, three stages cost more than two wide ones
-//   else forward, to 240 points           1.00-1.11 (252 = 18 x 14 against 7 x 6 x 6: 0.78; 256 0.99, 270 1.00, 280 0.93)
-//   else inverse, to 180 points           1.00-1.23 (192 0.98, 196 0.94, 216 0.93, 240 0.97, 252 0.69, 256 0.96)
-constexpr bool col_pairs(int n1, int n, int dir) { return n1 > 20 ? n <= 270 : n <= (dir < 0 ? 240 : 180); }
-
-// Residual spectra keep the scalar form's order of roundings in their forward transforms (GridSet.plain).
+// Which columns of up to 270 points go in pairs (above, three stages cost more than the scalar form's two); time of the
+// scalar form over the pairs', y columns of jobs with 21 grids of 250 x-points, and z lines of one 540x540 plane set:
+//   scalar split with a factor above 20   1.33-1.92 (125, 147, 175, 189, 243, 250 points), z lines 1.12-1.54
+//   up to 180 points                      1.00-1.23, z lines 0.99-1.09
+//   above, forward                        1.00-1.13 (252 points 0.96), z lines 0.99-1.16
+//   above, inverse                        0.91-1.03, z lines 0.96-1.01, but 1.04-1.13 with 64 x-points: there the
+//                                         scalar form, its tiles too few to hide its longer rounds, is the slower
 template <int N1, int N2>
 static cudaError_t line4(const GridSet& gs, int ni, size_t pstride, int no, size_t ostride, const float2* tw,
                          float sign, cudaStream_t st) {
   constexpr int N = N1 * N2;
-  if (sign > 0.f) {
-    if constexpr (col_pairs(N1, N, 1)) return line4_pairs<N, 1>(gs, ni, pstride, no, ostride, tw, st);
-    else return line4_scalar<N1, N2, 1>(gs, ni, pstride, no, ostride, tw, st);
+  if constexpr (N <= 270) {
+    if (sign > 0.f && (N1 > 20 || N <= 180 || ni <= 64)) return line4_pairs<N, 1>(gs, ni, pstride, no, ostride, tw, st);
+    // residual spectra keep the scalar form's order of roundings in their forward transforms
+    if (sign < 0.f && !gs.plain) return line4_pairs<N, -1>(gs, ni, pstride, no, ostride, tw, st);
   }
-  if constexpr (col_pairs(N1, N, -1)) {
-    if (!gs.plain) return line4_pairs<N, -1>(gs, ni, pstride, no, ostride, tw, st);
-  }
-  return line4_scalar<N1, N2, -1>(gs, ni, pstride, no, ostride, tw, st);
+  return sign < 0.f ? line4_scalar<N1, N2, -1>(gs, ni, pstride, no, ostride, tw, st)
+                    : line4_scalar<N1, N2, 1>(gs, ni, pstride, no, ostride, tw, st);
 }
 
 // Threads and lines per CTA of a row kernel whose passes have i1 and i2 items per line of c1 and
