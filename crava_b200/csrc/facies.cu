@@ -18,6 +18,7 @@
 
 namespace crava {
 
+template <bool PAIRS>
 __global__ void k_facies_prob_corners(const float* __restrict__ vp, const float* __restrict__ vs,
                                       const float* __restrict__ rho, int nx, int ny, int nz, int rnxp_in, int nyp_in,
                                       int rnxp_out, const __grid_constant__ FaciesCorners C, int nf, FaciesPrior pr,
@@ -36,7 +37,7 @@ __global__ void k_facies_prob_corners(const float* __restrict__ vp, const float*
       }
       const float v[3] = {vp[g0 + i], vs[g0 + i], rho[g0 + i]};
       float val[kMaxFacies];
-      const float sum = facies_voxel(v, i, j, nx, ny, C, nf, pr, undef_sum, val);
+      const float sum = facies_voxel<PAIRS>(v, i, j, nx, ny, C, nf, pr, undef_sum, val);
       for (int f = 0; f < nf; f++) out.p[f][e] = val[f] / sum;
       out.p[nf][e] = undef_sum / sum;
       if (seis_lh) seis_lh[e] = sum;
@@ -46,7 +47,7 @@ __global__ void k_facies_prob_corners(const float* __restrict__ vp, const float*
 
 // The same for one volume (no local noise) of at most four facies, the usual case, with everything in
 // registers: the general form keeps its facies in local memory and spends 562 instructions a voxel.
-// 270x270x256, 3 facies, 100x100x50 bins, with the packing: 0.66 -> 0.33 ms.
+// 270x270x256, 3 facies, 100x100x50 bins, with the packing: 0.66 -> 0.37 ms.
 struct FaciesSingle {
   const float4* dens;
   int nb[3];
@@ -318,8 +319,8 @@ cudaError_t launch_facies_eval(const float* vp, const float* vs, const float* rh
         vp, vs, rho, nx, ny, nz, rnxp_in, nyp_in, rnxp_out, F, nf, pr, undef_sum, po, seis_lh);
     return cudaGetLastError();
   }
-  k_facies_prob_corners<<<blocks, dim3(32, 8), 0, st>>>(vp, vs, rho, nx, ny, nz, rnxp_in, nyp_in, rnxp_out, C, nf, pr,
-                                                        undef_sum, po, seis_lh);
+  (hc.pairs ? k_facies_prob_corners<true> : k_facies_prob_corners<false>)<<<blocks, dim3(32, 8), 0, st>>>(
+      vp, vs, rho, nx, ny, nz, rnxp_in, nyp_in, rnxp_out, C, nf, pr, undef_sum, po, seis_lh);
   return cudaGetLastError();
 }
 
@@ -357,11 +358,11 @@ size_t facies_packed_bytes(const FaciesBoxHost& b, int nf, bool pairs) {
   return (pairs ? 2 : 1) * sizeof(float4) * (size_t)b.nb[0] * b.nb[1] * b.nb[2] * ((nf + 3) / 4);
 }
 
-// 128 MB: the L2 holds 126.  4 volumes of 128 MB in all are faster in pairs, 16 of 256 MB are not (facies.cuh).
+// Above 8 MB, where scattered cells are fetched from the L2, and up to the 128 MB that it holds (facies.cuh has both sides).
 bool facies_pairs(const FaciesCornersHost& hc, int nf) {
   size_t bytes = 0;
   for (int c = 0; c < (1 << hc.nang); c++) bytes += facies_packed_bytes(hc.box[c], nf, true);
-  return bytes <= 128u << 20;
+  return bytes > 8u << 20 && bytes <= 128u << 20;
 }
 
 cudaError_t launch_spec_mul(float2* a, const float2* b, size_t n, cudaStream_t st) {

@@ -58,14 +58,17 @@ __device__ __forceinline__ void ldg_pair(const float4* p, float4& a, float4& b) 
 // clamped densities of (j, k, l) in 16 bytes or, packed in pairs, those of (j, k, l) and (j + 1, k, l) in
 // 32, so that a voxel makes four 32-byte loads per volume and group instead of eight, and computes the cell indexes
 // once per volume.  The lookups are bound by the L1's one line a clock for scattered lanes where the
-// volumes sit in the L2 (facies_pairs; with the packing, volumes of 100x100x50, eight against four loads: 270x270x256, one
-// volume, 3 facies 647 -> 428 us, 6 facies 1495 -> 1067; 200x200x100, 4 volumes, 6 facies, 128 MB in pairs 1568 -> 1270),
-// and by the bytes beyond it (16 volumes, 3 facies, 256 MB in pairs 3512 -> 3640, 6 facies 5843 -> 8856).  The
-// float operations per facies are the reference's, in its order.
+// volumes sit in the L2, by the bytes beyond it, and by the L1's hits below it, which pairs halve (facies_pairs; us with
+// the packing, eight against four loads, a smooth mean and one of white noise):
+//   270x270x256, 3 facies   64x64x32 bins 332 / 332, 362 / 373   100x100x50 369 / 359, 510 / 396
+//                9 facies   20x20x10 bins 874 / 970, 1049 / 1040   64x64x32 1149 / 1185, 1627 / 1388   100x100x50 1377 / 1350, 1927 / 1423
+//   200x200x100, 16 volumes of 100x100x50 bins, 256 MB in pairs, 3 facies 3512 / 3640, 6 facies 5843 / 8856
+// The float operations per facies are the reference's, in its order.
 //
 // facies_voxel: the densities of voxel (i, j) of trace row j at the parameters v, prior-
 // weighted: val[f] = prior_f max(0, dens_f) and the returned sum = undef_sum + sum_f val[f]
 // (the voxel's probabilities are val[f] / sum and undef_sum / sum).
+template <bool PAIRS>
 __device__ __forceinline__ float facies_voxel(const float (&v)[3], int i, int j, int nx, int ny,
                                               const FaciesCorners& C, int nf, const FaciesPrior& pr,
                                               float undef_sum, float (&val)[kMaxFacies]) {
@@ -100,7 +103,7 @@ __device__ __forceinline__ float facies_voxel(const float (&v)[3], int i, int j,
 #pragma unroll
       for (int q = 0; q < 4; q++) {
         const size_t at = cell[q] * nf4 + g;
-        if (C.pairs) {
+        if constexpr (PAIRS) {
           ldg_pair(P4 + 2 * at, x[q], x[4 + q]);
           if (edge) x[4 + q] = x[q];
         } else {

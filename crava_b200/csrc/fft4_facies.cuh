@@ -50,7 +50,8 @@ __global__ void __launch_bounds__(256) k_xc2r4_facies(const __grid_constant__ Fa
     const int s = 2 * r * CN + i;   // sample i of row r in a grid's buffer of 2 bw floats
     const float v[3] = {Vf[s], Vf[2 * bw + s], Vf[4 * bw + s]};
     float val[kMaxFacies];
-    const float sum = facies_voxel(v, i, j, F.nx, F.ny, C, F.nf, F.pr, F.undef_sum, val);
+    const float sum = C.pairs ? facies_voxel<true>(v, i, j, F.nx, F.ny, C, F.nf, F.pr, F.undef_sum, val)
+                              : facies_voxel<false>(v, i, j, F.nx, F.ny, C, F.nf, F.pr, F.undef_sum, val);
     for (int f = 0; f < F.nf; f++) F.out.p[f][o] = val[f] / sum;
     F.out.p[F.nf][o] = F.undef_sum / sum;
     if (F.seis_lh) F.seis_lh[o] = sum;

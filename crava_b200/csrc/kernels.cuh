@@ -11,11 +11,12 @@ namespace crava {
 
 // Launches whose kernels follow one another in a stream overlap the next one's launch with the last one's
 // end (programmatic dependent launch) where the grids they work on hold less than kDepBytes: there the
-// launch gaps are a good part of the pass (32x30x40: 33 -> 23 us, 64x64x128 with 26 MB: 76 -> 66).
-// Larger ones run slower that way (105x135x125 with 16 realisations, 400 MB: 0.91 -> 1.00 ms), the
-// waiting CTAs taking room from the last wave.  dep_wait, before a kernel touches memory that another
-// may have written or still reads, waits until the grids before it are over; dep_launch lets the next
-// grid's CTAs take their places.
+// launch gaps are a good part of the pass (64x64x128, 37 MB in all: 73.7 -> 65.1 us; 90x90x128, 73 MB: 120 -> 111).
+// Larger ones run slower that way, the waiting CTAs taking room from the last wave (all launches so: 105x135x125 with 4
+// to 16 realisations, 190 to 440 MB, 9 % slower; 160x160x160 10 %).  A job mixes both, each launch by its own
+// grids; of 20 blocks of 37 to 500 MB none is slower than without at this limit, while 96 MB costs 90x90x125 3 %.
+// dep_wait, before a kernel touches memory that another may have written or still reads, waits until the grids before
+// it are over; dep_launch lets the next grid's CTAs take their places.
 constexpr size_t kDepBytes = 64u << 20;
 template <class... P, class... A>
 inline cudaError_t launch_dep(size_t bytes, void (*fn)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st,
@@ -358,7 +359,7 @@ struct FaciesCornersHost {
   float4* packed[1 << kMaxFaciesAngles];          // device scratch of facies_packed_bytes each
 };
 size_t facies_packed_bytes(const FaciesBoxHost& b, int nf, bool pairs);
-// whether the volumes of hc.box are packed in pairs: while they then fit the L2
+// whether the volumes of hc.box are packed in pairs: neither small ones nor those that then pass the L2
 bool facies_pairs(const FaciesCornersHost& hc, int nf);
 // the probabilities from volumes already packed (launch_facies_prob_corners = pack + eval)
 cudaError_t launch_facies_eval(const float* vp, const float* vs, const float* rho, int nx, int ny, int nz, int rnxp_in,

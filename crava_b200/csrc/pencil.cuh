@@ -42,12 +42,12 @@
 // What bounds it: the latency of packed chains, shared memory and barriers at 16 warps an SM (128
 // registers, the tile in most of the shared memory), not HBM.  Against the scalar kernels with one
 // bin a lane (5 angles, 4 realisations unless noted; ms):
-//     540x540x256              6.52 -> 5.25   (25 % of the copy bandwidth)
+//     540x540x256              6.52 -> 5.21   (25 % of the copy bandwidth)
 //     768x768x320, 6 angles, 1 13.16 -> 10.18
-//     270x270x256              1.60 -> 1.25   (999 -> 596 M warp instructions, 42 % of the issue slots)
-//     250x250x200              2.18 -> 1.24
+//     270x270x256              1.60 -> 1.25   (999 -> 627 M warp instructions, 44 % of the issue slots)
+//     250x250x200              2.18 -> 1.28
 //     105x135x125, 16          0.61 -> 0.53
-//     200x216x200, prior grids 1.35 -> 0.96
+//     200x216x200, prior grids 1.35 -> 0.74, with FP64 0.82
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

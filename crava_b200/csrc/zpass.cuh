@@ -6,7 +6,7 @@
 // order of the forward transforms' roundings, however exact, changes them by that much.  For these jobs
 // the forward transforms keep the order they had (GridSet.plain for x and y), and this kernel
 // keeps it in z; at 128, 256 and 320 points pencil.cuh has the same splits and agrees to 1e-6.
-// (Timings beside pencil.cuh: 250x250x200, 5 angles, 4 realisations 2.18 against 1.24 ms.)
+// (Timings beside pencil.cuh: 250x250x200, 5 angles, 4 realisations 2.21 against 1.28 ms.)
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
