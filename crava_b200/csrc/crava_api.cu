@@ -2429,7 +2429,7 @@ namespace {
 // probabilities of crava_job_set_facies: the x transform and the evaluation in one pass
 // (launch_x4_facies) where the x length has a four-step split and the schedule key
 // facies_fused (n = nxp/2) is 1, else the x transform and then the facies pass.  The default
-// is the two passes: at 540x540x256, 3 facies, the one-pass form takes 4.77 ms against 0.37 + 1.36 ms, its
+// is the two passes: at 540x540x256, 3 facies, the one-pass form takes 3.56 ms against 0.36 + 1.37 ms, its
 // density gathers (L2-latency bound) running at the transform kernel's occupancy (8 warps
 // per SM against about 40 in the facies pass).
 crava_status inv_mean_facies(crava_ctx* ctx, crava_job* job, float ps, cudaStream_t st) {

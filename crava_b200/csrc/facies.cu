@@ -23,25 +23,27 @@ __global__ void k_facies_prob_corners(const float* __restrict__ vp, const float*
                                       const float* __restrict__ rho, int nx, int ny, int nz, int rnxp_in, int nyp_in,
                                       int rnxp_out, const __grid_constant__ FaciesCorners C, int nf, FaciesPrior pr,
                                       float undef_sum, FaciesOut out, float* __restrict__ seis_lh) {
-  // a warp per row (32-bit index arithmetic), eight rows per CTA; blockIdx.y takes a part of the rows
-  const int rows = ny * nz;
-  for (int r = blockIdx.x * blockDim.y + threadIdx.y; r < rows; r += gridDim.x * blockDim.y) {
-    const int k = r / ny, j = r - k * ny;
-    const size_t e0 = (size_t)rnxp_out * r, g0 = (size_t)rnxp_in * ((size_t)j + (size_t)nyp_in * k);
-    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < rnxp_out; i += gridDim.y * blockDim.x) {
-      const size_t e = e0 + i;
-      if (i >= nx) {
-        for (int f = 0; f <= nf; f++) out.p[f][e] = kRMissing;
-        if (seis_lh) seis_lh[e] = kRMissing;
-        continue;
-      }
-      const float v[3] = {vp[g0 + i], vs[g0 + i], rho[g0 + i]};
-      float val[kMaxFacies];
-      const float sum = facies_voxel<PAIRS>(v, i, j, nx, ny, C, nf, pr, undef_sum, val);
-      for (int f = 0; f < nf; f++) out.p[f][e] = val[f] / sum;
-      out.p[nf][e] = undef_sum / sum;
-      if (seis_lh) seis_lh[e] = sum;
+  // One voxel a thread and round, across the row ends: a voxel costs several hundred instructions, so that rows by whole
+  // warps pay for their idle lanes (37x400x60, 6 facies, 20x20x10 bins: 68 -> 53 us; 270x270x256 797 -> 745) and two
+  // 32-bit divisions do not show.  k_facies_prob_single, a few times cheaper, takes rows.
+  const size_t n = (size_t)rnxp_out * ny * nz;
+  const bool word = n <= 0xffffffffu;      // 32-bit divisions
+  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
+    const size_t r = word ? (size_t)((unsigned)e / (unsigned)rnxp_out) : e / rnxp_out;
+    const int i = (int)(e - r * rnxp_out), k = (int)(word ? (unsigned)r / (unsigned)ny : r / ny);
+    const int j = (int)(r - (size_t)k * ny);
+    if (i >= nx) {
+      for (int f = 0; f <= nf; f++) out.p[f][e] = kRMissing;
+      if (seis_lh) seis_lh[e] = kRMissing;
+      continue;
     }
+    const size_t g = i + (size_t)rnxp_in * ((size_t)j + (size_t)nyp_in * k);
+    const float v[3] = {vp[g], vs[g], rho[g]};
+    float val[kMaxFacies];
+    const float sum = facies_voxel<PAIRS>(v, i, j, nx, ny, C, nf, pr, undef_sum, val);
+    for (int f = 0; f < nf; f++) out.p[f][e] = val[f] / sum;
+    out.p[nf][e] = undef_sum / sum;
+    if (seis_lh) seis_lh[e] = sum;
   }
 }
 
@@ -303,11 +305,11 @@ cudaError_t launch_facies_eval(const float* vp, const float* vs, const float* rh
   for (int f = 0; f < nf; f++) pr.p[f] = prior[f];
   for (int f = 0; f <= nf; f++) po.p[f] = out[f];
   const FaciesCorners C = facies_corners(hc);
-  // a few long rows (a section of 4000 traces has 2 per slice) are shared by several warps each, until eight CTAs an
-  // SM have work (4000x2x40, 6 facies: 449 -> 58 us; 2000x1x200: 260 -> 64)
-  dim3 blocks((unsigned)std::min<size_t>(((size_t)ny * nz + 7) / 8, 148 * 32));
-  blocks.y = (unsigned)std::max(1, std::min((rnxp_out + 31) / 32, (148 * 8 + (int)blocks.x - 1) / (int)blocks.x));
   if (hc.nang == 0 && nf <= 4 && (size_t)hc.box[0].nb[0] * hc.box[0].nb[1] * hc.box[0].nb[2] < (1u << 30)) {
+    // a few long rows (a section of 4000 traces has 2 per slice) are shared by several warps each, until eight CTAs an
+    // SM have work
+    dim3 blocks((unsigned)std::min<size_t>(((size_t)ny * nz + 7) / 8, 148 * 32));
+    blocks.y = (unsigned)std::max(1, std::min((rnxp_out + 31) / 32, (148 * 8 + (int)blocks.x - 1) / (int)blocks.x));
     FaciesSingle F;
     F.dens = hc.packed[0];
     for (int d = 0; d < 3; d++) {
@@ -319,7 +321,8 @@ cudaError_t launch_facies_eval(const float* vp, const float* vs, const float* rh
         vp, vs, rho, nx, ny, nz, rnxp_in, nyp_in, rnxp_out, F, nf, pr, undef_sum, po, seis_lh);
     return cudaGetLastError();
   }
-  (hc.pairs ? k_facies_prob_corners<true> : k_facies_prob_corners<false>)<<<blocks, dim3(32, 8), 0, st>>>(
+  const int flat = (int)std::min<size_t>(((size_t)rnxp_out * ny * nz + 255) / 256, 148 * 32);
+  (hc.pairs ? k_facies_prob_corners<true> : k_facies_prob_corners<false>)<<<flat, 256, 0, st>>>(
       vp, vs, rho, nx, ny, nz, rnxp_in, nyp_in, rnxp_out, C, nf, pr, undef_sum, po, seis_lh);
   return cudaGetLastError();
 }
@@ -358,11 +361,12 @@ size_t facies_packed_bytes(const FaciesBoxHost& b, int nf, bool pairs) {
   return (pairs ? 2 : 1) * sizeof(float4) * (size_t)b.nb[0] * b.nb[1] * b.nb[2] * ((nf + 3) / 4);
 }
 
-// Above 8 MB, where scattered cells are fetched from the L2, and up to the 128 MB that it holds (facies.cuh has both sides).
+// Above 8 MB, where scattered cells are fetched from the L2, and up to 256 MB, twice what it holds (facies.cuh has both
+// sides).
 bool facies_pairs(const FaciesCornersHost& hc, int nf) {
   size_t bytes = 0;
   for (int c = 0; c < (1 << hc.nang); c++) bytes += facies_packed_bytes(hc.box[c], nf, true);
-  return bytes > 8u << 20 && bytes <= 128u << 20;
+  return bytes > 8u << 20 && bytes <= 256u << 20;
 }
 
 cudaError_t launch_spec_mul(float2* a, const float2* b, size_t n, cudaStream_t st) {

@@ -60,9 +60,10 @@ __device__ __forceinline__ void ldg_pair(const float4* p, float4& a, float4& b) 
 // once per volume.  The lookups are bound by the L1's one line a clock for scattered lanes where the
 // volumes sit in the L2, by the bytes beyond it, and by the L1's hits below it, which pairs halve (facies_pairs; us with
 // the packing, eight against four loads, a smooth mean and one of white noise):
-//   270x270x256, 3 facies   64x64x32 bins 332 / 332, 362 / 373   100x100x50 369 / 359, 510 / 396
-//                9 facies   20x20x10 bins 874 / 970, 1049 / 1040   64x64x32 1149 / 1185, 1627 / 1388   100x100x50 1377 / 1350, 1927 / 1423
-//   200x200x100, 16 volumes of 100x100x50 bins, 256 MB in pairs, 3 facies 3512 / 3640, 6 facies 5843 / 8856
+//   270x270x256, 3 facies    64x64x32 bins 341 / 338, 366 / 376   100x100x50 378 / 363, 512 / 401
+//                6 facies    20x20x10 bins 746 / 707, 831 / 794   64x64x32 896 / 934, 1113 / 1003   100x100x50 1133 / 1009, 1305 / 1018
+//                9 facies    20x20x10 bins 805 / 907, 971 / 965   64x64x32 1223 / 1224, 1609 / 1325   100x100x50 1652 / 1333, 1914 / 1369
+//   200x200x100, 16 volumes of 100x100x50 bins   3 facies, 256 MB in pairs 2258 / 1869, 2620 / 1990   6 facies, 512 MB 4185 / 6484, 4675 / 6853
 // The float operations per facies are the reference's, in its order.
 //
 // facies_voxel: the densities of voxel (i, j) of trace row j at the parameters v, prior-

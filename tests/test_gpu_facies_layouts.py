@@ -1,4 +1,4 @@
-"""Density volumes are packed in pairs of cells while they then take 8 to 128 MB, and one by one below and beyond: a large
+"""Density volumes are packed in pairs of cells while they then take 8 to 256 MB, and one by one below and beyond: a large
 volume and its crops, all with the bins that the parameters reach, lie in different layouts and give the same bits, in
 both kernels (up to four facies, more) and with corner volumes, from below the first bin centre on."""
 import numpy as np
